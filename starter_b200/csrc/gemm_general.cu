@@ -1,79 +1,296 @@
 // General matrix product C[M,N] = A[M,K] * W[N,K]^T on the CUDA cores, any M, N, K.
 //
-// This is the true 32-bit product of the float32 path (no tensor-core, no reduced-precision
-// mode) and the fallback of the bfloat16 path for shapes the tensor-core kernels refuse.
-// Each output element is one running sum over k = 0..K-1 in order, so a row's result does
-// not depend on how many other rows the call has.  The reference's products are
-// `x @ W.T` with W as [out, in] (engine/model.py:291,295,297,299).
+// This is the true 32-bit product of the float32 path (no tensor-core, no reduced-precision mode) and the fallback of
+// the bfloat16 path for shapes the tensor-core kernels refuse.  The reference's products are `x @ W.T` with W as
+// [out, in] (engine/model.py:291,295,297,299).
+//
+// Each output element is the sum, in order, of the sums over GG_CHUNK columns of k, each of them one running sum in
+// order: a function of K alone, so a row's result does not depend on how many other rows the call has, nor on which of
+// the tiles below took it, nor on whether the chunks ran side by side.
+//
+// Bound: the 32-bit multiply-adds (148 SMs x 128 a clock: 74 TFLOP/s at 1,965 MHz).  A block of 256 threads owns a tile of
+// BM x BN, a thread TM x TN of it as pairs (`fma.rn.f32x2`: half the instructions, which leaves issue slots for the
+// shared-memory reads); 16 columns of k at a time through two shared-memory buffers, the next ones in registers while
+// a tile is worked on.  Rows of few activations take a tile of 8, 32 or 64 rows, so that a product of a few rows streams
+// its weights instead of working for padding.  Where the tiles do not fill the GPU, the chunks of k run as blocks of
+// their own and a second kernel adds them up in order (`SPLIT`).
+// Measured (B200, 32-bit; the kernel before had one tile of 64 x 64 with scalar loads: 12 TFLOP/s at 300 rows): 300 rows of
+// [6144, 2560] 245 us (38 TFLOP/s), [2560, 4096] 196, [19456, 2560] 759, [2560, 9728] 382; 2,048 rows of [19456, 2560] 4.06 ms
+// (50 TFLOP/s); one row of [151936, 2560] 456 us (3.4 TB/s); 300 rows' error against 64 bits 4.1e-7.
 #include "common.cuh"
 
-#define GG_BM 64
-#define GG_BN 64
 #define GG_BK 16
+#define GG_CHUNK 512   // columns of k per running sum; a multiple of GG_BK
+#define GG_THREADS 256
 
-template <class TA, class TO>
-__global__ void __launch_bounds__(256) gemm_general_kernel(const TA* __restrict__ A, const TA* __restrict__ W,
-                                                           TO* __restrict__ C, int M, int N, int K) {
-    __shared__ float As[GG_BK][GG_BM + 4];
-    __shared__ float Ws[GG_BK][GG_BN + 4];
+template <class TA> struct GgFour;
+template <> struct GgFour<float> {
+    static __device__ __forceinline__ float4 load(const float* p) { return *reinterpret_cast<const float4*>(p); }
+};
+template <> struct GgFour<__nv_bfloat16> {
+    static __device__ __forceinline__ float4 load(const __nv_bfloat16* p) {
+        const uint2 v = *reinterpret_cast<const uint2*>(p);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+};
+
+// Four values of a row from column k on; zeros beyond the row count or beyond k_end.  VEC: K and the base allow one load.
+template <class TA, bool VEC>
+__device__ __forceinline__ float4 gg_fetch(const TA* __restrict__ X, int row, int rows, int k, int k_end, int K) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row >= rows) return v;
+    const TA* p = X + (long long)row * K + k;
+    if (VEC) {   // K % 4 == 0, and a chunk ends at a multiple of 4
+        if (k < k_end) v = GgFour<TA>::load(p);
+    } else {
+        if (k < k_end) v.x = to_f<TA>(p[0]);
+        if (k + 1 < k_end) v.y = to_f<TA>(p[1]);
+        if (k + 2 < k_end) v.z = to_f<TA>(p[2]);
+        if (k + 3 < k_end) v.w = to_f<TA>(p[3]);
+    }
+    return v;
+}
+
+template <class TA, class TO, int BM, int TM, int TN, bool SPLIT, bool VEC>
+__global__ void __launch_bounds__(GG_THREADS, BM == 8 ? 4 : SPLIT || BM < 128 ? 2 : 1)
+gemm_general_kernel(const TA* __restrict__ A, const TA* __restrict__ W, TO* __restrict__ C, int M, int N, int K) {
+    constexpr int GROUPS_M = BM / TM, GROUPS_N = GG_THREADS / GROUPS_M, BN = GROUPS_N * TN;
+    constexpr int LA = BM + 4, LW = BN + 4;
+    constexpr int FA = (BM * 4 + GG_THREADS - 1) / GG_THREADS, FW = BN * 4 / GG_THREADS;   // fours of k a thread fetches
+    constexpr int PM = TN == 1 ? TM / 2 : TM, PN = TN == 1 ? 1 : TN / 2;                    // pairs lie along n, or along m for TN = 1
+    __shared__ __align__(16) float As[2][GG_BK][LA];
+    __shared__ __align__(16) float Ws[2][GG_BK][LW];
     pdl_wait();
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * GG_BM, n0 = blockIdx.x * GG_BN;
-    const int tx = tid % 16, ty = tid / 16;  // thread computes rows ty*4.., cols tx*4..
-    const int lr = tid / 4, lk = (tid % 4) * 4;  // loader: row lr, k offset lk..lk+3
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    const int tid = threadIdx.x, tx = tid % GROUPS_N, ty = tid / GROUPS_N;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int k_first = SPLIT ? blockIdx.z * GG_CHUNK : 0;
+    const int k_last = SPLIT ? min(K, k_first + GG_CHUNK) : K;
 
-    for (int k0 = 0; k0 < K; k0 += GG_BK) {
+    float2 acc[PM][PN], total[SPLIT ? 1 : PM][SPLIT ? 1 : PN];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int k = k0 + lk + e;
-            const int am = m0 + lr, wn = n0 + lr;
-            As[lk + e][lr] = (am < M && k < K) ? to_f<TA>(A[(long long)am * K + k]) : 0.f;
-            Ws[lk + e][lr] = (wn < N && k < K) ? to_f<TA>(W[(long long)wn * K + k]) : 0.f;
+    for (int i = 0; i < PM; ++i)
+#pragma unroll
+        for (int j = 0; j < PN; ++j) {
+            acc[i][j] = make_float2(0.f, 0.f);
+            if (!SPLIT) total[i][j] = make_float2(0.f, 0.f);
         }
-        __syncthreads();
+
+    float4 fa[FA], fw[FW];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int e = 0; e < FA; ++e) {
+            const int i = tid + e * GG_THREADS;
+            fa[e] = i < BM * 4 ? gg_fetch<TA, VEC>(A, m0 + i / 4, M, k0 + (i % 4) * 4, k_last, K) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int e = 0; e < FW; ++e) {
+            const int i = tid + e * GG_THREADS;
+            fw[e] = gg_fetch<TA, VEC>(W, n0 + i / 4, N, k0 + (i % 4) * 4, k_last, K);
+        }
+    };
+    auto stage = [&](int buf) {
+#pragma unroll
+        for (int e = 0; e < FA; ++e) {
+            const int i = tid + e * GG_THREADS, r = i / 4, c = (i % 4) * 4;
+            if (i < BM * 4) {
+                As[buf][c][r] = fa[e].x;
+                As[buf][c + 1][r] = fa[e].y;
+                As[buf][c + 2][r] = fa[e].z;
+                As[buf][c + 3][r] = fa[e].w;
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < FW; ++e) {
+            const int i = tid + e * GG_THREADS, r = i / 4, c = (i % 4) * 4;
+            Ws[buf][c][r] = fw[e].x;
+            Ws[buf][c + 1][r] = fw[e].y;
+            Ws[buf][c + 2][r] = fw[e].z;
+            Ws[buf][c + 3][r] = fw[e].w;
+        }
+    };
+
+    fetch(k_first);
+    stage(0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = k_first; k0 < k_last; k0 += GG_BK, buf ^= 1) {
+        const bool more = k0 + GG_BK < k_last;
+        if (more) fetch(k0 + GG_BK);
 #pragma unroll
         for (int kk = 0; kk < GG_BK; ++kk) {
-            float a[4], w[4];
+            if constexpr (TN == 1) {
+                float a[TM];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+                for (int i = 0; i < TM; i += 4) *reinterpret_cast<float4*>(a + i) = *reinterpret_cast<const float4*>(&As[buf][kk][i]);
+                const float w = Ws[buf][kk][tx];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = Ws[kk][tx * 4 + j];
+                for (int i = 0; i < PM; ++i) acc[i][0] = fma_pair(make_float2(a[2 * i], a[2 * i + 1]), make_float2(w, w), acc[i][0]);
+            } else {   // the thread's rows and columns lie in runs of four, so that a warp's reads are whole lines
+                float a[TM], w[TN];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < TM; i += 4)
+                    *reinterpret_cast<float4*>(a + i) = *reinterpret_cast<const float4*>(&As[buf][kk][i * GROUPS_M + ty * 4]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+                for (int j = 0; j < TN; j += 4)
+                    *reinterpret_cast<float4*>(w + j) = *reinterpret_cast<const float4*>(&Ws[buf][kk][j * GROUPS_N + tx * 4]);
+#pragma unroll
+                for (int i = 0; i < PM; ++i)
+#pragma unroll
+                    for (int j = 0; j < PN; ++j)
+                        acc[i][j] = fma_pair(make_float2(a[i], a[i]), make_float2(w[2 * j], w[2 * j + 1]), acc[i][j]);
+            }
         }
+        if constexpr (!SPLIT) {
+            if ((k0 + GG_BK) % GG_CHUNK == 0 || !more) {
+#pragma unroll
+                for (int i = 0; i < PM; ++i)
+#pragma unroll
+                    for (int j = 0; j < PN; ++j) {
+                        total[i][j] = add_pair(total[i][j], acc[i][j]);
+                        acc[i][j] = make_float2(0.f, 0.f);
+                    }
+            }
+        }
+        if (more) stage(buf ^ 1);   // the buffer that everybody left before the last barrier
         __syncthreads();
     }
+    TO* out = C + (SPLIT ? (long long)blockIdx.z * M * N : 0ll);
+    auto value = [&](int i, int j) {
+        const float2 p = TN == 1 ? (SPLIT ? acc[i / 2][0] : total[SPLIT ? 0 : i / 2][0])
+                                 : (SPLIT ? acc[i][j / 2] : total[SPLIT ? 0 : i][SPLIT ? 0 : j / 2]);
+        return (TN == 1 ? i : j) % 2 ? p.y : p.x;
+    };
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + (TN == 1 ? i : (i / 4) * 4 * GROUPS_M + ty * 4 + i % 4);
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n < N) C[(long long)m * N + n] = from_f<TO>(acc[i][j]);
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + (TN == 1 ? tx : (j / 4) * 4 * GROUPS_N + tx * 4 + j % 4);
+            if (n < N) out[(long long)m * N + n] = from_f<TO>(value(i, j));
         }
     }
 }
 
-extern "C" int sb_gemm_general(int dtype, int out_f32, const void* A, const void* W, void* C, int M, int N, int K,
-                               cudaStream_t stream) {
+// The chunks' sums, added in order.
+template <class TO>
+__global__ void __launch_bounds__(256) gemm_general_add_kernel(const float* __restrict__ parts, TO* __restrict__ C, long long count,
+                                                               int chunks) {
+    pdl_wait();
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < count; i += gridDim.x * 256ll) {
+        float v = 0.f;
+        for (int c = 0; c < chunks; ++c) v += parts[(long long)c * count + i];
+        C[i] = from_f<TO>(v);
+    }
+}
+
+// A product of few outputs (bfloat16 run): a warp per output element, its lanes along k, so that a handful of columns
+// does not run as one block's serial chain (32 rows of [16, 1024]: 58 us as one tile, 3 as 512 warps).
+template <class TA, class TO>
+__global__ void __launch_bounds__(256) gemm_general_dot_kernel(const TA* __restrict__ A, const TA* __restrict__ W, TO* __restrict__ C,
+                                                               int M, int N, int K, int vec) {
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long long o = blockIdx.x * 8ll + (threadIdx.x >> 5);
+    if (o >= (long long)M * N) return;
+    const TA* a = A + (o / N) * (long long)K;
+    const TA* w = W + (o % N) * (long long)K;
+    float sum = 0.f;
+    if (vec) {
+        for (int k = lane * 4; k < K; k += 128) {
+            const float4 x = GgFour<TA>::load(a + k), y = GgFour<TA>::load(w + k);
+            sum = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, sum))));
+        }
+    } else {
+        for (int k = lane; k < K; k += 32) sum = fmaf(to_f<TA>(a[k]), to_f<TA>(w[k]), sum);
+    }
+    sum = warp_sum(sum);
+    if (lane == 0) C[o] = from_f<TO>(sum);
+}
+
+template <class TA, class TO, int BM, int TM, int TN>
+static void gg_launch(const void* A, const void* W, void* C, int M, int N, int K, float* parts, int vec, cudaStream_t stream) {
+    constexpr int BN = GG_THREADS / (BM / TM) * TN;
+    const int chunks = (K + GG_CHUNK - 1) / GG_CHUNK;
+    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, parts != nullptr ? chunks : 1);
+    if (parts != nullptr) {
+        if (vec)
+            sb_launch(gemm_general_kernel<TA, float, BM, TM, TN, true, true>, grid, GG_THREADS, 0, stream, (const TA*)A, (const TA*)W, parts, M, N, K);
+        else
+            sb_launch(gemm_general_kernel<TA, float, BM, TM, TN, true, false>, grid, GG_THREADS, 0, stream, (const TA*)A, (const TA*)W, parts, M, N, K);
+        const long long count = (long long)M * N;
+        const long long blocks = (count + 255) / 256;
+        sb_launch(gemm_general_add_kernel<TO>, dim3((unsigned int)(blocks < 4736 ? blocks : 4736)), 256, 0, stream, (const float*)parts, (TO*)C,
+                  count, chunks);
+    } else if (vec) {
+        sb_launch(gemm_general_kernel<TA, TO, BM, TM, TN, false, true>, grid, GG_THREADS, 0, stream, (const TA*)A, (const TA*)W, (TO*)C, M, N, K);
+    } else {
+        sb_launch(gemm_general_kernel<TA, TO, BM, TM, TN, false, false>, grid, GG_THREADS, 0, stream, (const TA*)A, (const TA*)W, (TO*)C, M, N, K);
+    }
+}
+
+static int gg_tile_rows(int M) {
+    if (M <= 8) return 8;
+    if (M <= 32) return 32;
+    if (M <= 64) return 64;
+    const int big = (M + 127) / 128 * 128, small = (M + 63) / 64 * 64;   // a tile of 64 rows reads half as much again per multiply-add
+    return big * 100 <= small * 120 ? 128 : 64;
+}
+
+template <class TA, class TO>
+static void gg_pick(const void* A, const void* W, void* C, int M, int N, int K, float* parts, int vec, cudaStream_t stream) {
+    switch (gg_tile_rows(M)) {
+        case 8: return gg_launch<TA, TO, 8, 8, 1>(A, W, C, M, N, K, parts, vec, stream);
+        case 32: return gg_launch<TA, TO, 32, 4, 4>(A, W, C, M, N, K, parts, vec, stream);
+        case 64: return gg_launch<TA, TO, 64, 4, 8>(A, W, C, M, N, K, parts, vec, stream);
+        default: return gg_launch<TA, TO, 128, 8, 8>(A, W, C, M, N, K, parts, vec, stream);
+    }
+}
+
+extern "C" {
+
+// Floats of scratch that a 32-bit product wants, 0 when its chunks of k run in one block.  Side by side they fill the
+// GPU (two blocks to an SM); in one block they save the trip of their sums through memory.  In units of one chunk of one
+// tile on one SM (44 us for 128 x 128 x 512 at three quarters of the peak): tiles / 148 rounds of all chunks against
+// tiles * chunks / 296 rounds of two, and 8 bytes a sum at 5 TB/s.
+long long sb_gemm_general_scratch(int M, int N, int K, int sms) {
+    const int chunks = (K + GG_CHUNK - 1) / GG_CHUNK;
+    if (chunks < 2 || M <= 0 || N <= 0 || sms <= 0) return 0;
+    const int bm = gg_tile_rows(M), bn = bm == 8 ? 256 : 128;
+    const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+    const long long floats = (long long)M * N * chunks;
+    if (floats > (64ll << 20)) return 0;
+    const double unit = 44.0 * (bm * (double)bn) / (128.0 * 128.0);   // us
+    const int resident = bm == 128 ? 1 : 2;
+    const double together = (double)((tiles + (long long)sms * resident - 1) / ((long long)sms * resident)) * resident * chunks * unit;
+    const double apart = (double)((tiles * chunks + 2ll * sms - 1) / (2ll * sms)) * 2 * unit + floats * 8.0 / 5e6 + 2.0;
+    return apart < together ? floats : 0;
+}
+
+int sb_gemm_general(int dtype, int out_f32, const void* A, const void* W, void* C, int M, int N, int K, float* parts,
+                    cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
-    dim3 grid((N + GG_BN - 1) / GG_BN, (M + GG_BM - 1) / GG_BM);
-    if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-    if (dtype == SB_F32)
-        sb_launch(gemm_general_kernel<float, float>, grid, 256, 0, stream, (const float*)A, (const float*)W, (float*)C, M, N, K);
-    else if (out_f32)
-        sb_launch(gemm_general_kernel<__nv_bfloat16, float>, grid, 256, 0, stream, (const __nv_bfloat16*)A, (const __nv_bfloat16*)W,
-                                                                           (float*)C, M, N, K);
-    else
-        sb_launch(gemm_general_kernel<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, stream, 
-            (const __nv_bfloat16*)A, (const __nv_bfloat16*)W, (__nv_bfloat16*)C, M, N, K);
+    if ((M + 63) / 64 > 65535) return (int)cudaErrorInvalidValue;
+    const unsigned long long low = (unsigned long long)A | (unsigned long long)W;
+    const int vec = K % 4 == 0 && low % (dtype == SB_F32 ? 16 : 8) == 0;
+    if (dtype == SB_F32) {
+        gg_pick<float, float>(A, W, C, M, N, K, parts, vec, stream);
+    } else if ((long long)M * N <= 4096) {
+        const dim3 grid((unsigned int)(((long long)M * N + 7) / 8));
+        if (out_f32)
+            sb_launch(gemm_general_dot_kernel<__nv_bfloat16, float>, grid, 256, 0, stream, (const __nv_bfloat16*)A, (const __nv_bfloat16*)W,
+                      (float*)C, M, N, K, vec);
+        else
+            sb_launch(gemm_general_dot_kernel<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)A,
+                      (const __nv_bfloat16*)W, (__nv_bfloat16*)C, M, N, K, vec);
+    } else if (out_f32) {
+        gg_pick<__nv_bfloat16, float>(A, W, C, M, N, K, parts, vec, stream);
+    } else {
+        gg_pick<__nv_bfloat16, __nv_bfloat16>(A, W, C, M, N, K, parts, vec, stream);
+    }
     SB_LAUNCH_CHECK();
 }
+
+}  // extern "C"

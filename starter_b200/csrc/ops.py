@@ -96,7 +96,7 @@ class Ops:
             "sb_rmsnorm": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
             "sb_swiglu": [c_int, c_void_p, c_void_p, c_int, c_int, c_void_p],
             "sb_advance_lengths": [SbBatch, c_void_p, c_void_p],
-            "sb_gemm_general": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+            "sb_gemm_general": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
             "sb_qk_rope_store": [c_int, c_int, c_void_p, c_void_p, SbBatch, SbKV, c_int, c_int, c_void_p, c_void_p,
                                  c_float, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
             "sb_attention_general": [c_int, c_void_p, c_void_p, SbBatch, SbKV, c_int, c_float, c_int, c_void_p],
@@ -209,6 +209,8 @@ class Ops:
             fn.restype = c_longlong
         lib.sb_delta_chunk_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.sb_delta_chunk_floats.restype = c_longlong
+        lib.sb_gemm_general_scratch.argtypes = [c_int, c_int, c_int, c_int]
+        lib.sb_gemm_general_scratch.restype = c_longlong
         lib.sb_set_pdl.argtypes = [c_int]
         lib.sb_set_pdl.restype = None
         self._scratch = {}
@@ -584,8 +586,10 @@ class Ops:
                     return torch.mm(a, w.t(), out_dtype=torch.float32)
                 return torch.mm(a, w.t())
         out = torch.empty((M, N), dtype=torch.float32 if out_float32 else a.dtype, device=a.device)
+        floats = self.lib.sb_gemm_general_scratch(M, N, K, self.sm_count())
+        parts = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
         self._check(self.lib.sb_gemm_general(_code(a.dtype), int(out_float32 or a.dtype == torch.float32), _ptr(a), _ptr(w),
-                                             _ptr(out), M, N, K, self._stream()), "gemm_general")
+                                             _ptr(out), M, N, K, _ptr(parts), self._stream()), "gemm_general")
         return out
 
     def linear_swiglu(self, h, w_gate_up, norm=None):

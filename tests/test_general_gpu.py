@@ -1,0 +1,69 @@
+"""The 32-bit product and attention at the borders of their tiles, chunks and head groups, against 64 bits."""
+
+import math
+
+import pytest
+import torch
+
+from starter_b200.cache import Cache, KVRequest
+from starter_b200.engine.context import StepContext
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from starter_b200.csrc.ops import get_ops
+    return get_ops(verbose=False)
+
+
+def rand(shape, seed):
+    return torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda")
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 32, 33, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("N, K", [(1, 3), (127, 512), (130, 513), (257, 1030), (40, 1537), (600, 2564)])
+def test_product_32_bit(ops, M, N, K):
+    a, w = rand((M, K), 1), rand((N, K), 2) * K ** -0.5
+    got = ops.linear(a, w)
+    want = a.double() @ w.double().T
+    # one rounding (2^-24 of the running sum) per multiply-add, errors of both signs: a few 1e-7 of the result's size
+    assert float((got - want).norm() / want.norm()) < 1e-6
+    assert float((got - want).abs().max()) < 2e-5
+    assert torch.equal(ops.linear(a[-1:].contiguous(), w), got[-1:]), "a row's sums depend on the rows beside it"
+
+
+@pytest.mark.parametrize("M, N, K", [(17, 3, 40), (64, 64, 1000), (32, 16, 1024), (70, 50, 37), (200, 33, 70)])
+def test_small_products_bfloat16(ops, M, N, K):
+    a, w = rand((M, K), 1).bfloat16(), (rand((N, K), 2) * K ** -0.5).bfloat16()
+    want = a.double() @ w.double().T
+    assert float((ops.linear(a, w, out_float32=True) - want).norm() / want.norm()) < 1e-6
+    assert float((ops.linear(a, w).double() - want).norm() / want.norm()) < 2.5e-3      # stored as bfloat16: 2^-9 a value
+
+
+@pytest.mark.parametrize("D, G, Gk", [(128, 4, 2), (80, 8, 1), (33, 2, 3), (256, 3, 2)])
+@pytest.mark.parametrize("window", [None, 70])
+def test_attention_32_bit(ops, D, G, Gk, window):
+    H, lens = G * Gk, [257, 1, 300]      # enough rows that a warp takes two or four heads where the group has them
+    cache = Cache([KVRequest(Gk, D)], n_slots=4, max_tokens=64 * 16, dtype=torch.float32, device="cuda", max_seq_tokens=320)
+    layer, slots = cache.layers[0], [cache.alloc() for _ in lens]
+    for s, n in zip(slots, lens):
+        cache.reserve(s, n)
+    cache.flush()
+    layer.k.copy_(rand(layer.k.shape, 3)), layer.v.copy_(rand(layer.v.shape, 4))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    cu = [0, 257, 258, 558]
+    ctx = StepContext(runtime=None, cache=cache, n_seqs=3, n_rows=558, max_q_len=300, kv_bound=300, seq_slot=i32(slots), cu_q=i32(cu),
+                      row_seq=i32([b for b, n in enumerate(lens) for _ in range(n)]), lengths=cache.lengths, status=i32([0]))
+    q = rand((558, H * D), 5)
+    got = ops.attention(ctx, q, layer, H, D ** -0.5, window)
+    for b, (s, n) in enumerate(zip(slots, lens)):
+        table = layer.group.table_host[s, :(n + 63) // 64].tolist()
+        k, v = (torch.cat([t[p] for p in table], dim=1)[:, :n].double() for t in (layer.k, layer.v))     # [Gk, n, D]
+        i, j = torch.arange(n, device="cuda")[:, None], torch.arange(n, device="cuda")[None]
+        seen = (j <= i) & (i - j < (window or n))
+        qs = q[cu[b]:cu[b + 1]].double().view(n, H, D)
+        for h in range(H):
+            sc = (qs[:, h] @ k[h // G].T * D ** -0.5).masked_fill(~seen, -math.inf)
+            want = torch.softmax(sc, -1) @ v[h // G]
+            assert float((got[cu[b]:cu[b + 1]].view(n, H, D)[:, h] - want).abs().max()) < 2e-5 * float(want.abs().max())
