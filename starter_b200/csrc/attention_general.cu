@@ -1,6 +1,6 @@
 // Causal grouped-query attention of a step's rows over the paged cache: any head size up
 // to 256, any number of heads and groups, any mix of row counts per sequence, with or
-// without a window.  One warp per (row, query head); keys in order, 32 at a time.
+// without a window.  One warp per row and up to four query heads of one key/value head; keys in order, 32 at a time.
 //
 // Reference: engine/kernels/attention.py:24-92.  Scores (q.k)*scale, running maximum,
 // exp and the sum l in 32-bit; the probabilities are rounded to T before they meet V
@@ -8,53 +8,67 @@
 // (attention.py:86-87).  Key n is visible to the row at position p when n <= p
 // (attention.py:75) and, with a window, p - n < window.  Query head h reads key/value head
 // h / (n_heads / n_kv_heads).  Tiles start at multiples of 32 in key index, so a row's
-// result depends on its position and its keys only, not on the batch around it.
+// result depends on its position and its keys only, not on the batch around it, nor on how many heads a warp takes.
+//
+// Bound: the reads of the keys, one row per lane (a line per lane and instruction).  Heads that share a key read it
+// together once there are enough warps for the GPU either way: 300 rows, 32 heads on 8 of 128, 32-bit: 404 us with a warp
+// per head, 154 with one per four heads (B200).
 #include "common.cuh"
 
 #define AG_MAX_D 256
 
-// q . k over D elements, in index order; 16-byte loads when the row allows them.
-__device__ __forceinline__ float dot_row(const float* qs, const float* kr, int D) {
-    float dot = 0.f;
+// q . k over D elements for HG queries, each in index order; 16-byte loads when the row allows them.
+template <int HG>
+__device__ __forceinline__ void dot_rows(const float* qs, const float* kr, int D, float (&dot)[HG]) {
     if ((D & 3) == 0) {
         for (int d = 0; d < D; d += 4) {
             const float4 v = *reinterpret_cast<const float4*>(kr + d);
-            dot = fmaf(qs[d], v.x, dot);
-            dot = fmaf(qs[d + 1], v.y, dot);
-            dot = fmaf(qs[d + 2], v.z, dot);
-            dot = fmaf(qs[d + 3], v.w, dot);
-        }
-    } else {
-        for (int d = 0; d < D; ++d) dot = fmaf(qs[d], kr[d], dot);
-    }
-    return dot;
-}
-
-__device__ __forceinline__ float dot_row(const float* qs, const __nv_bfloat16* kr, int D) {
-    float dot = 0.f;
-    if ((D & 7) == 0) {
-        for (int d = 0; d < D; d += 8) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(kr + d);
-            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = __bfloat1622float2(h[e]);
-                dot = fmaf(qs[d + 2 * e], f.x, dot);
-                dot = fmaf(qs[d + 2 * e + 1], f.y, dot);
+            for (int h = 0; h < HG; ++h) {
+                const float4 q = *reinterpret_cast<const float4*>(qs + h * AG_MAX_D + d);
+                dot[h] = fmaf(q.x, v.x, dot[h]);
+                dot[h] = fmaf(q.y, v.y, dot[h]);
+                dot[h] = fmaf(q.z, v.z, dot[h]);
+                dot[h] = fmaf(q.w, v.w, dot[h]);
             }
         }
     } else {
-        for (int d = 0; d < D; ++d) dot = fmaf(qs[d], __bfloat162float(kr[d]), dot);
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+            for (int h = 0; h < HG; ++h) dot[h] = fmaf(qs[h * AG_MAX_D + d], kr[d], dot[h]);
     }
-    return dot;
 }
 
-template <class T>
+template <int HG>
+__device__ __forceinline__ void dot_rows(const float* qs, const __nv_bfloat16* kr, int D, float (&dot)[HG]) {
+    if ((D & 7) == 0) {
+        for (int d = 0; d < D; d += 8) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(kr + d);
+            const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __bfloat1622float2(x[e]);
+#pragma unroll
+                for (int h = 0; h < HG; ++h) {
+                    dot[h] = fmaf(qs[h * AG_MAX_D + d + 2 * e], f.x, dot[h]);
+                    dot[h] = fmaf(qs[h * AG_MAX_D + d + 2 * e + 1], f.y, dot[h]);
+                }
+            }
+        }
+    } else {
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+            for (int h = 0; h < HG; ++h) dot[h] = fmaf(qs[h * AG_MAX_D + d], __bfloat162float(kr[d]), dot[h]);
+    }
+}
+
+// NJ: columns per lane (head sizes up to 32 * NJ).
+template <class T, int HG, int NJ>
 __global__ void attention_general_kernel(const T* __restrict__ q, T* __restrict__ out, SbBatch batch, SbKV kv,
                                          int n_heads, float scale, int window) {
-    __shared__ float qs[AG_MAX_D];
+    __shared__ __align__(16) float qs[HG * AG_MAX_D];
     pdl_wait();
-    const int row = blockIdx.x, head = blockIdx.y, lane = threadIdx.x;
+    const int row = blockIdx.x, head = blockIdx.y * HG, lane = threadIdx.x;
     const int D = kv.head_dim;
     const int kvh = head / (n_heads / kv.n_kv_heads);
     int slot, pos;
@@ -62,52 +76,91 @@ __global__ void attention_general_kernel(const T* __restrict__ q, T* __restrict_
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
 
     const T* qr = q + ((long long)row * n_heads + head) * D;
-    for (int d = lane; d < D; d += 32) qs[d] = to_f<T>(qr[d]);
+#pragma unroll
+    for (int h = 0; h < HG; ++h)
+        for (int d = lane; d < D; d += 32) qs[h * AG_MAX_D + d] = to_f<T>(qr[h * D + d]);
     __syncwarp();
 
-    float m = -INFINITY, l = 0.f;
-    float acc[AG_MAX_D / 32];
+    float m[HG], l[HG], acc[HG][NJ];
 #pragma unroll
-    for (int j = 0; j < AG_MAX_D / 32; ++j) acc[j] = 0.f;
+    for (int h = 0; h < HG; ++h) {
+        m[h] = -INFINITY;
+        l[h] = 0.f;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) acc[h][j] = 0.f;
+    }
     const T* kbase = (const T*)kv.k;
     const T* vbase = (const T*)kv.v;
 
     for (int n0 = (lo / 32) * 32; n0 <= pos; n0 += 32) {
         const int n = n0 + lane;
         const bool valid = n >= lo && n <= pos;
-        long long off = valid ? kv_offset(kv, slot, n, kvh) : -1;
-        float s = -INFINITY;
-        if (off >= 0) {
-            s = dot_row(qs, kbase + off, D) * scale;
-        }
-        const float m_new = fmaxf(m, warp_max(s));
-        if (m_new == -INFINITY) continue;  // no key of this tile has a page: nothing to add
-        const float p = off >= 0 ? expf(s - m_new) : 0.f;
-        const float alpha = expf(m - m_new);
-        l = l * alpha + warp_sum(p);
-        m = m_new;
-        const float pr = rnd<T>(p);
+        const long long off = valid ? kv_offset(kv, slot, n, kvh) : -1;
+        if (__all_sync(0xffffffffu, off < 0)) continue;  // no key of this tile has a page: nothing to add
+        float s[HG], pr[HG];
 #pragma unroll
-        for (int j = 0; j < AG_MAX_D / 32; ++j) acc[j] *= alpha;
+        for (int h = 0; h < HG; ++h) s[h] = 0.f;
+        if (off >= 0) dot_rows<HG>(qs, kbase + off, D, s);
+#pragma unroll
+        for (int h = 0; h < HG; ++h) {
+            s[h] = off >= 0 ? s[h] * scale : -INFINITY;
+            const float m_new = fmaxf(m[h], warp_max(s[h]));
+            const float p = off >= 0 && m_new != -INFINITY ? expf(s[h] - m_new) : 0.f;
+            const float alpha = m_new == -INFINITY ? 1.f : expf(m[h] - m_new);
+            l[h] = l[h] * alpha + warp_sum(p);
+            m[h] = m_new;
+            pr[h] = rnd<T>(p);
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) acc[h][j] *= alpha;
+        }
+#pragma unroll 4
         for (int t = 0; t < 32; ++t) {
             const long long voff = __shfl_sync(0xffffffffu, off, t);
-            const float pt = __shfl_sync(0xffffffffu, pr, t);
+            float pt[HG];
+#pragma unroll
+            for (int h = 0; h < HG; ++h) pt[h] = __shfl_sync(0xffffffffu, pr[h], t);
             if (voff < 0) continue;
             const T* vr = vbase + voff;
 #pragma unroll
-            for (int j = 0; j < AG_MAX_D / 32; ++j) {
+            for (int j = 0; j < NJ; ++j) {
                 const int d = lane + 32 * j;
-                if (d < D) acc[j] = fmaf(pt, to_f<T>(vr[d]), acc[j]);
+                if (d < D) {
+                    const float v = to_f<T>(vr[d]);
+#pragma unroll
+                    for (int h = 0; h < HG; ++h) acc[h][j] = fmaf(pt[h], v, acc[h][j]);
+                }
             }
         }
     }
-    T* orow = out + ((long long)row * n_heads + head) * D;
-    const float inv = 1.0f / l;
 #pragma unroll
-    for (int j = 0; j < AG_MAX_D / 32; ++j) {
-        const int d = lane + 32 * j;
-        if (d < D) orow[d] = from_f<T>(acc[j] * inv);
+    for (int h = 0; h < HG; ++h) {
+        T* orow = out + ((long long)row * n_heads + head + h) * D;
+        const float inv = 1.0f / l[h];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const int d = lane + 32 * j;
+            if (d < D) orow[d] = from_f<T>(acc[h][j] * inv);
+        }
     }
+}
+
+template <class T, int HG>
+static void ag_launch(const void* q, void* out, SbBatch batch, SbKV kv, int n_heads, float scale, int window, cudaStream_t stream) {
+    const dim3 grid(batch.n_rows, n_heads / HG);
+    if (kv.head_dim <= 128)
+        sb_launch(attention_general_kernel<T, HG, 4>, grid, 32, 0, stream, (const T*)q, (T*)out, batch, kv, n_heads, scale, window);
+    else
+        sb_launch(attention_general_kernel<T, HG, AG_MAX_D / 32>, grid, 32, 0, stream, (const T*)q, (T*)out, batch, kv, n_heads, scale, window);
+}
+
+// Heads of a key/value head that a warp takes together: as many as leave 1,184 warps (eight to each of 148 SMs).
+template <class T>
+static void ag_pick(const void* q, void* out, SbBatch batch, SbKV kv, int n_heads, float scale, int window, cudaStream_t stream) {
+    const int G = n_heads / kv.n_kv_heads;
+    const long long warps = (long long)batch.n_rows * n_heads;
+    if (G % 4 == 0 && warps / 4 >= 1184) return ag_launch<T, 4>(q, out, batch, kv, n_heads, scale, window, stream);
+    if (G % 2 == 0 && warps / 2 >= 1184) return ag_launch<T, 2>(q, out, batch, kv, n_heads, scale, window, stream);
+    return ag_launch<T, 1>(q, out, batch, kv, n_heads, scale, window, stream);
 }
 
 // q, out [rows, n_heads * head_dim]; window <= 0 means every earlier key.
@@ -115,12 +168,10 @@ extern "C" int sb_attention_general(int dtype, const void* q, void* out, SbBatch
                                     int window, cudaStream_t stream) {
     if (batch.n_rows <= 0) return 0;
     if (kv.head_dim > AG_MAX_D || n_heads % kv.n_kv_heads) return (int)cudaErrorInvalidValue;
-    dim3 grid(batch.n_rows, n_heads);
-    if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+    if (n_heads > 65535) return (int)cudaErrorInvalidValue;
     if (dtype == SB_F32)
-        sb_launch(attention_general_kernel<float>, grid, 32, 0, stream, (const float*)q, (float*)out, batch, kv, n_heads, scale, window);
+        ag_pick<float>(q, out, batch, kv, n_heads, scale, window, stream);
     else
-        sb_launch(attention_general_kernel<__nv_bfloat16>, grid, 32, 0, stream, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, batch,
-                                                                         kv, n_heads, scale, window);
+        ag_pick<__nv_bfloat16>(q, out, batch, kv, n_heads, scale, window, stream);
     SB_LAUNCH_CHECK();
 }
