@@ -38,10 +38,7 @@
 // scheduler; so were two threads per row, and the read of the next S overlapped with the write of P.
 // Every wait on an mbarrier is bounded; on a time-out the block raises SB_STATUS_TIMEOUT and a flag in shared
 // memory that ends every other wait of the block, which then frees its tensor memory and returns.
-#include <cuda.h>
-
-#include <mutex>
-
+#include "tc_maps.cuh"
 #include "tc_utils.cuh"
 
 #define PT_ROWS 128
@@ -377,38 +374,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
 // ---- host side ----------------------------------------------------------------------------------
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &qr) == cudaSuccess &&
-            qr == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    });
-    return fn;
-}
-
-// The pages of one layer's keys (or values) as a matrix [pages * kv_heads * 64 rows][128 columns] of
-// bfloat16, read in boxes of 64 rows x 64 columns with the 128-byte swizzle.
-static int make_page_map(CUtensorMap* map, const void* ptr, long long rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return (int)cudaErrorNotSupported;
-    cuuint64_t dims[2] = {PT_D, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {PT_D * 2};
-    cuuint32_t box[2] = {64, SB_PAGE};
-    cuuint32_t elem[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
-}
-
 // q, out [rows, n_heads * 128] bfloat16; n_pages: pages in the layer's pool (the null page included);
 // max_q_len bounds the rows any sequence brings.  Head size 128 only.
 extern "C" int sb_attn_prefill_tc(const void* q, void* out, SbBatch batch, SbKV kv, int n_heads, float scale, int window,
@@ -424,9 +389,9 @@ extern "C" int sb_attn_prefill_tc(const void* q, void* out, SbBatch batch, SbKV 
     }
     CUtensorMap mk, mv;
     const long long rows = (long long)n_pages * kv.n_kv_heads * SB_PAGE;
-    int e = make_page_map(&mk, kv.k, rows);
+    int e = make_rows_map(&mk, kv.k, rows, PT_D, PT_D, SB_PAGE);   // a layer's pages as rows of one token and kv head
     if (e) return e;
-    e = make_page_map(&mv, kv.v, rows);
+    e = make_rows_map(&mv, kv.v, rows, PT_D, PT_D, SB_PAGE);
     if (e) return e;
     const int G = n_heads / kv.n_kv_heads;
     const long long tiles = ((long long)max_q_len * G + PT_ROWS - 1) / PT_ROWS;

@@ -132,6 +132,10 @@ class Ops:
             "sb_flex_attention_general": [c_int, SbFlex, SbBatch, c_void_p, c_void_p],
             "sb_flex_attention_mma": [SbFlex, SbBatch, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p],
             "sb_flex_attention_rows64": [SbFlex, SbBatch, c_void_p, c_int, c_int, c_void_p],
+            "sb_flex_attention_tc": [SbFlex, SbBatch, c_void_p, c_int, c_int, c_void_p, c_void_p],
+            "sb_flex_attention_tc_rows": [SbFlex, SbBatch, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p,
+                                          c_int, c_void_p, c_void_p],
+            "sb_flex_attention_tc_takes": [c_int, c_int, c_int],
             "sb_kv_store": [c_int, c_void_p, c_longlong, c_void_p, c_longlong, SbBatch, SbFlex, c_int, c_float, c_void_p, c_void_p],
             "sb_rotate_pairs": [c_int, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, SbBatch, c_void_p,
                                 c_int, c_int, c_int, c_float, c_int, c_void_p],
@@ -231,6 +235,7 @@ class Ops:
         self.fuse_qk_balanced = os.environ.get("STARTER_B200_FUSE_QK_BALANCED", "0") != "0"
         self.prefetch_next_bytes = int(os.environ.get("STARTER_B200_PREFETCH_MAX", 24 << 20))
         self.prefill_tensor_memory = os.environ.get("STARTER_B200_PREFILL", "tc") != "mma"
+        self.flex_tc = True   # for tests and tuning runs: False leaves prompts to the mma.sync kernels
         self.flex_tensor_cores = os.environ.get("STARTER_B200_FLEX", "mma") != "general"   # "general": the warp-per-row kernel only
 
     # ---- plumbing -----------------------------------------------------------------------
@@ -578,14 +583,15 @@ class Ops:
             return self._skinny(a, w, N, False, out_float32, norm, add_to)
         if a.dtype == torch.bfloat16 and K % 8 == 0:
             if self._takes_stream(M, N, K, False):
-                return self._stream_product(a, w, N, False, out_float32)
+                return self._stream_product(a.contiguous(), w, N, False, out_float32)
             if M <= self.SKINNY_MAX_ROWS:
-                return self._skinny(a, w, N, False, out_float32)
-            if M * N * K > self.GENERAL_GEMM_MAX_WORK:
+                return self._skinny(a.contiguous(), w, N, False, out_float32)
+            if M * N * K > self.GENERAL_GEMM_MAX_WORK:   # a may be a view of wider rows here
                 if out_float32:
                     return torch.mm(a, w.t(), out_dtype=torch.float32)
                 return torch.mm(a, w.t())
         out = torch.empty((M, N), dtype=torch.float32 if out_float32 else a.dtype, device=a.device)
+        a = a.contiguous()
         floats = self.lib.sb_gemm_general_scratch(M, N, K, self.sm_count())
         parts = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
         self._check(self.lib.sb_gemm_general(_code(a.dtype), int(out_float32 or a.dtype == torch.float32), _ptr(a), _ptr(w),
@@ -954,6 +960,10 @@ class Ops:
         out = torch.empty((rows, H * v_dim), dtype=q.dtype, device=q.device)
         if v_dim > 1024:
             raise KernelError(f"attention takes values of up to 1024 columns, not {v_dim}")
+        if self._flex_takes_tc(ctx, q, p):
+            self._check(self.lib.sb_flex_attention_tc(p, self._batch(ctx), _ptr(out), ctx.max_q_len, layer_cache.group.pool_pages + 1,
+                                                      _ptr(self.kernel_status(q.device)), self._stream()), "flex_attention_tc")
+            return out
         if self._flex_takes_rows64(ctx, q, p, values_in_keys):
             self._check(self.lib.sb_flex_attention_rows64(p, self._batch(ctx), _ptr(out), ctx.max_q_len, int(values_in_keys),
                                                           self._stream()), "flex_attention_rows64")
@@ -987,6 +997,49 @@ class Ops:
         if smem < 0 or smem > self.MAX_BLOCK_SHARED:
             return False
         return q.stride(0) % 8 == 0 and q.stride(1) % 8 == 0 and q.data_ptr() % 16 == 0 and p.v_row % 8 == 0
+
+    FLEX_TC_MIN_ROWS = 128
+
+    def _flex_takes_tc(self, ctx, q, p: SbFlex) -> bool:
+        """The tcgen05 kernel takes prompts whose sequences bring a whole tile of 128 (position, head of the group) rows,
+        keys of 64 or 128 columns and values of 64 or 128.  Below a tile it would work for padding; there and up to some
+        200 rows both kernels take what their launch takes (18 to 25 us a call alone), from 500 rows on this one is ahead
+        (39 / 26 us at 500 tokens, 220 / 52 at 2,048: attention_flex_tc.cu has more)."""
+        if not self.flex_tensor_cores or not self.flex_tc or q.dtype != torch.bfloat16 or not self.lib.sb_flex_attention_tc_takes(p.k_dim, p.v_dim, 0):
+            return False
+        if ctx.max_q_len * (p.n_heads // p.n_kv_heads) < self.FLEX_TC_MIN_ROWS or p.pinned_pages:
+            return False
+        if not p.head_scale and not p.slopes and not p.scale > 0.0:
+            return False
+        return q.stride(0) % 8 == 0 and q.stride(1) % 8 == 0 and q.data_ptr() % 16 == 0 and p.v_row % 8 == 0
+
+    def takes_rows_attention(self, dtype, head_dim, shared_dim, v_dim) -> bool:
+        """Whether ``rows_attention`` takes heads of ``head_dim`` columns of their own, ``shared_dim`` shared ones and these values."""
+        return (self.flex_tensor_cores and self.flex_tc and dtype == torch.bfloat16 and head_dim % 64 == 0 and 0 < shared_dim <= 64
+                and bool(self.lib.sb_flex_attention_tc_takes(head_dim + shared_dim, v_dim, 1)))
+
+    def rows_attention(self, ctx, q, keys, shared, values, scale, sink=None):
+        """Causal attention among the step's own rows, every sequence from its first token on (nothing is read from a
+        cache): queries [rows, heads, D + R], a head's own key columns ``keys`` [rows, heads * D], R columns that all heads
+        share ``shared`` [rows, R], ``values`` [rows, heads * V] (views of wider rows will do) -> [rows, heads * V]."""
+        rows, H, kd = q.shape
+        R = shared.shape[1]
+        D, V = keys.shape[1] // H, values.shape[1] // H
+        for t in (q, keys, shared, values):
+            if t.dtype != torch.bfloat16 or t.stride(-1) != 1 or t.stride(0) % 8 or t.data_ptr() % 16 or t.shape[0] != rows:
+                raise KernelError("rows_attention: bfloat16 rows at multiples of 16 bytes")
+        if D + R != kd or keys.shape[1] != H * D or values.shape[1] != H * V or q.stride(1) % 8 or not scale > 0.0 \
+                or not self.takes_rows_attention(q.dtype, D, R, V):
+            raise KernelError(f"rows_attention does not take heads of {D} + {R} columns with values of {V}")
+        if sink is not None and (sink.dtype != torch.float32 or sink.numel() != H or not sink.is_contiguous()):
+            raise KernelError("per-head numbers of the attention are 32-bit, one per query head")
+        p = SbFlex(_ptr(q), q.stride(0), q.stride(1), None, None, None, None, None, _ptr(sink), 0, 0, H, H, kd, V, V, 0, 0, float(scale), 0, 0, 0,
+                   0.0, None)
+        out = torch.empty((rows, H * V), dtype=q.dtype, device=q.device)
+        self._check(self.lib.sb_flex_attention_tc_rows(p, self._batch(ctx), _ptr(keys), keys.stride(0), _ptr(shared), shared.stride(0),
+                                                       _ptr(values), values.stride(0), _ptr(out), ctx.max_q_len,
+                                                       _ptr(self.kernel_status(q.device)), self._stream()), "flex_attention_tc_rows")
+        return out
 
     FLEX_PROMPT_MIN_ROWS = 32
 

@@ -46,6 +46,7 @@ class StepContext:
     lengths: torch.Tensor   # int32 [n_slots + 1], the cache's
     status: torch.Tensor    # int32 [1], kernels raise bits here instead of faulting
     scratch: Dict[str, Any] = field(default_factory=dict)
+    first: bool = False     # host-side: no sequence of the step holds any token yet
     uneven: bool = False    # host-side hint: the longest sequence is several times the mean (see lengths_uneven)
 
     @property

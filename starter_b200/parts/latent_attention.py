@@ -13,12 +13,13 @@ denominator, with no key and no value.  A head's output may be multiplied by a g
 down-projections' product.  A layer with ``kv_from`` has no key/value down-projection and stores nothing: it reads the
 rows that the layer it names has cached, through its own W_uk and W_uv.
 
-A step that is ONE sequence's first (nothing cached before it: a whole prompt, or a prompt's first portion) may also
-take the narrow form: the step's own keys [W_uk[h] c | k_rot] and values W_uv[h] c are formed once, laid into pages of
-a scratch cache that the part keeps, and attended there with heads of head_dim + rot_dim and v_dim columns instead of
-kv_rank + rot_dim and kv_rank: a third of the arithmetic per (query, key) pair at usual sizes.  The step's rows go
-into the real cache all the same, for the steps that follow; they also wait in the step's scratch for the layers that
-read them.
+A step that is its sequences' first (nothing cached before it: whole prompts, or their first portions) may also
+take the narrow form: the step's own plain keys W_uk[h] c and values W_uv[h] c are formed once and attended as they lie
+(``rows_attention``), with heads of head_dim + rot_dim and v_dim columns instead of kv_rank + rot_dim and kv_rank: a
+third of the arithmetic per (query, key) pair at usual sizes.  Where the call table has no such call for these sizes, ONE
+sequence's rows are laid into pages of a scratch cache that the part keeps and attended there; several sequences' stay
+on the path that serves every step.  The step's rows go into the real cache all the same, for the steps that follow;
+they also wait in the step's scratch for the layers that read them.
 
 Steps: one product for both down-projections; one kernel that norms the query latent, norms the key/value latent,
 rotates the shared part and writes the cache row; the query's up-projection; its rotated part and, per head, its
@@ -74,8 +75,10 @@ class LatentAttention:
         # per head [kv_rank, head_dim]: the matrix that carries a plain query into the latent's space
         self.w_absorb = weights["uk"].view(H, D, spec.kv_rank).transpose(1, 2).contiguous()
         self.w_uv = weights["uv"].view(H, V, spec.kv_rank).contiguous()
-        self.w_uk_rows = self.ops.prepare_matrix(weights["uk"])      # [heads * head_dim, kv_rank]: the narrow form's keys
-        self.w_uv_rows = self.ops.prepare_matrix(weights["uv"])
+        # [heads * (head_dim + v_dim), kv_rank]: the narrow form's keys and values in one product
+        self.w_kv_rows = self.ops.prepare_matrix(torch.cat([weights["uk"], weights["uv"]], dim=0))
+        takes = getattr(self.ops, "takes_rows_attention", None)
+        self.in_place = takes is not None and spec.scale > 0 and spec.kv_rank % 8 == 0 and takes(runtime.dtype, D, R, V)   # the narrow form reads rows as they lie
         self._scratch = None                                         # (scratch cache of the narrow form, its batch description)
         self.q_norm = weights["dq_norm"]
         self.kv_norm = weights["dkv_norm"] if self.own_rows else None
@@ -112,14 +115,17 @@ class LatentAttention:
         H, D, R, V, rank = s.num_heads, s.head_dim, s.rot_dim, s.v_dim, s.kv_rank
         q = ops.linear(cq, self.w_uq).view(rows, H, D + R)
         ops.rotate_pairs(ctx, q[:, :, D:], q[:, :, D:], *self.turn)          # in place: a pair is read and written by one thread
-        latent = kept[:, :rank].contiguous()
-        keys = torch.empty((rows, H, D + R), dtype=q.dtype, device=q.device)
-        keys[:, :, :D] = ops.linear(latent, self.w_uk_rows).view(rows, H, D)
-        keys[:, :, D:] = kept[:, None, rank:]
-        values = ops.linear(latent, self.w_uv_rows)
-        layer, alone = self._scratch_cache(ctx, rows)
-        ops.kv_store(alone, keys.view(rows, H * (D + R)), values, layer)
-        o = ops.flex_attention(alone, q, layer, self.scale, v_dim=V, sink=self.sink)
+        if self.in_place:
+            kv = ops.linear(kept[:, :rank], self.w_kv_rows)
+            o = ops.rows_attention(ctx, q, kv[:, :H * D], kept[:, rank:], kv[:, H * D:], self.scale, sink=self.sink)
+        else:
+            kv = ops.linear(kept[:, :rank].contiguous(), self.w_kv_rows)
+            keys = torch.empty((rows, H, D + R), dtype=q.dtype, device=q.device)
+            keys[:, :, :D] = kv[:, :H * D].view(rows, H, D)
+            keys[:, :, D:] = kept[:, None, rank:]
+            layer, alone = self._scratch_cache(ctx, rows)
+            ops.kv_store(alone, keys.view(rows, H * (D + R)), kv[:, H * D:], layer)
+            o = ops.flex_attention(alone, q, layer, self.scale, v_dim=V, sink=self.sink)
         if gate is not None:
             o = ops.gate_heads(o.view(rows, H, V), gate).view(rows, H * V)
         return ops.linear(o, self.w_o)
@@ -130,7 +136,8 @@ class LatentAttention:
         rows = h.shape[0]
         down = ops.linear(h, self.w_down)
         gate = down[:, self.gate_col:] if s.head_gate else None
-        narrow = ctx.n_seqs == 1 and ctx.kv_bound == rows and rows >= NARROW_MIN_ROWS     # one sequence's first step
+        first = (ctx.n_seqs == 1 and ctx.kv_bound == rows) or (ctx.first and self.in_place)   # nothing cached before the step
+        narrow = first and rows >= NARROW_MIN_ROWS
         place = ("latent rows", id(layer_cache.group), layer_cache.index)                 # where the step's rows wait for their readers
         if not self.own_rows:
             cq, kept = ops.latent_prepare(ctx, down, None, s.q_rank, 0, 0, self.q_norm, None, self.eps), ctx.scratch.get(place)
