@@ -58,6 +58,15 @@ class SbDelta(Structure):
                 ("state", c_void_p), ("state_slot", c_longlong), ("H", c_int), ("G", c_int), ("D", c_int), ("V", c_int)]
 
 
+class SbChunkMem(Structure):
+    _fields_ = [("q", c_void_p), ("k", c_void_p), ("v", c_void_p), ("g", c_void_p), ("ld", c_longlong), ("z", c_void_p),
+                ("z_ld", c_longlong), ("i_col", c_int), ("f_col", c_int), ("bias", c_void_p), ("bias2", c_void_p), ("norm", c_void_p),
+                ("norm_stride", c_int), ("eps", c_float), ("inv_tau", c_float), ("cap", c_float), ("q_scale", c_float),
+                ("out_scale", c_float), ("state", c_void_p), ("state_stride", c_longlong), ("last", c_void_p), ("last_width", c_int),
+                ("last_offset", c_int), ("y", c_void_p), ("y_ld", c_longlong), ("work", c_void_p), ("H", c_int), ("D", c_int),
+                ("V", c_int)]
+
+
 class SbDecay(Structure):
     _fields_ = [("p", c_void_p), ("ld", c_longlong), ("q_col", c_int), ("k_col", c_int), ("v_col", c_int), ("act", c_int),
                 ("decay", c_void_p), ("log2_decay", c_void_p), ("dt", c_void_p), ("dt_ld", c_longlong), ("dt_bias", c_void_p),
@@ -186,6 +195,7 @@ class Ops:
                              c_float, c_float, c_int, c_void_p],
             "sb_moe_combine": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                c_int, c_void_p, c_int, c_void_p],
+            "sb_chunk_memory": [c_int, SbChunkMem, SbBatch, c_void_p],
             "sb_decay_step": [c_int, SbDecay, SbBatch, c_void_p, c_int, c_void_p],
             "sb_decay_chunk": [SbDecay, SbBatch, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p],
             "sb_silu_columns": [c_int, c_void_p, c_longlong, c_int, c_int, c_void_p],
@@ -211,6 +221,8 @@ class Ops:
         for fn in (lib.sb_flex_attention_mma_smem, lib.sb_flex_attention_rows64_smem, lib.sb_talking_attention_mma_smem):
             fn.argtypes = [c_int, c_int, c_int, c_int]
             fn.restype = c_longlong
+        lib.sb_chunk_memory_floats.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int]
+        lib.sb_chunk_memory_floats.restype = c_longlong
         lib.sb_delta_chunk_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.sb_delta_chunk_floats.restype = c_longlong
         lib.sb_gemm_general_scratch.argtypes = [c_int, c_int, c_int, c_int]
@@ -1147,10 +1159,49 @@ class Ops:
             if t.dtype != torch.float32 or not t.is_contiguous():
                 raise KernelError("wkv_scan: decay, bonus and norm weights are 32-bit")
         y = torch.empty((h.shape[0], inner), dtype=h.dtype, device=h.device)
+        if self.chunk_memory(ctx, self.CHUNK_WKV, heads, dim, dim, r, k, v, g, inner, decay_pre, w0, u, norm, dim, eps, state, y,
+                             last=h, last_offset=int(prev_offset)):
+            return y
         self._check(self.lib.sb_wkv_scan(_code(h.dtype), _ptr(r), _ptr(k), _ptr(v), _ptr(g), _ptr(decay_pre), _ptr(w0), _ptr(u),
                                          _ptr(norm), float(eps), _ptr(h), h.shape[1], _ptr(state), state.stride(0),
                                          int(prev_offset), self._batch(ctx), heads, dim, _ptr(y), self._stream()), "wkv_scan")
         return y
+
+    CHUNK_WKV, CHUNK_GLA, CHUNK_MLSTM = 0, 1, 2
+    force_chunk_memory = None   # True or False for tests and tuning; None = the rule below
+
+    def chunk_memory_pays(self, n_seqs: int, rows: int, max_q_len: int, H: int, V: int) -> bool:
+        """Whether a step of this shape is sooner done in chunks than token by token.  The walk is a chain over the longest
+        sequence's tokens and fills the GPU with many sequences; the chunks' three or four kernels have a price of their own and
+        one per chunk and head.  The three rates below are fits to (us, walk / chunks): 32 heads of 64 x 64 (wkv), one sequence of
+        64 / 128 / 256 / 2,048 rows: 34 / 33, 62 / 34, 118 / 38, 903 / 113, 16 of 64 and 128 rows: 93 / 75, 172 / 123, 64 of 16 and 64
+        rows: 97 / 171, 325 / 246; 16 heads of 64 x 128, one of 64 / 128 / 3,333 rows: gla 32 / 39, 55 / 39, 1,277 / 140, mlstm 32 / 34,
+        55 / 34, 1,135 / 118, 64 of 16 and 64 rows: gla 99 / 152, 320 / 214, mlstm 154 / 181, 385 / 183."""
+        if self.force_chunk_memory is not None:
+            return self.force_chunk_memory
+        chunks = rows / 64 + n_seqs / 2
+        walk = max(10 + 0.43 * max_q_len, 0.0025 * rows * H * -(-V // 64))
+        return 35 + (0.1 if V <= 64 else 0.15) * chunks * H < walk
+
+    def chunk_memory(self, ctx, kind, H, D, V, q, k, v, g, ld, z, bias, bias2, norm, norm_stride, eps, state, y, z_cols=(0, 0), inv_tau=0.0,
+                     cap=0.0, q_scale=1.0, out_scale=1.0, last=None, last_offset=0) -> bool:
+        """The recurrence of wkv_scan, gla_scan or mlstm_scan over 64 tokens at a time, all chunks side by side
+        (chunk_memory.cu); False, with nothing done, where the walk token by token has to do it: 32-bit runs, heads of more
+        than 128 channels, and steps that it does sooner."""
+        rows = q.shape[0]
+        if q.dtype != torch.bfloat16 or not self.chunk_memory_pays(ctx.n_seqs, rows, ctx.max_q_len, H, V):
+            return False
+        floats = self.lib.sb_chunk_memory_floats(kind, rows, ctx.n_seqs, H, D, V)
+        if floats < 0:
+            return False
+        work = torch.empty(floats, dtype=torch.float32, device=q.device)
+        a = SbChunkMem(_ptr(q), _ptr(k), _ptr(v), _ptr(g), ld, _ptr(z), z.stride(0), int(z_cols[0]), int(z_cols[1]), _ptr(bias), _ptr(bias2),
+                       _ptr(norm), norm_stride, float(eps), float(inv_tau), float(cap), float(q_scale), float(out_scale), _ptr(state),
+                       state.stride(0), _ptr(last), last.shape[1] if last is not None else 0, int(last_offset), _ptr(y), y.stride(0),
+                       _ptr(work), H, D, V)
+        self._check(self.lib.sb_chunk_memory(kind, a, self._batch(ctx), self._stream()), "chunk_memory")
+        self.launches += 3 if kind == self.CHUNK_MLSTM else 2   # the gates, the chunks' shares, the walk over them, the outputs
+        return True
 
     # ---- a residual in streams, two-map attention, gated linear attention, experts -------
 
@@ -1351,6 +1402,9 @@ class Ops:
             raise KernelError("mlstm_scan: the output has one column per head and value channel, in the run's dtype")
         else:
             y = out
+        if self.chunk_memory(ctx, self.CHUNK_MLSTM, heads, dim, vdim, q, k, v, g, ld, z, i_bias, f_bias, norm, vdim, eps, state, y,
+                             z_cols=(i_col, f_col), cap=cap, q_scale=q_scale, out_scale=out_scale):
+            return y
         raw = torch.empty((rows, heads * vdim), dtype=torch.float32, device=q.device) if vdim > 64 else None
         self._check(self.lib.sb_mlstm_scan(_code(q.dtype), _ptr(q), _ptr(k), _ptr(v), _ptr(g), ld, _ptr(z), z.stride(0), int(i_col),
                                            int(f_col), _ptr(i_bias), _ptr(f_bias), float(cap), _ptr(norm), float(eps), float(q_scale),
@@ -1375,6 +1429,9 @@ class Ops:
         if tuple(z.shape) != (rows, heads * dim) or state.shape[1] != heads * dim * vdim or norm.numel() != vdim:
             raise KernelError("gla_scan: sizes do not fit")
         y = torch.empty((rows, heads * vdim), dtype=q.dtype, device=q.device)
+        if tau > 0 and self.chunk_memory(ctx, self.CHUNK_GLA, heads, dim, vdim, q, k, v, g, ld, z, bias, None, norm, 0, eps, state, y,
+                                         inv_tau=1.0 / tau, q_scale=q_scale):
+            return y
         # heads of more than 64 value channels: their columns are shared out over blocks, which leave raw outputs here
         raw = torch.empty((rows, heads * vdim), dtype=torch.float32, device=q.device) if vdim > 64 else None
         self._check(self.lib.sb_gla_scan(_code(q.dtype), _ptr(q), _ptr(k), _ptr(v), _ptr(g), ld, _ptr(z), _ptr(bias), _ptr(norm),
