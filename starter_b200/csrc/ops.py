@@ -208,6 +208,7 @@ class Ops:
                                    c_void_p, c_void_p],
             "sb_xielu": [c_int, c_void_p, c_void_p, c_longlong, c_float, c_float, c_void_p],
             "sb_talking_attention_general": [c_int, SbFlex, SbBatch, c_void_p, c_int, c_void_p, c_void_p],
+            "sb_talking_decode": [SbFlex, SbBatch, c_void_p, c_int, c_void_p, c_void_p],
             "sb_talking_attention_mma": [SbFlex, SbBatch, c_void_p, c_int, c_int, c_void_p, c_void_p],
             "sb_qk_norm_store": [c_int, c_void_p, c_void_p, SbBatch, SbFlex, c_int, c_void_p, c_void_p, c_float, c_void_p, c_void_p],
             "sb_argmax": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p],
@@ -218,7 +219,8 @@ class Ops:
             fn = getattr(lib, name)
             fn.argtypes = argtypes
             fn.restype = c_int
-        for fn in (lib.sb_flex_attention_mma_smem, lib.sb_flex_attention_rows64_smem, lib.sb_talking_attention_mma_smem):
+        for fn in (lib.sb_flex_attention_mma_smem, lib.sb_flex_attention_rows64_smem, lib.sb_talking_attention_mma_smem,
+                   lib.sb_talking_decode_smem):
             fn.argtypes = [c_int, c_int, c_int, c_int]
             fn.restype = c_longlong
         lib.sb_chunk_memory_floats.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int]
@@ -1818,7 +1820,9 @@ class Ops:
         p = self._flex(layer_cache, q, H, scale, g.v_dim, False, sink, None, None, None, window, keep_first, softcap, talk)
         out = torch.empty((rows, H * g.v_dim), dtype=q.dtype, device=q.device)
         mma = self._talk_takes_mma(ctx, q, p)
-        n_splits = self.talk_mma_splits(ctx, p, g.table_width) if mma else self.talk_splits(ctx, p, g.table_width)
+        decode = not mma and self._talk_takes_decode(q, p)
+        n_splits = (self.talk_mma_splits(ctx, p, g.table_width) if mma else self.talk_decode_splits(ctx, p, g.table_width) if decode
+                    else self.talk_splits(ctx, p, g.table_width))
         partial = None
         if n_splits > 1:
             key = ("talk_partial", q.device, rows, H, n_splits, g.v_dim)
@@ -1828,6 +1832,8 @@ class Ops:
         if mma:
             self._check(self.lib.sb_talking_attention_mma(p, self._batch(ctx), _ptr(out), ctx.max_q_len, n_splits, _ptr(partial),
                                                           self._stream()), "talking_attention_mma")
+        elif decode:
+            self._check(self.lib.sb_talking_decode(p, self._batch(ctx), _ptr(out), n_splits, _ptr(partial), self._stream()), "talking_decode")
         else:
             self._check(self.lib.sb_talking_attention_general(_code(q.dtype), p, self._batch(ctx), _ptr(out), n_splits, _ptr(partial),
                                                               self._stream()), "talking_attention_general")
@@ -1840,14 +1846,33 @@ class Ops:
     def _talk_takes_mma(self, ctx, q, p: SbFlex) -> bool:
         """The tensor-core kernel (16 positions with all their heads per block) takes bfloat16 steps in which a sequence
         brings at least 4 rows, key widths that are multiples of 16, values of 64 or 128 columns, up to 32 heads (16 with
-        values of 128 columns) and rows it can fetch 16 bytes at a time; the block-per-row kernel serves everything else
-        (decoding, and every 32-bit run)."""
+        values of 128 columns) and rows it can fetch 16 bytes at a time; decoding has a kernel of its own (_talk_takes_decode),
+        the block-per-row kernel serves everything else (every 32-bit run, other widths)."""
         if not self.flex_tensor_cores or q.dtype != torch.bfloat16 or ctx.max_q_len < self.TALK_PROMPT_MIN_ROWS:
             return False
         smem = self.lib.sb_talking_attention_mma_smem(p.n_heads, p.n_kv_heads, p.k_dim, p.v_dim)
         if smem < 0 or smem > self.MAX_BLOCK_SHARED:
             return False
         return q.stride(0) % 8 == 0 and q.stride(1) % 8 == 0 and q.data_ptr() % 16 == 0 and p.v_row % 8 == 0
+
+    def _talk_takes_decode(self, q, p: SbFlex) -> bool:
+        """The tensor-core kernel of a row at a time (attention_talk_decode.cu): bfloat16, widths of 64 or 128, up to 5 query
+        heads per key/value head and 16 key/value heads, rows it can fetch 16 bytes at a time."""
+        if not self.flex_tensor_cores or q.dtype != torch.bfloat16:
+            return False
+        smem = self.lib.sb_talking_decode_smem(p.n_heads, p.n_kv_heads, p.k_dim, p.v_dim)
+        return (0 <= smem <= self.MAX_BLOCK_SHARED and p.v_heads in (0, p.n_kv_heads) and q.stride(0) % 8 == 0 and q.stride(1) % 8 == 0
+                and q.data_ptr() % 16 == 0 and p.v_row % 8 == 0)
+
+    def talk_decode_splits(self, ctx, p: SbFlex, max_pages: int) -> int:
+        """Blocks along the keys per row: enough to fill the GPU with two blocks of eight warps per SM (measured in the step, us at
+        8 / 16 / 24 / 32 warps per SM: 8 rows of 2,049 keys 737 / 697 / 696 / 696, 32 rows 1,545 / 1,248 / 1,426 / 1,283), none with
+        less than a page.  A function of shapes only, so that a captured graph stays valid."""
+        reach = max_pages
+        if p.window:
+            reach = min(reach, (p.window + 62) // 64 + 1 + -(-p.keep_first // 64))
+        pages = max(1, min(reach, -(-ctx.kv_bound // 64)))
+        return max(1, min(16 * self.sm_count() // max(1, ctx.n_rows * p.n_kv_heads), pages, 64))
 
     def talk_splits(self, ctx, p: SbFlex, max_pages: int) -> int:
         """Blocks along the keys per row of the block-per-row kernel: enough for two blocks per SM, none with less than

@@ -576,3 +576,24 @@ def test_the_trace_runner_replays_this_design(folders, tmp_path):
     want = {0: torch.stack([ref[0][14], ref[1][0], ref[1][7]]), 1: torch.stack([ref[0][15], ref[1][8]]), 3: ref[0][19:20]}
     for i, r in want.items():
         assert float((read(i) - r).abs().max()) <= 1e-4 * float(r.abs().max()), f"step {i}"
+
+
+@pytest.mark.parametrize("splits", [None, 1, 2, 7])
+@pytest.mark.parametrize("sizes", [
+    dict(H=10, G=2, D=128, V=64, window=None, softcap=20.0),              # five heads per key/value head: all 15 rows of weights
+    dict(H=16, G=16, D=64, V=128, window=300, keep=70, softcap=30.0),     # sixteen warps, kept pages before the window's
+    dict(H=3, G=1, D=64, V=64, window=129, keep=3),                       # one warp, no cap
+    dict(H=6, G=3, D=128, V=128, window=None, talk=False),                # no table, warps that are no whole number of 64 keys
+])
+def test_decoding_over_any_share_of_the_pages(monkeypatch, sizes, splits):
+    """One row at a time after a prompt: blocks of one page and of several, shares that come out empty, one block per row."""
+    rt = runtime("bfloat16")
+    if splits is not None:
+        monkeypatch.setattr(rt.ops, "talk_decode_splits", lambda *a: splits, raising=False)
+    spec = talk_spec(**sizes)
+    w = talk_weights(spec, 140)
+    n = 450
+    h = rand((n, spec.hidden_size), 9)
+    want = plain_attention(h, w, spec)
+    got, _, _ = run_mixer(rt, talk_part(rt, spec, w), h, [n - 70] + [1] * 70, max_step_tokens=512, pages=24)
+    close(got, want, "bfloat16", f"{splits} shares")
