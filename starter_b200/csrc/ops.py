@@ -1668,7 +1668,7 @@ class Ops:
                 pair_of_slot = torch.empty(pairs, dtype=torch.int32, device=h.device)
                 self._check(self.lib.sb_moe_sort(_ptr(chosen), pairs, n_experts, _ptr(ends), _ptr(slot_of_pair), _ptr(pair_of_slot),
                                                  self._stream()), "moe_sort")
-                xs = torch.zeros((pairs, width), dtype=h.dtype, device=h.device)
+                xs = torch.empty((pairs, width), dtype=h.dtype, device=h.device)
                 self._check(self.lib.sb_moe_gather(dt, _ptr(h), _ptr(pair_of_slot), _ptr(ends), n_experts, pairs, top, width,
                                                    _ptr(xs), self._stream()), "moe_gather")
                 gu = torch._grouped_mm(xs, w_gate_up.transpose(1, 2), offs=ends)
