@@ -84,7 +84,110 @@ __global__ void conv_qk_store_kernel(const T* __restrict__ q, long long q_ld, co
     }
 }
 
-// After the kernel above: a sequence's record becomes its last taps - 1 biased projections.  A step of fewer rows
+#define CQ_RUN 8
+
+// Many bfloat16 rows with heads of 32 N columns and up to four taps: a warp takes a head and CQ_RUN rows one after another, N
+// columns a lane, the earlier inputs and the weights in registers (missing taps are zeros that meet zeros); the sums run in the
+// order of the kernel above.  A block per row, which read every input and weight once per tap: 3,333 rows of 12 heads of 128 67 us,
+// this 25.
+template <int N>
+__global__ void __launch_bounds__(128)
+conv_qk_rows_kernel(const __nv_bfloat16* __restrict__ q, long long q_ld, const __nv_bfloat16* __restrict__ k, long long k_ld,
+                    const float* __restrict__ q_bias, const float* __restrict__ k_bias, const float* __restrict__ q_conv,
+                    const float* __restrict__ k_conv, int taps, const float* __restrict__ state, long long state_slot,
+                    const float* __restrict__ q_norm, const float* __restrict__ k_norm, float eps, float temp_coef, int temp_every,
+                    __nv_bfloat16* __restrict__ q_out, SbBatch batch, SbFlex p, int H, int* status) {
+    constexpr int D = 32 * N;
+    pdl_wait();
+    const int lane = threadIdx.x & 31, u = blockIdx.y * 4 + (threadIdx.x >> 5), G = p.n_kv_heads;
+    if (u >= H + G) return;
+    const int row0 = blockIdx.x * CQ_RUN, nr = min(CQ_RUN, batch.n_rows - row0);
+    const bool is_q = u < H;
+    const int h = is_q ? u : u - H, c = lane * N, ch = h * D + c, keep = taps - 1, rec_width = (H + G) * D;
+    const __nv_bfloat16* x = (is_q ? q : k) + ch;
+    const long long ld = is_q ? q_ld : k_ld;
+    const float* bias_p = is_q ? q_bias : k_bias;
+    const float* conv = (is_q ? q_conv : k_conv) + (long long)ch * taps;
+    const float* norm_p = is_q ? q_norm : k_norm;
+    float w[4][N], bias[N], nw[N], in[4][N];       // in: the inputs of the row three before to the row itself
+    float rows[CQ_RUN][N];
+#pragma unroll
+    for (int r = 0; r < CQ_RUN; ++r) load_bf16<N>(x + (long long)min(row0 + r, batch.n_rows - 1) * ld, rows[r]);
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+        bias[e] = bias_p != nullptr ? bias_p[ch + e] : 0.f;
+        nw[e] = norm_p != nullptr ? norm_p[c + e] : 1.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j][e] = j >= 4 - taps ? conv[e * taps + j - (4 - taps)] : 0.f;
+    }
+    int last_s = -1, slot = 0, first = 0, held = 0;
+#pragma unroll
+    for (int r = 0; r < CQ_RUN; ++r) {
+        if (r >= nr) break;
+        const int row = row0 + r, s = batch.row_seq[row];
+        if (s != last_s) {
+            last_s = s;
+            slot = batch.seq_slot[s];
+            first = batch.cu_q[s];
+            held = batch.lengths[slot];
+#pragma unroll
+            for (int back = 3; back >= 1; --back) {
+                const int src = row - first - back;
+                float f[N];
+#pragma unroll
+                for (int e = 0; e < N; ++e) f[e] = 0.f;
+                if (back <= keep) {
+                    if (src >= 0) {
+                        load_bf16<N>(x + (long long)(first + src) * ld, f);
+#pragma unroll
+                        for (int e = 0; e < N; ++e) f[e] += bias[e];
+                    } else {
+                        const float* rec = state + (long long)slot * state_slot + (long long)(keep + src) * rec_width + (is_q ? 0 : H * D) + ch;
+#pragma unroll
+                        for (int e = 0; e < N; ++e) f[e] = rec[e];
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < N; ++e) in[3 - back][e] = f[e];
+            }
+        }
+        float y[N], ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            in[3][e] = rows[r][e] + bias[e];
+            float a = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) a = fmaf(w[j][e], in[j][e], a);
+            y[e] = a;
+            ss = fmaf(a, a, ss);
+            in[0][e] = taps >= 4 ? in[1][e] : 0.f;
+            in[1][e] = taps >= 3 ? in[2][e] : 0.f;
+            in[2][e] = taps >= 2 ? in[3][e] : 0.f;
+        }
+        const int pos = held + row - first;
+        const float rstd = norm_p != nullptr ? 1.0f / sqrtf(warp_sum(ss) / (float)D + eps) : 1.0f;
+        float out[N];
+        if (is_q) {
+            float temp = 1.0f;
+            if (temp_every > 0) temp = 1.0f + temp_coef * logf((float)((pos + 1) / temp_every + 1));
+#pragma unroll
+            for (int e = 0; e < N; ++e) out[e] = y[e] * rstd * nw[e] * temp;
+            store_bf16<N>(q_out + ((long long)row * H + h) * D + c, out);
+        } else {
+            const long long tok = flex_token(p, slot, pos, h);
+            if (tok < 0) {
+                if (lane == 0) atomicOr(status, SB_STATUS_NO_PAGE);
+                continue;
+            }
+#pragma unroll
+            for (int e = 0; e < N; ++e) out[e] = y[e] * rstd * nw[e];
+            store_bf16<N>((__nv_bfloat16*)p.k + tok * D + c, out);
+            store_bf16<N>((__nv_bfloat16*)p.v + flex_value_token(p, tok, h) * p.v_row + c, y);
+        }
+    }
+}
+
+// After the kernels above: a sequence's record becomes its last taps - 1 biased projections.  A step of fewer rows
 // than that keeps the later entries of the old record: a thread reads its channel's entries before it writes them.
 template <class T>
 __global__ void conv_qk_state_kernel(const T* __restrict__ q, long long q_ld, const T* __restrict__ k, long long k_ld,
@@ -121,6 +224,25 @@ __global__ void head_gate_kernel(const T* __restrict__ a, const float* __restric
     }
 }
 
+// bfloat16 with heads of a multiple of 8 columns: 16 bytes a thread.  3,333 rows of 8 heads of 128, a number a thread 20 us, this 5.
+__global__ void __launch_bounds__(256) head_gate_vec_kernel(const __nv_bfloat16* __restrict__ a, const float* __restrict__ z, long long z_ld,
+                                                            int z_col, __nv_bfloat16* __restrict__ out, long long out_ld, long long rows, int H,
+                                                            int V8, float scale) {
+    pdl_wait();
+    const int per_row = H * V8;
+    const long long n = rows * per_row;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const long long row = i / per_row;
+        const int c = (int)(i - row * per_row);
+        float f[8];
+        load_bf16<8>(a + i * 8, f);
+        const float gate = 1.0f / (1.0f + expf(-z[row * z_ld + z_col + c / V8]));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = f[e] * gate * scale;
+        store_bf16<8>(out + row * out_ld + c * 8, f);
+    }
+}
+
 extern "C" {
 
 int sb_conv_qk_store(int dtype, const void* q, long long q_ld, const void* k, long long k_ld, const float* q_bias, const float* k_bias,
@@ -139,7 +261,17 @@ int sb_conv_qk_store(int dtype, const void* q, long long q_ld, const void* k, lo
     dim3 grid(batch.n_rows, per_row);
     const size_t smem = (size_t)D * sizeof(float);
     typedef __nv_bfloat16 bf;
-    if (dtype == SB_F32)
+    // below 128 rows the blocks per head of the kernel above reach more SMs
+    const bool runs = dtype == SB_BF16 && conv && taps <= 4 && (D == 64 || D == 128) && batch.n_rows >= 128 && q_ld % 4 == 0 && k_ld % 4 == 0
+                      && p.v_row % 4 == 0 && sb_aligned(8, q, k, q_out, p.k, p.v);
+    const dim3 run_grid((batch.n_rows + CQ_RUN - 1) / CQ_RUN, (units + 3) / 4);
+    if (runs && D == 64)
+        sb_launch(conv_qk_rows_kernel<2>, run_grid, 128, 0, stream, (const bf*)q, q_ld, (const bf*)k, k_ld, q_bias, k_bias, q_conv, k_conv, taps,
+                  (const float*)state, state_slot, q_norm, k_norm, eps, temp_coef, temp_every, (bf*)q_out, batch, p, H, status);
+    else if (runs)
+        sb_launch(conv_qk_rows_kernel<4>, run_grid, 128, 0, stream, (const bf*)q, q_ld, (const bf*)k, k_ld, q_bias, k_bias, q_conv, k_conv, taps,
+                  (const float*)state, state_slot, q_norm, k_norm, eps, temp_coef, temp_every, (bf*)q_out, batch, p, H, status);
+    else if (dtype == SB_F32)
         sb_launch(conv_qk_store_kernel<float>, grid, threads, smem, stream, (const float*)q, q_ld, (const float*)k, k_ld, q_bias, k_bias,
                   q_conv, k_conv, taps, (const float*)state, state_slot, q_norm, k_norm, eps, temp_coef, temp_every, (float*)q_out, batch,
                   p, H, status);
@@ -168,6 +300,9 @@ int sb_head_gate(int dtype, const void* a, const float* z, long long z_ld, int z
     if (dtype == SB_F32)
         sb_launch(head_gate_kernel<float>, blocks, 256, 0, stream, (const float*)a, z, z_ld, z_col, (float*)out, out_ld, (long long)rows,
                   H, V, scale);
+    else if (V % 8 == 0 && out_ld % 8 == 0 && sb_aligned(16, a, out))
+        sb_launch(head_gate_vec_kernel, (int)((n / 8 + 255) / 256 < 8192 ? (n / 8 + 255) / 256 : 8192), 256, 0, stream, (const __nv_bfloat16*)a, z,
+                  z_ld, z_col, (__nv_bfloat16*)out, out_ld, (long long)rows, H, V / 8, scale);
     else
         sb_launch(head_gate_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const __nv_bfloat16*)a, z, z_ld, z_col, (__nv_bfloat16*)out,
                   out_ld, (long long)rows, H, V, scale);

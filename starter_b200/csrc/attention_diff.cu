@@ -72,6 +72,120 @@ __global__ void rotate_store_kernel(const T* __restrict__ q, long long q_row, co
     }
 }
 
+#define RS_ROWS 4
+
+// Many bfloat16 rows: RS_ROWS rows per block, their sines and cosines taken once, 16 bytes of a head per thread and turn (of a
+// turned head with `halves` the two pieces whose columns turn together).  A number a thread, with the sines taken again by each of
+// a row's four blocks: 4,599 rows of 20 heads of 64 and 128 values 29 us, this 12; 3,333 of 24 heads of 128 and 512 values 47, this 17.
+__global__ void __launch_bounds__(256)
+rotate_store_rows_kernel(const __nv_bfloat16* __restrict__ q, long long q_row, const __nv_bfloat16* __restrict__ k, long long k_row,
+                         const __nv_bfloat16* __restrict__ v, long long v_row, __nv_bfloat16* __restrict__ q_out, SbBatch batch, SbFlex p,
+                         const float* __restrict__ freqs, int rot, float mag, int halves, int nq, int* status) {
+    typedef __nv_bfloat16 bf;
+    extern __shared__ float trig[];       // [RS_ROWS][rot]: cosines, then sines
+    __shared__ int slot_s[RS_ROWS], pos_s[RS_ROWS];
+    pdl_wait();
+    const int row0 = blockIdx.x * RS_ROWS, nr = min(RS_ROWS, batch.n_rows - row0), D = p.k_dim, half = rot >> 1;
+    if (threadIdx.x < nr) row_place(batch, row0 + threadIdx.x, slot_s[threadIdx.x], pos_s[threadIdx.x]);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nr * half; e += blockDim.x) {
+        const int r = e / half, i = e - r * half;
+        float s, c;
+        sincosf((float)pos_s[r] * freqs[i], &s, &c);
+        trig[r * rot + i] = c * mag;
+        trig[r * rot + half + i] = s * mag;
+    }
+    __syncthreads();
+    const int vh = p.v_heads > 0 ? p.v_heads : p.n_kv_heads, per = p.n_kv_heads / vh;
+    const int turned = halves ? half / 8 : rot / 8, pieces = turned + (D - rot) / 8, v_pieces = p.v_dim / 8;
+    const int head_items = (nq + p.n_kv_heads) * pieces, items = head_items + vh * v_pieces;
+    for (int it = threadIdx.x; it < nr * items; it += blockDim.x) {
+        const int r = it / items, i = it - r * items, row = row0 + r, slot = slot_s[r], pos = pos_s[r];
+        if (i >= head_items) {
+            const int h = (i - head_items) / v_pieces, c = (i - head_items - h * v_pieces) * 8;
+            const long long tok = flex_value_token(p, flex_token(p, slot, pos, h * per), h * per);
+            if (tok >= 0)
+                *reinterpret_cast<uint4*>((bf*)p.v + tok * p.v_row + c) = *reinterpret_cast<const uint4*>(v + row * v_row + (long long)h * p.v_dim + c);
+            continue;
+        }
+        const int u = i / pieces, c = i - u * pieces;
+        const bf* src;
+        bf* dst;
+        if (u < nq) {
+            src = q + row * q_row + (long long)u * D;
+            dst = q_out + ((long long)row * nq + u) * D;
+        } else {
+            const long long tok = flex_token(p, slot, pos, u - nq);
+            if (tok < 0) {
+                atomicOr(status, SB_STATUS_NO_PAGE);
+                continue;
+            }
+            src = k + row * k_row + (long long)(u - nq) * D;
+            dst = (bf*)p.k + tok * D;
+        }
+        if (c >= turned) {
+            const int at = rot + (c - turned) * 8;
+            *reinterpret_cast<uint4*>(dst + at) = *reinterpret_cast<const uint4*>(src + at);
+            continue;
+        }
+        const float* cs = trig + r * rot;
+        const float* sn = cs + half;
+        float x[8], y[8];
+        load_bf16<8>(src + c * 8, x);
+        if (halves) {
+            float a[8], b[8];
+            load_bf16<8>(src + half + c * 8, y);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                a[e] = x[e] * cs[c * 8 + e] - y[e] * sn[c * 8 + e];
+                b[e] = y[e] * cs[c * 8 + e] + x[e] * sn[c * 8 + e];
+            }
+            store_bf16<8>(dst + c * 8, a);
+            store_bf16<8>(dst + half + c * 8, b);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                y[2 * e] = x[2 * e] * cs[c * 4 + e] - x[2 * e + 1] * sn[c * 4 + e];
+                y[2 * e + 1] = x[2 * e + 1] * cs[c * 4 + e] + x[2 * e] * sn[c * 4 + e];
+            }
+            store_bf16<8>(dst + c * 8, y);
+        }
+    }
+}
+
+// diff_combine in bfloat16 with heads of 32 N values, N of them a lane and access: 4,599 rows of 8 heads of 64, a number a lane 14
+// us, this 9; 3,333 rows of 8 heads of 128 with a gate 16, this 11.
+template <int N>
+__global__ void diff_combine_vec_kernel(const __nv_bfloat16* __restrict__ a, __nv_bfloat16* __restrict__ out, int rows, int H, int G, float lam,
+                                        float eps, float post, const __nv_bfloat16* __restrict__ gate, long long gate_ld) {
+    constexpr int V = 32 * N;
+    pdl_wait();
+    const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (wid >= (long long)rows * H) return;
+    const long long row = wid / H;
+    const int h = (int)(wid % H), per = H / G, g = h / per, r = h % per;
+    float x[N], y[N], ss = 0.f;
+    load_bf16<N>(a + ((row * 2 * H) + (long long)(2 * g) * per + r) * V + lane * N, x);
+    load_bf16<N>(a + ((row * 2 * H) + (long long)(2 * g + 1) * per + r) * V + lane * N, y);
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+        x[e] = fmaf(-lam, y[e], x[e]);
+        ss = fmaf(x[e], x[e], ss);
+    }
+    ss = warp_sum(ss);
+    const float mul = post / sqrtf(ss / (float)V + eps);
+    if (gate != nullptr) {
+        load_bf16<N>(gate + row * gate_ld + (long long)h * V + lane * N, y);
+#pragma unroll
+        for (int e = 0; e < N; ++e) x[e] = x[e] * mul / (1.0f + expf(-y[e]));
+    } else {
+#pragma unroll
+        for (int e = 0; e < N; ++e) x[e] *= mul;
+    }
+    store_bf16<N>(out + (row * H + h) * V + lane * N, x);
+}
+
 // One warp per (row, head).  a [rows, 2 H, V] holds the maps in the order (key/value head, map, head of the group).
 template <class T>
 __global__ void diff_combine_kernel(const T* __restrict__ a, T* __restrict__ out, int rows, int H, int G, int V, float lam, float eps,
@@ -114,6 +228,14 @@ int sb_rotate_store(int dtype, const void* q, long long q_row, const void* k, lo
     const int per_row = batch.n_rows >= 1024 ? min(units, 4) : (batch.n_rows >= 128 ? min(units, 8) : min(units, 64));
     dim3 grid(batch.n_rows, per_row);
     const size_t smem = (size_t)rot * sizeof(float);
+    // below 128 rows the blocks per head of the kernel above reach more SMs than blocks of four rows would
+    if (dtype == SB_BF16 && batch.n_rows >= 128 && p.k_dim % 8 == 0 && p.v_dim % 8 == 0 && p.v_row % 8 == 0 && rot % (halves ? 16 : 8) == 0
+        && q_row % 8 == 0 && k_row % 8 == 0 && v_row % 8 == 0 && rot <= 1024 && sb_aligned(16, q, k, v, q_out, p.k, p.v)) {
+        typedef __nv_bfloat16 bf;
+        sb_launch(rotate_store_rows_kernel, (batch.n_rows + RS_ROWS - 1) / RS_ROWS, 256, RS_ROWS * smem, stream, (const bf*)q, q_row, (const bf*)k,
+                  k_row, (const bf*)v, v_row, (bf*)q_out, batch, p, freqs, rot, mag, halves, nq, status);
+        SB_LAUNCH_CHECK();
+    }
     if (dtype == SB_F32)
         sb_launch(rotate_store_kernel<float>, grid, threads, smem, stream, (const float*)q, q_row, (const float*)k, k_row,
                   (const float*)v, v_row, (float*)q_out, batch, p, freqs, rot, mag, halves, nq, status);
@@ -131,7 +253,14 @@ int sb_diff_combine(int dtype, const void* a, void* out, int rows, int H, int G,
     const long long warps = (long long)rows * H;
     const int threads = 128;
     const unsigned int blocks = (unsigned int)((warps * 32 + threads - 1) / threads);
-    if (dtype == SB_F32)
+    typedef __nv_bfloat16 bf;
+    if (dtype == SB_BF16 && V == 64 && gate_ld % 2 == 0 && sb_aligned(4, a, out, gate))
+        sb_launch(diff_combine_vec_kernel<2>, blocks, threads, 0, stream, (const bf*)a, (bf*)out, rows, H, G, lam, eps, post, (const bf*)gate,
+                  gate_ld);
+    else if (dtype == SB_BF16 && V == 128 && gate_ld % 4 == 0 && sb_aligned(8, a, out, gate))
+        sb_launch(diff_combine_vec_kernel<4>, blocks, threads, 0, stream, (const bf*)a, (bf*)out, rows, H, G, lam, eps, post, (const bf*)gate,
+                  gate_ld);
+    else if (dtype == SB_F32)
         sb_launch(diff_combine_kernel<float>, blocks, threads, 0, stream, (const float*)a, (float*)out, rows, H, G, V, lam, eps, post,
                   (const float*)gate, gate_ld);
     else

@@ -101,6 +101,40 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// N (2, 4 or 8) neighbouring bfloat16 numbers in one access, as floats; the address is a multiple of N numbers.
+template <int N> __device__ __forceinline__ void load_bf16(const __nv_bfloat16* p, float (&f)[N]) {
+    unsigned int w[N / 2];
+    if (N == 8) {
+        const uint4 v = *reinterpret_cast<const uint4*>(p);
+        w[0] = v.x, w[1 % (N / 2)] = v.y, w[2 % (N / 2)] = v.z, w[3 % (N / 2)] = v.w;
+    } else if (N == 4) {
+        const uint2 v = *reinterpret_cast<const uint2*>(p);
+        w[0] = v.x, w[1 % (N / 2)] = v.y;
+    } else {
+        w[0] = *reinterpret_cast<const unsigned int*>(p);
+    }
+#pragma unroll
+    for (int e = 0; e < N / 2; ++e) {
+        f[2 * e] = __uint_as_float(w[e] << 16);
+        f[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+    }
+}
+template <int N> __device__ __forceinline__ void store_bf16(__nv_bfloat16* p, const float (&f)[N]) {
+    unsigned int w[N / 2];
+#pragma unroll
+    for (int e = 0; e < N / 2; ++e) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+        w[e] = *reinterpret_cast<const unsigned int*>(&v);
+    }
+    if (N == 8) *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1 % (N / 2)], w[2 % (N / 2)], w[3 % (N / 2)]);
+    else if (N == 4) *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1 % (N / 2)]);
+    else *reinterpret_cast<unsigned int*>(p) = w[0];
+}
+// Whether every address given is a multiple of `bytes` (a power of two).
+template <class... P> static inline bool sb_aligned(size_t bytes, const P*... p) {
+    return (((reinterpret_cast<size_t>(p) | ...) & (bytes - 1)) == 0);
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.  `red` holds 33 floats.
 __device__ __forceinline__ float block_sum(float v, float* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = (blockDim.x + 31) >> 5;

@@ -1,0 +1,118 @@
+"""Row kernels that take 16 bytes a thread for long steps, beside the kernels that take a number a thread: the same rows in one
+step of three sequences and in steps of fewer than 128 rows must leave the same outputs, cache rows and records.  Both compute
+in 32 bits and differ in the order of one sum over a head, 2^-22 of it, so a bfloat16 result may differ by one rounding (2^-7)."""
+
+import pytest
+import torch
+
+from starter_b200.cache import Cache, KVRequest, StateRequest
+from test_nifalorn_gpu import context, runtime
+
+pytestmark = pytest.mark.gpu
+LENGTHS = [141, 2, 77]
+
+
+def rand(shape, seed, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).cuda()
+
+
+def same(a, b, what):
+    assert a.shape == b.shape and bool(torch.isfinite(a.float()).all()), what
+    d = (a.float() - b.float()).abs()
+    assert bool((d <= 2.0 ** -7 * b.float().abs() + 1e-6).all()), f"{what}: {float(d.max())}"
+
+
+def both_ways(requests, call):
+    """call(ops, ctx, layer cache, first row of the piece, one past its last row) for one step of all sequences, and for pieces
+    of each: [(outputs, cache)] of both."""
+    rt = runtime("bfloat16")
+    res = []
+    for whole in (True, False):
+        cache = Cache([requests], n_slots=4, max_tokens=64 * 16, dtype=rt.dtype, device="cuda")
+        cache.alloc()
+        slots = [cache.alloc() for _ in LENGTHS]
+        starts = [sum(LENGTHS[:i]) for i in range(len(LENGTHS))]
+        outs = [None] * len(LENGTHS)
+        steps = [list(zip(slots, LENGTHS))] if whole else [[(s, min(100, n - at))] for s, n in zip(slots, LENGTHS) for at in range(0, n, 100)]
+        done = dict.fromkeys(slots, 0)
+        for step in steps:
+            ctx = context(rt, cache, [s for s, _ in step], [n for _, n in step])
+            first = starts[slots.index(step[0][0])] + done[step[0][0]]
+            out = call(rt.ops, ctx, cache.layers[0], first, first + sum(n for _, n in step))
+            rt.ops.advance_lengths(ctx)
+            at = 0
+            for s, n in step:
+                i = slots.index(s)
+                outs[i] = out[at:at + n] if outs[i] is None else torch.cat([outs[i], out[at:at + n]])
+                cache.advance_host(s, n)
+                done[s] += n
+                at += n
+            assert int(ctx.status.item()) == 0
+        res.append((torch.cat(outs), cache))
+    return res
+
+
+@pytest.mark.parametrize("D, V, nq, G, vh, rot, halves", [(64, 128, 8, 4, 2, 64, True), (128, 128, 6, 2, 1, 64, True), (128, 64, 3, 3, 3, 16, True),
+                                                          (64, 64, 4, 2, 2, 64, False), (24, 8, 5, 1, 1, 8, False), (72, 40, 2, 2, 2, 48, True),
+                                                          (64, 64, 2, 2, 1, 0, True), (40, 16, 2, 1, 1, 24, True)])
+def test_rotated_rows(D, V, nq, G, vh, rot, halves):
+    rows = sum(LENGTHS)
+    p = rand((rows, nq * D + G * D + vh * V + 8), 1).bfloat16()
+    freqs = torch.tensor([10000.0 ** (-2.0 * i / max(rot, 1)) for i in range(rot // 2)], dtype=torch.float32, device="cuda") if rot else None
+    request = KVRequest(num_kv_heads=G, head_dim=D, v_dim=V, v_heads=vh)
+
+    def call(ops, ctx, lc, a, b):
+        x = p[a:b]
+        return ops.rotate_store(ctx, x[:, :nq * D].unflatten(1, (nq, D)), x[:, nq * D:(nq + G) * D].unflatten(1, (G, D)),
+                                x[:, (nq + G) * D:(nq + G) * D + vh * V], lc, freqs, rot, 1.1, halves)
+    (o1, c1), (o2, c2) = both_ways(request, call)
+    same(o1, o2, "queries")
+    same(c1.layers[0].k, c2.layers[0].k, "keys")
+    assert torch.equal(c1.layers[0].v, c2.layers[0].v)
+
+
+@pytest.mark.parametrize("D, H, G, taps, bias, norm", [(128, 5, 2, 4, True, True), (64, 4, 4, 3, False, True), (128, 2, 1, 2, True, False),
+                                                       (64, 1, 1, 1, True, True), (64, 3, 1, 4, True, True)])
+def test_convolved_rows(D, H, G, taps, bias, norm):
+    rows = sum(LENGTHS)
+    p = rand((rows, (H + G) * D + 4), 2).bfloat16()
+    w = dict(q_bias=rand((H * D,), 3, 0.2) if bias else None, k_bias=rand((G * D,), 4, 0.2) if bias else None,
+             q_conv=rand((H * D, taps), 5, 0.5), k_conv=rand((G * D, taps), 6, 0.5),
+             q_norm=rand((D,), 7) if norm else None, k_norm=rand((D,), 8) if norm else None)
+    kv = KVRequest(num_kv_heads=G, head_dim=D, v_dim=D)
+    request = (kv, StateRequest((taps - 1, (H + G) * D))) if taps > 1 else kv
+
+    def call(ops, ctx, lc, a, b):
+        x = p[a:b]
+        return ops.conv_qk_store(ctx, x[:, :H * D], x[:, H * D:(H + G) * D], lc, lc.aux.state if taps > 1 else None, H, w["q_bias"], w["k_bias"],
+                                 w["q_conv"], w["k_conv"], w["q_norm"], w["k_norm"], 1e-5, 0.2, 16)
+    (o1, c1), (o2, c2) = both_ways(request, call)
+    same(o1, o2, "queries")
+    same(c1.layers[0].k, c2.layers[0].k, "keys")
+    same(c1.layers[0].v, c2.layers[0].v, "keys before the norm")
+    if taps > 1:
+        assert torch.equal(c1.layers[0].aux.state, c2.layers[0].aux.state)
+
+
+@pytest.mark.parametrize("V", [64, 128, 40, 12])
+@pytest.mark.parametrize("pad", [0, 3, 8])
+def test_rows_that_are_joined_gated_and_biased(V, pad):
+    """Widths and strides that the 16-byte kernels take and ones that they do not, against the formula in 64 bits."""
+    ops, rows, H, G = runtime("bfloat16").ops, 37, 4, 2
+    a, gate = rand((rows, 2 * H * V), 11).bfloat16(), rand((rows, H * V + pad), 12).bfloat16()
+    x = a.double().reshape(rows, G, 2, H // G, V)
+    o = x[:, :, 0] - 0.3 * x[:, :, 1]
+    o = (o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-5) * 0.5).reshape(rows, H * V)
+    for g in (None, gate[:, :H * V]):
+        want = o if g is None else o * torch.sigmoid(g.double())
+        got = ops.diff_combine(a, H, G, V, 0.3, 1e-5, 0.5, gate=g).double()
+        assert float((got - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
+    z, b = rand((rows, H + pad), 13), rand((H * V,), 14)
+    y = a[:, :H * V].contiguous()
+    wide = torch.zeros((rows, H * V + pad), dtype=torch.bfloat16, device="cuda")
+    got = ops.head_gate(y, z, pad, H, 0.7, out=wide[:, :H * V]).double()
+    want = y.double() * torch.sigmoid(z[:, pad:].double()).repeat_interleave(V, 1) * 0.7
+    assert float((got - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
+    want = y.double() + b.double()
+    assert float((ops.add_bias(y.clone(), b).double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
+    assert torch.equal(ops.relu2(y), (torch.relu(y.float()) ** 2).bfloat16())
