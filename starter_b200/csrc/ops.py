@@ -193,6 +193,8 @@ class Ops:
             "sb_moe_gather": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
             "sb_moe_pairs": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                              c_float, c_float, c_int, c_void_p],
+            "sb_moe_few": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
+                           c_int, c_void_p],
             "sb_moe_combine": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                c_int, c_void_p, c_int, c_void_p],
             "sb_chunk_memory": [c_int, SbChunkMem, SbBatch, c_void_p],
@@ -1644,12 +1646,26 @@ class Ops:
 
     MOE_PAIRS_MAX = int(os.environ.get("STARTER_B200_MOE_PAIRS_MAX", 64))   # pairs up to which every pair streams its expert
 
+    MOE_FEW_MAX = int(os.environ.get("STARTER_B200_MOE_FEW_MAX", 512))   # pairs up to which moe_few.cu serves a step
+
+    def _moe_takes_few(self, h, pairs, n_experts, width, ff, w_gate_up, w_down) -> bool:
+        """The kernel of an expert at a time (moe_few.cu).  With fewer pairs than experts hardly two pairs share one, and a
+        block per pair is ahead (up to the 64 pairs it is built for); beyond some 32 pairs an expert the weights are read too
+        often and the grouped product is.  Measured (us a layer, pair by pair / this / grouped): 16 experts of 3 x 1,024 x 512: 8
+        pairs 13 / 14 / 38, 16: 18 / 16 / 39, 64: 39 / 20 / 41, 96: 52 / 21 / 42, 256: - / 28 / 42, 512: - / 39 / 42, 768: - / 51 /
+        43; 32 of 3 x 2,048 x 1,024: 16 pairs 40 / 42 / 72, 32: 57 / 53 / 92, 64: 110 / 65 / 96, 96: 157 / 78 / 114, 512: - / 113 /
+        123, 768: - / 150 / 120."""
+        if self.MOE_FEW_MAX < pairs or pairs > 32 * n_experts or pairs < min(n_experts, self.MOE_PAIRS_MAX + 1):
+            return False
+        return (h.dtype == torch.bfloat16 and width % 32 == 0 and ff % 32 == 0 and h.is_contiguous() and h.data_ptr() % 16 == 0
+                and w_gate_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
+
     def moe_experts(self, h, chosen, weight, w_gate_up, w_down, n_experts, alpha, limit, base, base_gate=None):
         """base (times sigmoid(base_gate), 32-bit [rows, 1], when given) + sum_k weight[:, k] * expert_chosen[:, k](h): experts are gated feed-forwards (the clamped activation with
         its sigmoid factor ``alpha`` and ``limit``, or silu(gate) * up when ``alpha`` is None) with stacked
         matrices w_gate_up [experts, 2 ff, width] (gate over up) and w_down [experts, width, ff]; a choice >= n_experts
-        is an identity output and adds weight * h.  A few pairs: each pair streams its expert's matrices (this library's
-        kernels).  Many pairs in bfloat16: the pairs are put in the order of their experts on the device and each matrix
+        is an identity output and adds weight * h.  A few pairs: each pair streams its expert's matrices; some hundreds: every
+        expert's matrices are read once for its pairs (this library's kernels).  Many pairs in bfloat16: the pairs are put in the order of their experts on the device and each matrix
         takes one grouped product of the vendor's library, as the plain products of a prompt do."""
         rows, width = h.shape
         top = chosen.shape[1]
@@ -1661,7 +1677,15 @@ class Ops:
             if (tuple(w_gate_up.shape) != (n_experts, 2 * ff, width) or tuple(w_down.shape) != (n_experts, width, ff)
                     or not w_gate_up.is_contiguous() or not w_down.is_contiguous() or w_gate_up.dtype != h.dtype):
                 raise KernelError("moe_experts: stacked matrices [experts, 2 ff, width] and [experts, width, ff] in the run's dtype")
-            if (h.dtype == torch.bfloat16 and pairs > self.MOE_PAIRS_MAX and width % 8 == 0 and ff % 8 == 0
+            few = self._moe_takes_few(h, pairs, n_experts, width, ff, w_gate_up, w_down)
+            if few:
+                act = torch.empty((pairs, ff), dtype=h.dtype, device=h.device)
+                down = torch.empty((pairs, width), dtype=h.dtype, device=h.device)
+                self._check(self.lib.sb_moe_few(_ptr(h), _ptr(chosen), _ptr(w_gate_up), _ptr(w_down), _ptr(act), _ptr(down), pairs, top,
+                                                n_experts, width, ff, float(alpha or 0.0), float(limit or 0.0), int(alpha is None),
+                                                self._stream()), "moe_few")
+                self.launches += 1
+            elif (h.dtype == torch.bfloat16 and pairs > self.MOE_PAIRS_MAX and width % 8 == 0 and ff % 8 == 0
                     and hasattr(torch, "_grouped_mm")):
                 ends = torch.empty(n_experts, dtype=torch.int32, device=h.device)
                 slot_of_pair = torch.empty(pairs, dtype=torch.int32, device=h.device)
