@@ -22,6 +22,7 @@ from .build import BuildError, load
 
 F32, BF16 = 0, 1
 _RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)   # (device index) -> cudaStream_t as an int
+_DEVICE = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)   # without current_device's own look at whether CUDA is up
 
 
 class KernelError(RuntimeError):
@@ -83,7 +84,7 @@ def _code(dtype: torch.dtype) -> int:
 
 
 def _ptr(t):
-    return None if t is None else c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()   # ctypes makes the pointer; an object of its own costs the host as much again
 
 
 class Ops:
@@ -262,8 +263,8 @@ class Ops:
         Stream object and costs the host ~14 us a call (measured: a quarter of the host's time in an eager step);
         the raw query is a fraction of a microsecond."""
         if _RAW_STREAM is not None:
-            return c_void_p(_RAW_STREAM(torch.cuda.current_device()))
-        return c_void_p(torch.cuda.current_stream().cuda_stream)
+            return _RAW_STREAM(_DEVICE())
+        return torch.cuda.current_stream().cuda_stream
 
     def _check(self, code: int, what: str) -> None:
         self.launches += 1
