@@ -16,8 +16,9 @@
 // their own and a second kernel adds them up in order (`SPLIT`).
 // Measured (B200, 32-bit; the kernel before had one tile of 64 x 64 with scalar loads: 12 TFLOP/s at 300 rows): 300 rows of
 // [6144, 2560] 245 us (38 TFLOP/s), [2560, 4096] 196, [19456, 2560] 759, [2560, 9728] 382; 2,048 rows of [19456, 2560] 4.06 ms
-// (50 TFLOP/s); one row of [151936, 2560] 456 us (3.4 TB/s); 300 rows' error against 64 bits 4.1e-7.
+// (50 TFLOP/s); one row of [151936, 2560] 275 us (5.7 TB/s); 300 rows' error against 64 bits 4.1e-7.
 #include "common.cuh"
+#include "mma_utils.cuh"
 
 #define GG_BK 16
 #define GG_CHUNK 512   // columns of k per running sum; a multiple of GG_BK
@@ -174,6 +175,108 @@ gemm_general_kernel(const TA* __restrict__ A, const TA* __restrict__ W, TO* __re
     }
 }
 
+#define GR_BK 32        // columns of k per stage: a whole line of every weight row
+#define GR_LD (GR_BK + 4)
+#define GR_COLS 128     // weight rows (output columns) per block, one per thread
+#define GR_STAGES 4
+
+// Up to MR <= 8 rows of 32-bit activations: the weights stream through shared memory, a line of each of the block's 128 rows per
+// stage and three stages on their way, a thread owns one output column with all rows; the sums run in the order of the
+// kernel above.  Bound: the weights' bytes.  A tile of 8 rows of the kernel above fetched half a line a row and one stage ahead:
+// one row of [151936, 2560], 1,556 MB, 456 us (3.4 TB/s), this 275
+// (5.7 TB/s).
+template <int MR>
+__global__ void __launch_bounds__(GR_COLS) gemm_general_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
+                                                                    int M, int N, int K, int split) {
+    extern __shared__ __align__(16) float gr_sm[];    // [GR_STAGES] of W [GR_COLS][GR_LD] and A [MR][GR_BK]
+    constexpr int STAGE = GR_COLS * GR_LD + MR * GR_BK, PM = MR / 2;
+    const int tid = threadIdx.x, n0 = blockIdx.x * GR_COLS;
+    const int k_first = split ? blockIdx.z * GG_CHUNK : 0, k_last = split ? min(K, k_first + GG_CHUNK) : K;
+    const int turns = (k_last - k_first + GR_BK - 1) / GR_BK;
+    auto copy = [](float* dst, const float* src, bool ok) {
+        const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
+        const int n = ok ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n));
+    };
+    auto fetch_w = [&](int turn) {
+        float* ws = gr_sm + (turn % GR_STAGES) * STAGE;
+        const int k0 = k_first + turn * GR_BK;
+#pragma unroll
+        for (int e = 0; e < GR_COLS * GR_BK / 4 / GR_COLS; ++e) {
+            const int i = tid + e * GR_COLS, r = i / (GR_BK / 4), c = (i % (GR_BK / 4)) * 4;
+            const bool ok = n0 + r < N && k0 + c < k_last;
+            copy(ws + r * GR_LD + c, ok ? W + (long long)(n0 + r) * K + k0 + c : W, ok);
+        }
+    };
+    auto fetch_a = [&](int turn) {
+        if (tid >= MR * GR_BK / 4) return;
+        const int r = tid / (GR_BK / 4), c = (tid % (GR_BK / 4)) * 4, k = k_first + turn * GR_BK + c;
+        const bool ok = r < M && k < k_last;
+        copy(gr_sm + (turn % GR_STAGES) * STAGE + GR_COLS * GR_LD + r * GR_BK + c, ok ? A + (long long)r * K + k : A, ok);
+    };
+    float2 acc[PM], total[PM];
+#pragma unroll
+    for (int i = 0; i < PM; ++i) acc[i] = total[i] = make_float2(0.f, 0.f);
+    for (int t = 0; t < GR_STAGES - 1 && t < turns; ++t) fetch_w(t);   // weights: they do not depend on the kernel before
+    pdl_wait();
+    for (int t = 0; t < GR_STAGES - 1 && t < turns; ++t) fetch_a(t);
+    cp_async_commit();
+    for (int t = 1; t < GR_STAGES - 1; ++t) cp_async_commit();         // a group per turn from here on
+    for (int turn = 0; turn < turns; ++turn) {
+        if (turn == 0) cp_async_wait<0>();
+        else cp_async_wait<GR_STAGES - 2>();
+        __syncthreads();
+        if (turn + GR_STAGES - 1 < turns) {
+            fetch_w(turn + GR_STAGES - 1);
+            fetch_a(turn + GR_STAGES - 1);
+        }
+        cp_async_commit();
+        const float* ws = gr_sm + (turn % GR_STAGES) * STAGE + tid * GR_LD;
+        const float* as = gr_sm + (turn % GR_STAGES) * STAGE + GR_COLS * GR_LD;
+#pragma unroll
+        for (int c = 0; c < GR_BK; c += 4) {
+            const float4 w4 = *reinterpret_cast<const float4*>(ws + c);
+            const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+            float4 a4[MR];
+#pragma unroll
+            for (int i = 0; i < MR; ++i) a4[i] = *reinterpret_cast<const float4*>(as + i * GR_BK + c);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int i = 0; i < PM; ++i) {
+                    const float4 x = a4[2 * i], y = a4[2 * i + 1];
+                    const float2 a = kk == 0 ? make_float2(x.x, y.x) : kk == 1 ? make_float2(x.y, y.y) : kk == 2 ? make_float2(x.z, y.z) : make_float2(x.w, y.w);
+                    acc[i] = fma_pair(a, make_float2(w[kk], w[kk]), acc[i]);
+                }
+        }
+        if (((turn + 1) * GR_BK) % GG_CHUNK == 0 || turn + 1 == turns) {
+#pragma unroll
+            for (int i = 0; i < PM; ++i) {
+                total[i] = add_pair(total[i], acc[i]);
+                acc[i] = make_float2(0.f, 0.f);
+            }
+        }
+    }
+    const int n = n0 + tid;
+    if (n >= N) return;
+    float* out = C + (split ? (long long)blockIdx.z * M * N : 0ll);
+#pragma unroll
+    for (int i = 0; i < PM; ++i) {
+        if (2 * i < M) out[(long long)(2 * i) * N + n] = total[i].x;
+        if (2 * i + 1 < M) out[(long long)(2 * i + 1) * N + n] = total[i].y;
+    }
+}
+
+template <int MR>
+static int gr_launch(const float* A, const float* W, float* C, int M, int N, int K, int split, cudaStream_t stream) {
+    constexpr int smem = GR_STAGES * (GR_COLS * GR_LD + MR * GR_BK) * (int)sizeof(float);
+    const cudaError_t err = cudaFuncSetAttribute(gemm_general_rows_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err != cudaSuccess) return (int)err;
+    sb_launch(gemm_general_rows_kernel<MR>, dim3((N + GR_COLS - 1) / GR_COLS, 1, split ? (K + GG_CHUNK - 1) / GG_CHUNK : 1), GR_COLS, smem, stream, A, W,
+              C, M, N, K, split);
+    return 0;
+}
+
 // The chunks' sums, added in order.
 template <class TO>
 __global__ void __launch_bounds__(256) gemm_general_add_kernel(const float* __restrict__ parts, TO* __restrict__ C, long long count,
@@ -275,7 +378,20 @@ int sb_gemm_general(int dtype, int out_f32, const void* A, const void* W, void* 
     if ((M + 63) / 64 > 65535) return (int)cudaErrorInvalidValue;
     const unsigned long long low = (unsigned long long)A | (unsigned long long)W;
     const int vec = K % 4 == 0 && low % (dtype == SB_F32 ? 16 : 8) == 0;
-    if (dtype == SB_F32) {
+    if (dtype == SB_F32 && M <= 8 && vec) {
+        const float* a = (const float*)A;
+        const float* w = (const float*)W;
+        float* c = parts != nullptr ? parts : (float*)C;
+        const int split = parts != nullptr;
+        const int err = M <= 2 ? gr_launch<2>(a, w, c, M, N, K, split, stream) : M <= 4 ? gr_launch<4>(a, w, c, M, N, K, split, stream)
+                                                                                       : gr_launch<8>(a, w, c, M, N, K, split, stream);
+        if (err) return err;
+        if (split) {
+            const long long count = (long long)M * N, blocks = (count + 255) / 256;
+            sb_launch(gemm_general_add_kernel<float>, dim3((unsigned int)(blocks < 4736 ? blocks : 4736)), 256, 0, stream, (const float*)parts,
+                      (float*)C, count, (K + GG_CHUNK - 1) / GG_CHUNK);
+        }
+    } else if (dtype == SB_F32) {
         gg_pick<float, float>(A, W, C, M, N, K, parts, vec, stream);
     } else if ((long long)M * N <= 4096) {
         const dim3 grid((unsigned int)(((long long)M * N + 7) / 8));

@@ -67,3 +67,17 @@ def test_attention_32_bit(ops, D, G, Gk, window):
             sc = (qs[:, h] @ k[h // G].T * D ** -0.5).masked_fill(~seen, -math.inf)
             want = torch.softmax(sc, -1) @ v[h // G]
             assert float((got[cu[b]:cu[b + 1]].view(n, H, D)[:, h] - want).abs().max()) < 2e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("M", [2, 3, 4, 5, 7, 8])
+@pytest.mark.parametrize("N, K", [(127, 20), (128, 512), (300, 516), (1000, 2560)])
+def test_product_32_bit_of_a_few_rows(ops, M, N, K):
+    """The weight-streaming kernel: ragged columns, a last stage that is cut short, chunks of k in one block and side by side, and
+    weights that are not 16-byte aligned (the general tiles); every row as the tiles of many rows leave it."""
+    a, w = rand((M, K), 1), rand((N, K), 2) * K ** -0.5
+    got = ops.linear(a, w)
+    want = a.double() @ w.double().T
+    assert float((got - want).norm() / want.norm()) < 1e-6
+    assert torch.equal(ops.linear(torch.cat([a, rand((60, K), 3)]), w)[:M], got)
+    shifted = torch.empty(N * K + 1, device="cuda")[1:].view(N, K).copy_(w)
+    assert torch.equal(ops.linear(a, shifted), got)
