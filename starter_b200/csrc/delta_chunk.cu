@@ -364,6 +364,33 @@ __global__ void delta_chunk_finish_kernel(const float* __restrict__ o_raw, SbDel
     for (int c = lane; c < V; c += 32) y[wid * V + c] = from_f<T>(o[c] * rstd * p.norm[c] * (1.0f / (1.0f + expf(-gate[c]))));
 }
 
+// The same for heads of 64 or 128 values (LANES 16 or 32 of four each), 16 bytes a lane: Siparax's 3 prompts, 32 heads of 64: a number
+// a lane 51 us, this 19.
+template <int LANES>
+__global__ void __launch_bounds__(256) delta_chunk_finish_vec_kernel(const float* __restrict__ o_raw, SbDelta p, int rows, __nv_bfloat16* __restrict__ y) {
+    pdl_wait();
+    const long long wid = ((long long)blockIdx.x * 256 + threadIdx.x) / LANES;
+    const int c = (threadIdx.x % LANES) * 4, H = p.H;
+    constexpr int V = 4 * LANES;
+    const bool in = wid < (long long)rows * H;
+    const long long row = in ? wid / H : 0;
+    const int head = in ? (int)(wid - row * H) : 0;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f), g = o;
+    if (in) {
+        o = *reinterpret_cast<const float4*>(o_raw + wid * V + c);
+        g = *reinterpret_cast<const float4*>(p.z + row * p.z_ld + (long long)H * p.D + (long long)head * V + c);
+    }
+    float ss = fmaf(o.x, o.x, fmaf(o.y, o.y, fmaf(o.z, o.z, o.w * o.w)));
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    if (!in) return;
+    const float rstd = 1.0f / sqrtf(ss / (float)V + p.eps);
+    const float4 n = *reinterpret_cast<const float4*>(p.norm + c);
+    const float out[4] = {o.x * rstd * n.x * (1.0f / (1.0f + expf(-g.x))), o.y * rstd * n.y * (1.0f / (1.0f + expf(-g.y))),
+                          o.z * rstd * n.z * (1.0f / (1.0f + expf(-g.z))), o.w * rstd * n.w * (1.0f / (1.0f + expf(-g.w)))};
+    store_bf16<4>(y + wid * V + c, out);
+}
+
 template <int CT, int DP>
 static int launch_chunk_scan(SbDelta p, SbBatch batch, const float* ws, float* o_raw, int VP, cudaStream_t stream) {
     const size_t smem = (size_t)(DC_STAGES * (dc_shared_part(DP) + DC * 4 * CT) + 4 * DP * CT + 4 * DC * CT) * sizeof(float);
@@ -404,7 +431,12 @@ int sb_delta_chunk(int dtype, SbDelta p, SbBatch batch, float* ws, float* o_raw,
     if (err) return err;
     const long long warps = (long long)batch.n_rows * p.H;
     const unsigned int blocks = (unsigned int)((warps * 32 + 255) / 256);
-    if (dtype == SB_F32) sb_launch(delta_chunk_finish_kernel<float>, blocks, 256, 0, stream, (const float*)o_raw, p, batch.n_rows, (float*)y);
+    const bool wide = dtype == SB_BF16 && p.z_ld % 4 == 0 && (p.H * p.D) % 4 == 0 && sb_aligned(16, o_raw, p.z, p.norm) && sb_aligned(8, y);
+    if (wide && p.V == 64)
+        sb_launch(delta_chunk_finish_vec_kernel<16>, (unsigned int)((warps + 15) / 16), 256, 0, stream, (const float*)o_raw, p, batch.n_rows, (__nv_bfloat16*)y);
+    else if (wide && p.V == 128)
+        sb_launch(delta_chunk_finish_vec_kernel<32>, (unsigned int)((warps + 7) / 8), 256, 0, stream, (const float*)o_raw, p, batch.n_rows, (__nv_bfloat16*)y);
+    else if (dtype == SB_F32) sb_launch(delta_chunk_finish_kernel<float>, blocks, 256, 0, stream, (const float*)o_raw, p, batch.n_rows, (float*)y);
     else
         sb_launch(delta_chunk_finish_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const float*)o_raw, p, batch.n_rows, (__nv_bfloat16*)y);
     SB_LAUNCH_CHECK();

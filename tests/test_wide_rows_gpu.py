@@ -116,3 +116,50 @@ def test_rows_that_are_joined_gated_and_biased(V, pad):
     want = y.double() + b.double()
     assert float((ops.add_bias(y.clone(), b).double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max())
     assert torch.equal(ops.relu2(y), (torch.relu(y.float()) ** 2).bfloat16())
+
+
+@pytest.mark.parametrize("rows", [1023, 1024, 1500])
+@pytest.mark.parametrize("width", [2048, 2044, 1024, 516, 64, 2052])
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_layer_norms_of_many_rows(rows, width, dtype):
+    """A warp per row from 1,024 rows of up to 2,048 columns on: 32-bit sums, one rounding to the output's type (bfloat16: half a unit
+    in the last of 8 bits, 2^-8 of the value at most; the 32-bit error of the sums, 2e-6, beside it)."""
+    ops, dt = runtime(dtype).ops, getattr(torch, dtype)
+    x, d, w, b = rand((rows, width), 21, 2.0) + 0.5, rand((rows, width), 22).to(dt), rand((width,), 23), rand((width,), 24)
+    for delta in (None, d):
+        y = x.clone()
+        got = ops.layernorm(y, delta, w, b, 1e-5, dt).double()
+        s = x.double() if delta is None else x.double() + d.double()
+        c = s - s.mean(-1, keepdim=True)
+        want = c / torch.sqrt((c * c).mean(-1, keepdim=True) + 1e-5) * w.double() + b.double()
+        assert float((y.double() - s).abs().max()) <= 2.0 ** -23 * float(s.abs().max())
+        assert float((got - want).abs().max()) <= ((2.0 ** -8 if dtype == "bfloat16" else 0.0) + 2e-6) * float(want.abs().max())
+
+
+@pytest.mark.parametrize("D, G, H, taps", [(64, 2, 4, 4), (128, 1, 2, 3), (64, 3, 3, 2)])
+def test_unit_heads_of_many_rows(D, G, H, taps):
+    """Runs of 8 rows from 512 rows on, sequences that begin inside a run and records from an earlier step, beside steps of fewer rows."""
+    ops, C = runtime("bfloat16").ops, (2 * G + H) * D
+    counts = [300, 1, 2, 221]
+    p, w = rand((sum(counts), C + 8), 31).bfloat16(), rand((taps, C), 32, 0.5)
+    inner = rand((sum(counts), 11), 33)
+    state0 = rand((6, taps - 1, C), 34)
+    slots = [4, 0, 3, 1]
+
+    def step(seqs, rows, state):
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+        from types import SimpleNamespace
+        ns = [counts[s] for s in seqs]
+        cu = [sum(ns[:i]) for i in range(len(ns) + 1)]
+        ctx = SimpleNamespace(seq_slot=i32([slots[s] for s in seqs]), cu_q=i32(cu), row_seq=i32([i for i, n in enumerate(ns) for _ in range(n)]),
+                              lengths=i32([0] * 6), n_seqs=len(ns), n_rows=cu[-1], max_q_len=max(ns), cache=SimpleNamespace(null_slot=5), scratch={})
+        return ops.conv_unit_heads(ctx, p[rows, :C], w, state, G, D, 0.3, inner[rows], 7, 16)
+    s1, s2 = state0.clone(), state0.clone()
+    whole = step([0, 1, 2, 3], slice(None), s1)
+    at = 0
+    for i, n in enumerate(counts):
+        part = step([i], slice(at, at + n), s2)
+        assert float((whole[0][at:at + n] - part[0]).abs().max()) <= 1e-6 * float(part[0].abs().max())
+        assert torch.equal(whole[1][at:at + n], part[1])
+        at += n
+    assert torch.equal(s1, s2)
