@@ -1642,7 +1642,8 @@ class Ops:
         self._check(self.lib.sb_moe_route(_code(h.dtype), _ptr(h), _ptr(router), _ptr(correction), _ptr(bias), int(bool(over_chosen)),
                                           _ptr(logits), _ptr(chosen), _ptr(weight), rows, width, n_out, int(top), float(scale),
                                           int(scores == "sigmoid"), int(groups), int(keep_groups), int(extra), self._stream()), "moe_route")
-        self.launches += 1   # logits, then the choice
+        if rows > 64 or n_out > 32 or width > 12288:
+            self.launches += 1   # logits, then the choice; few rows and outputs take both in one kernel
         return (chosen, weight, logits[:, n_out:]) if extra else (chosen, weight)
 
     MOE_PAIRS_MAX = int(os.environ.get("STARTER_B200_MOE_PAIRS_MAX", 64))   # pairs up to which every pair streams its expert

@@ -65,3 +65,32 @@ def test_the_rule_between_pairs_experts_and_grouped_products():
     assert [ops._moe_takes_few(h, n, 300, 64, 64, w, w) for n in (64, 65)] == [False, True]
     assert not ops._moe_takes_few(h.float(), 32, 16, 64, 64, w, w) and not ops._moe_takes_few(h, 32, 16, 64, 40, w, w)
     assert not ops._moe_takes_few(h, 32, 16, 64, 64, w[1:], w)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("n_out, top, groups, keep, extra, mode", [
+    (1, 1, 1, 1, 0, "softmax"), (32, 32, 1, 1, 0, "softmax"), (18, 4, 1, 1, 0, "softmax"), (31, 5, 1, 1, 2, "chosen"), (32, 6, 8, 3, 1, "sigmoid"),
+    (30, 4, 15, 2, 0, "softmax"), (32, 3, 32, 3, 0, "sigmoid"), (9, 2, 3, 1, 1, "sigmoid"), (4, 4, 2, 2, 0, "chosen"),
+])
+def test_routes_of_few_rows_as_of_many(n_out, top, groups, keep, extra, mode, dtype):
+    """Up to 64 rows one kernel takes logits and choice; the two kernels of more rows sum and compare in the same order, so the
+    same rows among 70 must leave the same logits, choices and weights; equal scores go to the lowest output."""
+    from starter_b200.csrc.ops import get_ops
+    ops, width = get_ops(verbose=False), 132
+    g = torch.Generator().manual_seed(5)
+    h = torch.randn(70, width, generator=g).to(getattr(torch, dtype)).cuda()
+    router = torch.randn(n_out + extra, width, generator=g).cuda() * 0.3
+    if n_out > 3:
+        router[3] = router[1]                       # two outputs that are always equal
+    correction = None if n_out % 2 else torch.randn(n_out, generator=g).cuda() * 0.1
+    if correction is not None and n_out > 3:
+        correction[3] = correction[1]
+    bias = torch.randn(n_out, generator=g).cuda() if mode == "chosen" else None
+    kind = dict(over_chosen=mode == "chosen", scores="sigmoid" if mode == "sigmoid" else "softmax", groups=groups, keep_groups=keep, extra=extra)
+    many = ops.moe_route(h, router, correction, top, 1.7, bias=bias, **kind)
+    for rows in (1, 64):
+        few = ops.moe_route(h[:rows].contiguous(), router, correction, top, 1.7, bias=bias, **kind)
+        assert torch.equal(few[0], many[0][:rows])
+        assert float((few[1] - many[1][:rows]).abs().max()) <= 1e-6
+        if extra:
+            assert torch.equal(few[2], many[2][:rows])
