@@ -21,12 +21,6 @@
 // atomic).  With more splits each block leaves its partial result in scratch memory and the last one
 // to arrive (an atomic counter per sequence and kv head) merges them.
 //
-// Order.  When the blocks are more than the GPU holds at once, they are handed out as others end, and a long sequence that starts
-// late is worked on alone at the end.  The (sequence, kv head) pairs are then taken in falling order of the sequences' lengths
-// (up to AD_ORDERED sequences: every block finds its sequence's rank for itself, before it waits for the kernel before it; with
-// more, the blocks are many and short against the whole).  64 sequences of 128 to 2,048 tokens, 8 kv heads of 128: 66 -> 59 us
-// (285 MB: 44 at the copy bandwidth; of equal length the order changes nothing).
-//
 // Fused preparation of q and k (FUSED).  The kernel can take the row of the fused q/k/v projection
 // instead of finished queries: it then applies the per-head RMSNorm and the rotary encoding to its own
 // G query heads (engine/kernels/rope.py:95-144), and the block whose pages hold the new token's
@@ -43,13 +37,12 @@ namespace cg = cooperative_groups;
 #define AD_WARPS 4
 #define AD_KEYS_PER_WARP (SB_PAGE / AD_WARPS)  // 16
 #define AD_MAX_CLUSTER 8
-#define AD_ORDERED 128
 #define AD_MAX_DEVICES 64     // devices whose per-device set-up this file remembers
 
 template <int D, bool FUSED, int AD_STAGES>
 __global__ void __launch_bounds__(AD_WARPS * 32)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ out, SbBatch batch, SbKV kv,
-                   int n_heads, float scale_log2, int window, int n_splits, int cluster_merge, int ordered, float* __restrict__ partial,
+                   int n_heads, float scale_log2, int window, int n_splits, int cluster_merge, float* __restrict__ partial,
                    int* __restrict__ counters, SbFusedQK fused) {
     constexpr int CH = D / 8;                              // 16-byte chunks per row
     constexpr int SLICE = AD_KEYS_PER_WARP * D * 2;        // bytes of one warp's keys (or values) of a page
@@ -64,24 +57,8 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restric
     // the lengths, the page table, the norm weights and rotary tables, and pages before the one that holds
     // the new token.  If that kernel releases this one early, the look-ups and first copies below overlap it.
     sb_stamp(4, 0);
-    const int split = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int seq = blockIdx.x, kvh = blockIdx.y;
-    if (ordered) {
-        __shared__ int s_len[AD_ORDERED], s_seq;
-        const int turn = blockIdx.y * gridDim.x + blockIdx.x, want = turn / kv.n_kv_heads;
-        const int mine = tid < batch.n_seqs ? batch.lengths[batch.seq_slot[tid]] : 0;
-        if (tid < batch.n_seqs) s_len[tid] = mine;
-        __syncthreads();
-        if (tid < batch.n_seqs) {
-            int rank = 0;
-#pragma unroll 8
-            for (int j = 0; j < batch.n_seqs; ++j) rank += s_len[j] > mine || (s_len[j] == mine && j < tid);
-            if (rank == want) s_seq = tid;
-        }
-        __syncthreads();
-        seq = s_seq;
-        kvh = turn - want * kv.n_kv_heads;
-    }
+    const int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = n_heads / kv.n_kv_heads;
     const int slot = batch.seq_slot[seq];
     const int row = batch.cu_q[seq];
@@ -458,7 +435,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restric
 
 template <int D, bool FUSED, int AD_STAGES>
 static int launch_decode_staged(const void* q, void* out, SbBatch batch, SbKV kv, int n_heads, float scale, int window, int n_splits,
-                         int ordered, float* partial, int* counters, SbFusedQK fused, cudaStream_t stream) {
+                         float* partial, int* counters, SbFusedQK fused, cudaStream_t stream) {
     const int pipe_bytes = AD_WARPS * AD_STAGES * 2 * AD_KEYS_PER_WARP * D * 2;
     const int merge_bytes = (AD_WARPS * 16 * D + 2 * AD_WARPS * 16 + 16 * D + 32) * 4;
     const int smem = 16 * D * 2 + (pipe_bytes > merge_bytes ? pipe_bytes : merge_bytes);
@@ -494,7 +471,7 @@ static int launch_decode_staged(const void* q, void* out, SbBatch batch, SbKV kv
     config.attrs = attr;
     config.numAttrs = n_attr;
     cudaError_t e = cudaLaunchKernelEx(&config, attn_decode_kernel<D, FUSED, AD_STAGES>, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, batch,
-                                       kv, n_heads, scale * 1.4426950408889634f, window, n_splits, cluster_merge, ordered, partial,
+                                       kv, n_heads, scale * 1.4426950408889634f, window, n_splits, cluster_merge, partial,
                                        counters, fused);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
@@ -515,9 +492,8 @@ static int launch_decode(const void* q, void* out, SbBatch batch, SbKV kv, int n
     const int sm_count = sm_counts[device];
     const long long blocks = (long long)batch.n_seqs * kv.n_kv_heads * n_splits;
     if (blocks <= sm_count)
-        return launch_decode_staged<D, FUSED, 4>(q, out, batch, kv, n_heads, scale, window, n_splits, 0, partial, counters, fused, stream);
-    const int ordered = blocks > (D > 64 ? 2 : 4) * sm_count && batch.n_seqs <= AD_ORDERED;
-    return launch_decode_staged<D, FUSED, 3>(q, out, batch, kv, n_heads, scale, window, n_splits, ordered, partial, counters, fused, stream);
+        return launch_decode_staged<D, FUSED, 4>(q, out, batch, kv, n_heads, scale, window, n_splits, partial, counters, fused, stream);
+    return launch_decode_staged<D, FUSED, 3>(q, out, batch, kv, n_heads, scale, window, n_splits, partial, counters, fused, stream);
 }
 
 // Most splits whose merge fits: the last block of a (sequence, kv head) keeps two floats per (query head of the
