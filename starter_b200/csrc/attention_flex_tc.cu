@@ -26,7 +26,7 @@
 #include "tc_utils.cuh"
 
 #define FT_ROWS 128
-#define FT_IDS 128
+#define FT_IDS 128       // one per row thread
 #define FT_THREADS 256   // the rows; and a group of four warps of which one thread issues products and one copies
 
 // Where a DENSE call's keys and values lie (column offsets are in the maps' matrices).
@@ -42,6 +42,7 @@ flex_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
                          const __grid_constant__ CUtensorMap map_v, SbFlex p, SbBatch batch, __nv_bfloat16* __restrict__ out,
                          FlexRows dense, int* status) {
     constexpr int ATOMS = (KD + 63) / 64, V_ATOMS = VD / 64, V_STAGES = KD > 128 ? 1 : 2;
+    static_assert(DENSE || V_STAGES == 2, "the refill of the page ids counts on values being asked for before the keys after them");
     constexpr int SHARED_ATOM = DENSE ? ATOMS - 1 : ATOMS;   // the last block of 64 columns comes from the shared matrix
     constexpr int Q_ATOM = FT_ROWS * 128;          // bytes of a [128 rows][64 columns] block of Q
     constexpr int KV_ATOM = SB_PAGE * 128;         // bytes of a [64 keys][64 columns] block of K or V
@@ -138,11 +139,9 @@ flex_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
             *reinterpret_cast<uint4*>(q_s + (c >> 3) * Q_ATOM + tid * 128 + (((c & 7) ^ (tid & 7)) << 4)) = v;
         }
     }
-    // Ids of the block's pages: a ring of FT_IDS entries in two halves, refilled 64 at a time well ahead of their use.
-    auto load_ids = [&](int first, int count) {
-        for (int j = tid; j < count && first + j < n_pages; j += FT_ROWS) s_pages[(first + j) & (FT_IDS - 1)] = page_id(first_page + first + j);
-    };
-    if (!DENSE && owns_row) load_ids(0, FT_IDS);
+    // Ids of the block's pages: a ring of FT_IDS entries in two halves.  Both are filled at the start; every 64 pages the rows
+    // refill the half behind them with the pages 64 to 127 ahead (below).
+    if (!DENSE && owns_row && tid < n_pages) s_pages[tid] = page_id(first_page + tid);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // Q was written by ordinary stores
     tc_fence_before();
     __syncthreads();
@@ -213,9 +212,14 @@ flex_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
         float m_ref = -INFINITY, l_run = 0.f;
         for (int i = 0; i < n_pages; ++i) {
             const int b = i & 1;
-            if (!DENSE && i > 0 && (i & 63) == 0) load_ids(i + 64, 64);
+            // The half of pages i - 64 to i - 1 may be overwritten once S of page i is done: that took the keys of page i, which
+            // the copying thread asked for after the values of page i - 1, the last id it reads there.  The fetch of the new ids
+            // needs no such wait, and is under way during it.
+            const bool refill = !DENSE && i > 0 && (i & 63) == 0 && tid < 64 && i + 64 + tid < n_pages;
+            const int next_id = refill ? page_id(first_page + i + 64 + tid) : 0;
             mbar_wait(&s_done[b], (i >> 1) & 1, abort_flag, status);
             if (*abort_flag) break;
+            if (refill) s_pages[(i + 64 + tid) & (FT_IDS - 1)] = next_id;
             tc_fence_after();
             const int key0 = (first_page + i) * SB_PAGE;
             float s[SB_PAGE];

@@ -43,7 +43,7 @@
 
 #define PT_ROWS 128
 #define PT_D 128
-#define PT_IDS 128
+#define PT_IDS 128        // one per row thread
 #define PT_THREADS 256   // two groups of four warps: the rows; and the warp of the thread that issues the products, that of the thread that
                          // issues the copies and two spare ones, which together hand most of their registers to the rows
 
@@ -147,15 +147,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         }
     }
     // Ids of the block's pages: a ring of PT_IDS entries in two halves.  Both halves are filled at the start;
-    // every 64 pages the rows refill the half whose pages are behind them with the pages 64 to 127 ahead.
-    auto load_ids = [&](int first, int count) {
-        for (int j = tid; j < count && first + j < n_pages; j += PT_ROWS) {
-            int lp = first_page + first + j;
-            if (kv.ring_pages) lp %= kv.ring_pages;
-            s_pages[(first + j) & (PT_IDS - 1)] = max(table[lp], 0);
-        }
+    // every 64 pages the rows refill the half behind them with the pages 64 to 127 ahead (below).
+    auto page_id = [&](int i) {
+        int lp = first_page + i;
+        if (kv.ring_pages) lp %= kv.ring_pages;
+        return max(table[lp], 0);
     };
-    if (owns_row) load_ids(0, PT_IDS);
+    if (owns_row && tid < n_pages) s_pages[tid] = page_id(tid);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // Q was written by ordinary stores
     tc_fence_before();
     __syncthreads();
@@ -247,10 +245,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         const int lo_max = window > 0 ? max(0, pos_max - window + 1) : 0;
         for (int i = 0; i < n_pages; ++i) {
             const int b = i & 1;
-            if (i > 0 && (i & 63) == 0) load_ids(i + 64, 64);   // read by the issuer 62 pages (and as many barriers) from now
+            // The half of pages i - 64 to i - 1 may be overwritten once S of page i is done: that took the keys of page i, which
+            // the copying thread asked for after the values of page i - 1, the last id it reads there.  The new ids are read 62
+            // pages (and as many barriers) from now; their fetch needs no such wait, and is under way during it.
+            const bool refill = i > 0 && (i & 63) == 0 && tid < 64 && i + 64 + tid < n_pages;
+            const int next_id = refill ? page_id(i + 64 + tid) : 0;
             if (tid == 0) PT_STAMP(i, 7);
             mbar_wait(&s_done[b], (i >> 1) & 1, abort_flag, status);
             if (*abort_flag) break;
+            if (refill) s_pages[(i + 64 + tid) & (PT_IDS - 1)] = next_id;
             tc_fence_after();
             if (tid == 0) PT_STAMP(i, 3);
 

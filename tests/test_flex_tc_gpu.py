@@ -139,3 +139,50 @@ def test_rows_of_the_step(D, R, V, H, q_lens, with_sink):
         k = torch.cat([kv[piece, :H * D].view(n, H, D), latent[piece, None, 40:].expand(n, H, R)], -1)
         close(got[piece], oracle(q[piece], k, kv[piece, H * D:].view(n, H, V), 0, 0.11, lambda h: h, sink=sink), f"sequence {b}")
         at += n
+
+
+def long_context(rt, G, D, V, held, rows, seed=11):
+    """One sequence of ``held`` + ``rows`` tokens on pages in a shuffled order, every other page full of other numbers."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").bfloat16()   # noqa: E731
+    total = held + rows
+    cache = Cache([KVRequest(G, D, v_dim=V)], n_slots=2, max_tokens=64 * 260, dtype=torch.bfloat16, device="cuda", max_seq_tokens=total,
+                  max_step_tokens=rows)
+    layer, slot = cache.layers[0], cache.alloc()
+    layer.k.copy_(rnd(*layer.k.shape)), layer.v.copy_(rnd(*layer.v.shape))
+    cache.reserve(slot, total)
+    cache.flush()
+    pages = -(-total // 64)
+    ids = layer.group.table[slot, :pages].clone()
+    ids = ids[torch.randperm(pages, generator=g, device="cuda")]
+    layer.group.table[slot, :pages] = ids
+    cache.lengths[slot] = held
+    k, v = (t[ids.long()].transpose(1, 2).reshape(pages * 64, G, -1)[:total] for t in (layer.k, layer.v))
+    return describe(rt, cache, [slot], [held], [rows]), layer, k, v, rnd
+
+
+@pytest.mark.parametrize("held", [64 * 128 - 130, 9300, 13000])     # 128 pages exactly; one refill of the page ids; two, and a wrap
+@pytest.mark.parametrize("options", ["plain", "biased", "window"])
+def test_more_pages_than_the_kernel_keeps_ids_for(held, options):
+    rt, rows, H, G, D, V = runtime(), 130, 4, 2, 64, 128
+    ctx, layer, k, v, rnd = long_context(rt, G, D, V, held, rows)
+    more = {"plain": {}, "window": dict(window=held - 70),
+            "biased": dict(head_scale=torch.linspace(-0.5, 2.0, H, device="cuda"), slopes=torch.linspace(1e-2, 1e-5, H, device="cuda"))}[options]
+    q = rnd(rows, H, D)
+    got = rt.ops.flex_attention(ctx, q, layer, D ** -0.5, v_dim=V, **more)
+    assert rt.ops.read_kernel_status() == 0
+    want = oracle(q, k, v, held, D ** -0.5, lambda h: h * G // H, more.get("head_scale"), more.get("slopes"), None, more.get("window"))
+    close(got, want, f"{held} tokens held")
+
+
+@pytest.mark.parametrize("held", [9300, 13000])
+def test_the_plain_prompt_kernel_far_into_a_long_context(held):
+    rt, rows, H, G, D = runtime(), 140, 4, 2, 128
+    ctx, layer, k, v, rnd = long_context(rt, G, D, D, held, rows)
+    q = rnd(rows, H * D)
+    got = rt.ops.attention(ctx, q, layer, H, D ** -0.5, None)
+    assert rt.ops.read_kernel_status() == 0
+    want = oracle(q.view(rows, H, D), k, v, held, D ** -0.5, lambda h: h * G // H)
+    # that kernel's weights meet the values rounded to bfloat16: 2^-9 each, averaging out over thousands of keys
+    got = got.view(rows, H, D).to(F)
+    assert float((got - want).norm() / want.norm()) < 5e-3 and float((got - want).abs().max() / want.abs().max()) < 2e-2
