@@ -63,7 +63,9 @@ __device__ __forceinline__ void mlstm_gates(const float* __restrict__ z, long lo
 // their shares with three shuffles per column.  EXACT: D = 8 * EMAX with EMAX a multiple of 4; a thread's key channels
 // are then dealt out four at a time, ((e / 4) * 8 + ig) * 4 + e % 4, so that the eight lanes read 128 consecutive
 // bytes, 16 a lane.  With o_raw the head's columns are shared out over several blocks, which leave h_t there for
-// mlstm_finish_kernel; without, one block holds the whole head and finishes it itself.
+// mlstm_finish_kernel; without, one block holds the whole head and finishes it itself.  Each of several blocks starts from the
+// record's normaliser and maximum, and may start when another has ended: the new ones wait behind h_t, [sequence][head][D + 1],
+// and reach the record with mlstm_finish_kernel.
 template <class T, int EMAX, bool EXACT>
 __global__ void __launch_bounds__(ML_THREADS)
 mlstm_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ g, long long ld,
@@ -284,26 +286,41 @@ mlstm_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
         }
     }
     __syncthreads();
+    float* tail = o_raw != nullptr ? o_raw + (long long)batch.n_rows * H * V + ((long long)s * H + head) * (D + 1) : nullptr;
+    float* n_out = tail != nullptr ? tail : ng;
+    float* m_out = tail != nullptr ? tail + D : mg;
 #pragma unroll
     for (int c = 0; c < ML_CG; ++c)
 #pragma unroll
         for (int e = 0; e < EMAX; ++e) {
             if (active && e < E && chan(e) < D) {
                 if (c0 + c < nv) Sg[(long long)chan(e) * V + j0 + c0 + c] = S[c][e];
-                else if (c0 + c == nv && blockIdx.z == 0) ng[chan(e)] = S[c][e];
+                else if (c0 + c == nv && blockIdx.z == 0) n_out[chan(e)] = S[c][e];
             }
         }
-    if (tid == 0 && blockIdx.z == 0) *mg = m_run;
+    if (tid == 0 && blockIdx.z == 0) *m_out = m_run;
 }
 
-// One warp per (row, head): the head's unit norm over its V values of h, the norm weight, the gate and the scale.
+// One warp per (row, head): the head's unit norm over its V values of h, the norm weight, the gate and the scale.  The warps
+// after them, one per (sequence, head), bring the record's normaliser and maximum up to date.
 template <class T>
 __global__ void mlstm_finish_kernel(const float* __restrict__ o_raw, const T* __restrict__ g, long long ld, const float* __restrict__ norm_w,
-                                    float eps, float out_scale, int rows, int H, int V, T* __restrict__ y, long long y_ld) {
+                                    float eps, float out_scale, float* __restrict__ state, long long state_stride, SbBatch batch, int H,
+                                    int D, int V, T* __restrict__ y, long long y_ld) {
     pdl_wait();
+    const int rows = batch.n_rows;
     const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (wid >= (long long)rows * H) return;
+    if (wid >= (long long)rows * H) {
+        const long long at = wid - (long long)rows * H;
+        if (at >= (long long)batch.n_seqs * H) return;
+        const int s = (int)(at / H), head = (int)(at % H);
+        const float* tail = o_raw + (long long)rows * H * V + at * (D + 1);
+        float* rec = state + (long long)batch.seq_slot[s] * state_stride + (long long)H * D * V;
+        for (int i = lane; i < D; i += 32) rec[(long long)head * D + i] = tail[i];
+        if (lane == 0) rec[(long long)H * D + head] = tail[D];
+        return;
+    }
     const long long row = wid / H;
     const int head = (int)(wid % H);
     const float* o = o_raw + (row * H + head) * V;
@@ -384,8 +401,8 @@ extern "C" {
 
 // q, k [rows, H * D], v, g [rows, H * V]: views whose rows are `ld` elements apart; z [rows, z_ld] 32-bit with head h's
 // input gate at column i_col + h and forget gate at f_col + h; state [slots] records of H * D * V + H * D + H floats,
-// `state_stride` floats apart; y [rows, H * V] with rows y_ld apart; o_raw: [rows, H * V] floats of scratch for heads
-// of more than ML_VB value channels.
+// `state_stride` floats apart; y [rows, H * V] with rows y_ld apart; o_raw: [rows, H * V] and behind them [n_seqs, H * (D + 1)]
+// floats of scratch for heads of more than ML_VB value channels.
 int sb_mlstm_scan(int dtype, const void* q, const void* k, const void* v, const void* g, long long ld, const float* z, long long z_ld,
                   int i_col, int f_col, const float* i_bias, const float* f_bias, float cap, const float* norm_w, float eps,
                   float q_scale, float out_scale, float* state, long long state_stride, SbBatch batch, int H, int D, int V, void* y,
@@ -437,14 +454,14 @@ int sb_mlstm_scan(int dtype, const void* q, const void* k, const void* v, const 
 #undef SB_ML_SIZES
 #undef SB_ML
     if (raw != nullptr) {
-        const long long warps = (long long)batch.n_rows * H;
+        const long long warps = ((long long)batch.n_rows + batch.n_seqs) * H;
         const unsigned int blocks = (unsigned int)((warps * 32 + 255) / 256);
         if (dtype == SB_F32)
             sb_launch(mlstm_finish_kernel<float>, blocks, 256, 0, stream, (const float*)raw, (const float*)g, ld, norm_w, eps, out_scale,
-                      batch.n_rows, H, V, (float*)y, y_ld);
+                      state, state_stride, batch, H, D, V, (float*)y, y_ld);
         else
             sb_launch(mlstm_finish_kernel<bf>, blocks, 256, 0, stream, (const float*)raw, (const bf*)g, ld, norm_w, eps, out_scale,
-                      batch.n_rows, H, V, (bf*)y, y_ld);
+                      state, state_stride, batch, H, D, V, (bf*)y, y_ld);
     }
     SB_LAUNCH_CHECK();
 }

@@ -1410,7 +1410,8 @@ class Ops:
         if self.chunk_memory(ctx, self.CHUNK_MLSTM, heads, dim, vdim, q, k, v, g, ld, z, i_bias, f_bias, norm, vdim, eps, state, y,
                              z_cols=(i_col, f_col), cap=cap, q_scale=q_scale, out_scale=out_scale):
             return y
-        raw = torch.empty((rows, heads * vdim), dtype=torch.float32, device=q.device) if vdim > 64 else None
+        # heads of more than 64 value channels: raw outputs, then the records' new normalisers and maxima
+        raw = torch.empty(rows * heads * vdim + ctx.n_seqs * heads * (dim + 1), dtype=torch.float32, device=q.device) if vdim > 64 else None
         self._check(self.lib.sb_mlstm_scan(_code(q.dtype), _ptr(q), _ptr(k), _ptr(v), _ptr(g), ld, _ptr(z), z.stride(0), int(i_col),
                                            int(f_col), _ptr(i_bias), _ptr(f_bias), float(cap), _ptr(norm), float(eps), float(q_scale),
                                            float(out_scale), _ptr(state), state.stride(0), self._batch(ctx), heads, dim, vdim,

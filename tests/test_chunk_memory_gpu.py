@@ -162,3 +162,37 @@ def test_chunks_against_the_recurrence_in_64_bits(kind, case):
     assert rel(y, want) < 2 ** -8
     assert rel(st, want_state) < 5.4e-5
     assert math.isfinite(float(st.abs().max()))
+
+
+@pytest.mark.parametrize("H, D, V, counts", [(16, 64, 128, [1] * 130), (16, 64, 128, [16] * 33 + [3, 70]), (20, 32, 72, [2] * 200), (9, 128, 200, [1, 40] * 60)])
+def test_a_walk_of_many_sequences_leaves_what_each_alone_does(H, D, V, counts):
+    """Heads whose value channels several blocks share out: more blocks than the GPU holds at a time, so that one starts from the
+    record when another of its head has long ended.  A sequence's outputs and record are the same numbers as alone."""
+    from starter_b200.csrc.ops import get_ops
+    ops = get_ops(verbose=False)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")   # noqa: E731
+    n, rows = len(counts), sum(counts)
+    p, z = rand(rows, 2 * H * D + 2 * H * V).bfloat16(), rand(rows, 2 * H) * 4
+    bi, bf, norm, state = rand(H), rand(H) + 2.0, rand(H * V), rand(n + 1, H * D * V + H * D + H)
+
+    def run(ctx, lo, hi, st):
+        at, views = 0, []
+        for c in (H * D, H * D, H * V, H * V):
+            views.append(p[lo:hi, at:at + c])
+            at += c
+        return ops.mlstm_scan(ctx, *views, z[lo:hi], 0, H, bi, bf, 15.0, norm, EPS, D ** -0.5, st, H, D, V)
+
+    ops.force_chunk_memory = False
+    try:
+        ctx, cu = batch_of(counts, list(range(n)), n)
+        together = state.clone()
+        y = run(ctx, 0, rows, together)
+        for s in range(n):
+            alone = state[s:s + 1].clone()
+            one, _ = batch_of(counts[s:s + 1], [0], 1)
+            assert torch.equal(run(one, cu[s], cu[s + 1], alone), y[cu[s]:cu[s + 1]]), f"outputs of sequence {s}"
+            assert torch.equal(alone[0], together[s]), f"record of sequence {s}"
+    finally:
+        del ops.force_chunk_memory
+    assert torch.equal(together[n], state[n])
