@@ -23,6 +23,7 @@
 #define GG_BK 16
 #define GG_CHUNK 512   // columns of k per running sum; a multiple of GG_BK
 #define GG_THREADS 256
+#define GG_DOT_MAX 16384   // outputs of a bfloat16 product up to which a warp takes one
 
 template <class TA> struct GgFour;
 template <> struct GgFour<float> {
@@ -290,7 +291,8 @@ __global__ void __launch_bounds__(256) gemm_general_add_kernel(const float* __re
 }
 
 // A product of few outputs (bfloat16 run): a warp per output element, its lanes along k, so that a handful of columns
-// does not run as one block's serial chain (32 rows of [16, 1024]: 58 us as one tile, 3 as 512 warps).
+// does not run as one block's serial chain (32 rows of [16, 1024]: 58 us as one tile, 3 as 512 warps).  GG_DOT_MAX of them are two
+// rounds of the GPU's warps; four times as many cost what a tile of the same columns of k does.
 template <class TA, class TO>
 __global__ void __launch_bounds__(256) gemm_general_dot_kernel(const TA* __restrict__ A, const TA* __restrict__ W, TO* __restrict__ C,
                                                                int M, int N, int K, int vec) {
@@ -334,17 +336,46 @@ static void gg_launch(const void* A, const void* W, void* C, int M, int N, int K
     }
 }
 
-static int gg_tile_rows(int M) {
-    if (M <= 8) return 8;
-    if (M <= 32) return 32;
-    if (M <= 64) return 64;
-    const int big = (M + 127) / 128 * 128, small = (M + 63) / 64 * 64;   // a tile of 64 rows reads half as much again per multiply-add
-    return big * 100 <= small * 120 ? 128 : 64;
+#define GG_SMS 148
+#define GG_MAX_SCRATCH (64ll << 20)   // floats
+
+// Rows of a product's tiles, and whether its chunks of k run side by side (`apart`; only where the caller can give scratch for
+// them).  A chunk of 512 columns takes an SM 21, 34 or 49 us for a tile of 32, 64 or 128 rows by 128 columns (two blocks of an SM
+// take turns): a larger tile has less to read per multiply-add, a smaller one reaches more SMs and works less for padding.  So the
+// rounds of the tiles, and for sums that travel through memory 8 bytes each at 5 TB/s and a launch.  With the largest tile that the
+// rows fill, 100 rows of [100, 512] take 51 us, so 22 (40 with the kernel of one tile of 64 x 64 before it); 1,000 rows of
+// [1000, 900] 93, so 60 (94).  Up to 8 rows (a thread per column) two blocks of an SM hide one another's reads.
+struct GgPlan {
+    int rows;
+    bool apart;
+};
+
+static GgPlan gg_plan(int M, int N, int K, bool may_split) {
+    static const int rows[4] = {8, 32, 64, 128};
+    static const double unit[4] = {5.5, 21.0, 34.0, 49.0};
+    const int chunks = (K + GG_CHUNK - 1) / GG_CHUNK;
+    const long long floats = (long long)M * N * chunks;
+    const bool split = may_split && chunks > 1 && floats <= GG_MAX_SCRATCH;
+    GgPlan best = {8, false};
+    double best_us = -1.0;
+    for (int i = M <= 8 ? 0 : 1; i < 4; ++i) {
+        if (i > 0 && (M <= 8 || (i > 1 && M <= rows[i] / 2))) break;
+        const int bn = i == 0 ? 256 : 128;
+        const long long wave = i == 0 ? 2 * GG_SMS : GG_SMS, tiles = (long long)((M + rows[i] - 1) / rows[i]) * ((N + bn - 1) / bn);
+        const double round = i == 0 ? 2 * unit[i] : unit[i];
+        const double together = (double)((tiles + wave - 1) / wave) * round * (i == 0 ? chunks : (double)K / GG_CHUNK);
+        if (best_us < 0.0 || together < best_us) best = {rows[i], false}, best_us = together;
+        const double apart = (double)((tiles * chunks + wave - 1) / wave) * round + floats * 8.0 / 5e6 + 2.0;
+        if (split && apart < best_us) best = {rows[i], true}, best_us = apart;
+    }
+    return best;
 }
 
 template <class TA, class TO>
 static void gg_pick(const void* A, const void* W, void* C, int M, int N, int K, float* parts, int vec, cudaStream_t stream) {
-    switch (gg_tile_rows(M)) {
+    const GgPlan plan = gg_plan(M, N, K, parts != nullptr);
+    if (!plan.apart) parts = nullptr;
+    switch (plan.rows) {
         case 8: return gg_launch<TA, TO, 8, 8, 1>(A, W, C, M, N, K, parts, vec, stream);
         case 32: return gg_launch<TA, TO, 32, 4, 4>(A, W, C, M, N, K, parts, vec, stream);
         case 64: return gg_launch<TA, TO, 64, 4, 8>(A, W, C, M, N, K, parts, vec, stream);
@@ -354,22 +385,10 @@ static void gg_pick(const void* A, const void* W, void* C, int M, int N, int K, 
 
 extern "C" {
 
-// Floats of scratch that a 32-bit product wants, 0 when its chunks of k run in one block.  Side by side they fill the
-// GPU (two blocks to an SM); in one block they save the trip of their sums through memory.  In units of one chunk of one
-// tile on one SM (44 us for 128 x 128 x 512 at three quarters of the peak): tiles / 148 rounds of all chunks against
-// tiles * chunks / 296 rounds of two, and 8 bytes a sum at 5 TB/s.
-long long sb_gemm_general_scratch(int M, int N, int K, int sms) {
-    const int chunks = (K + GG_CHUNK - 1) / GG_CHUNK;
-    if (chunks < 2 || M <= 0 || N <= 0 || sms <= 0) return 0;
-    const int bm = gg_tile_rows(M), bn = bm == 8 ? 256 : 128;
-    const long long tiles = (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn);
-    const long long floats = (long long)M * N * chunks;
-    if (floats > (64ll << 20)) return 0;
-    const double unit = 44.0 * (bm * (double)bn) / (128.0 * 128.0);   // us
-    const int resident = bm == 128 ? 1 : 2;
-    const double together = (double)((tiles + (long long)sms * resident - 1) / ((long long)sms * resident)) * resident * chunks * unit;
-    const double apart = (double)((tiles * chunks + 2ll * sms - 1) / (2ll * sms)) * 2 * unit + floats * 8.0 / 5e6 + 2.0;
-    return apart < together ? floats : 0;
+// Floats of scratch that a product wants, 0 when its chunks of k run in one block.  Without them it does that too.
+long long sb_gemm_general_scratch(int M, int N, int K) {
+    if (M <= 0 || N <= 0) return 0;
+    return gg_plan(M, N, K, true).apart ? (long long)M * N * ((K + GG_CHUNK - 1) / GG_CHUNK) : 0;
 }
 
 int sb_gemm_general(int dtype, int out_f32, const void* A, const void* W, void* C, int M, int N, int K, float* parts,
@@ -393,7 +412,7 @@ int sb_gemm_general(int dtype, int out_f32, const void* A, const void* W, void* 
         }
     } else if (dtype == SB_F32) {
         gg_pick<float, float>(A, W, C, M, N, K, parts, vec, stream);
-    } else if ((long long)M * N <= 4096) {
+    } else if ((long long)M * N <= GG_DOT_MAX) {
         const dim3 grid((unsigned int)(((long long)M * N + 7) / 8));
         if (out_f32)
             sb_launch(gemm_general_dot_kernel<__nv_bfloat16, float>, grid, 256, 0, stream, (const __nv_bfloat16*)A, (const __nv_bfloat16*)W,

@@ -230,7 +230,7 @@ class Ops:
         lib.sb_chunk_memory_floats.restype = c_longlong
         lib.sb_delta_chunk_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.sb_delta_chunk_floats.restype = c_longlong
-        lib.sb_gemm_general_scratch.argtypes = [c_int, c_int, c_int, c_int]
+        lib.sb_gemm_general_scratch.argtypes = [c_int, c_int, c_int]
         lib.sb_gemm_general_scratch.restype = c_longlong
         lib.sb_set_pdl.argtypes = [c_int]
         lib.sb_set_pdl.restype = None
@@ -609,7 +609,7 @@ class Ops:
                 return torch.mm(a, w.t())
         out = torch.empty((M, N), dtype=torch.float32 if out_float32 else a.dtype, device=a.device)
         a = a.contiguous()
-        floats = self.lib.sb_gemm_general_scratch(M, N, K, self.sm_count())
+        floats = self.lib.sb_gemm_general_scratch(M, N, K)
         parts = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
         self._check(self.lib.sb_gemm_general(_code(a.dtype), int(out_float32 or a.dtype == torch.float32), _ptr(a), _ptr(w),
                                              _ptr(out), M, N, K, _ptr(parts), self._stream()), "gemm_general")

@@ -81,3 +81,19 @@ def test_product_32_bit_of_a_few_rows(ops, M, N, K):
     assert torch.equal(ops.linear(torch.cat([a, rand((60, K), 3)]), w)[:M], got)
     shifted = torch.empty(N * K + 1, device="cuda")[1:].view(N, K).copy_(w)
     assert torch.equal(ops.linear(a, shifted), got)
+
+
+@pytest.mark.parametrize("M, N, K", [(33, 6200, 530), (65, 6200, 530), (129, 6300, 530), (300, 6144, 100), (1000, 1000, 1030), (2500, 1000, 70), (82, 50, 1000), (40, 6144, 2560),
+                                     (300, 2560, 4096)])
+def test_product_32_bit_whatever_the_tile(ops, M, N, K):
+    """Sizes whose tiles have 32, 64 and 128 rows, with the chunks of k in one block and side by side: the sums are those of the rows in
+    pieces that take other tiles."""
+    a, w = rand((M, K), 1), rand((N, K), 2) * K ** -0.5
+    got = ops.linear(a, w)
+    want = a.double() @ w.double().T
+    assert float((got - want).norm() / want.norm()) < 1e-6
+    assert torch.equal(torch.cat([ops.linear(piece, w) for piece in a.split(27)]), got)
+    if K % 8 or M * N * K <= ops.GENERAL_GEMM_MAX_WORK:     # others are the library's
+        got = ops.linear(a.bfloat16(), w.bfloat16(), out_float32=True)
+        want = a.bfloat16().double() @ w.bfloat16().double().T
+        assert float((got - want).norm() / want.norm()) < 1e-6
