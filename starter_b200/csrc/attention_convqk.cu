@@ -261,8 +261,11 @@ int sb_conv_qk_store(int dtype, const void* q, long long q_ld, const void* k, lo
     dim3 grid(batch.n_rows, per_row);
     const size_t smem = (size_t)D * sizeof(float);
     typedef __nv_bfloat16 bf;
-    // below 128 rows the blocks per head of the kernel above reach more SMs
-    const bool runs = dtype == SB_BF16 && conv && taps <= 4 && (D == 64 || D == 128) && batch.n_rows >= 128 && q_ld % 4 == 0 && k_ld % 4 == 0
+    // Where runs pay (us, block per row / runs; 10 heads of 64 and 12 of 128).  Prompts: 256 rows 7.2 / 8.8 and 9.8 / 9.2, 384 8.0 / 9.0
+    // and 12.3 / 9.4, 512 9.1 / 8.9 and 14.8 / 10.0.  One row a sequence, where a run starts from a record at every row: 512 rows
+    // 12.5 / 18.5 and 22.8 / 22.4, 768 14.9 / 18.6 and 28.2 / 23.2, 1,024 17.1 / 19.2, 2,048 30.3 / 26.3 and 62.8 / 46.6.
+    const bool runs = dtype == SB_BF16 && conv && taps <= 4 && (D == 64 || D == 128)
+                      && (long long)batch.n_rows * D >= (batch.n_rows >= 8ll * batch.n_seqs ? 32768 : 98304) && q_ld % 4 == 0 && k_ld % 4 == 0
                       && p.v_row % 4 == 0 && sb_aligned(8, q, k, q_out, p.k, p.v);
     const dim3 run_grid((batch.n_rows + CQ_RUN - 1) / CQ_RUN, (units + 3) / 4);
     if (runs && D == 64)

@@ -228,8 +228,9 @@ int sb_rotate_store(int dtype, const void* q, long long q_row, const void* k, lo
     const int per_row = batch.n_rows >= 1024 ? min(units, 4) : (batch.n_rows >= 128 ? min(units, 8) : min(units, 64));
     dim3 grid(batch.n_rows, per_row);
     const size_t smem = (size_t)rot * sizeof(float);
-    // below 128 rows the blocks per head of the kernel above reach more SMs than blocks of four rows would
-    if (dtype == SB_BF16 && batch.n_rows >= 128 && p.k_dim % 8 == 0 && p.v_dim % 8 == 0 && p.v_row % 8 == 0 && rot % (halves ? 16 : 8) == 0
+    // Below 256 rows the blocks per head of the kernel above reach more SMs than blocks of four rows would (us, above / four rows; 24 heads
+    // of 64 and of 128): 128 rows 4.5 / 4.7 and 4.9 / 6.5, 200 4.9 / 4.7 and 5.5 / 6.4, 256 6.4 / 4.7 and 6.8 / 6.4.
+    if (dtype == SB_BF16 && batch.n_rows >= 256 && p.k_dim % 8 == 0 && p.v_dim % 8 == 0 && p.v_row % 8 == 0 && rot % (halves ? 16 : 8) == 0
         && q_row % 8 == 0 && k_row % 8 == 0 && v_row % 8 == 0 && rot <= 1024 && sb_aligned(16, q, k, v, q_out, p.k, p.v)) {
         typedef __nv_bfloat16 bf;
         sb_launch(rotate_store_rows_kernel, (batch.n_rows + RS_ROWS - 1) / RS_ROWS, 256, RS_ROWS * smem, stream, (const bf*)q, q_row, (const bf*)k,

@@ -163,3 +163,44 @@ def test_unit_heads_of_many_rows(D, G, H, taps):
         assert torch.equal(whole[1][at:at + n], part[1])
         at += n
     assert torch.equal(s1, s2)
+
+
+LONGER = [441, 2, 277]      # beyond the rows from which the kernels of this file take the whole step
+
+
+@pytest.mark.parametrize("D, V, nq, G, vh, rot, halves", [(64, 128, 8, 4, 2, 64, True), (128, 64, 3, 3, 3, 16, True), (64, 64, 4, 2, 2, 64, False),
+                                                          (24, 8, 5, 1, 1, 8, False), (72, 40, 2, 2, 2, 48, True), (64, 64, 2, 2, 1, 0, True),
+                                                          (40, 16, 2, 1, 1, 24, True)])
+def test_rotated_rows_of_longer_steps(monkeypatch, D, V, nq, G, vh, rot, halves):
+    monkeypatch.setitem(globals(), "LENGTHS", LONGER)
+    test_rotated_rows(D, V, nq, G, vh, rot, halves)
+
+
+@pytest.mark.parametrize("D, H, G, taps, bias, norm", [(128, 5, 2, 4, True, True), (64, 4, 4, 3, False, True), (128, 2, 1, 2, True, False),
+                                                       (64, 1, 1, 1, True, True), (64, 3, 1, 4, True, True)])
+def test_convolved_rows_of_longer_steps(monkeypatch, D, H, G, taps, bias, norm):
+    monkeypatch.setitem(globals(), "LENGTHS", LONGER)
+    test_convolved_rows(D, H, G, taps, bias, norm)
+
+
+@pytest.mark.parametrize("D, taps", [(128, 4), (64, 3)])
+def test_convolved_rows_of_many_sequences(D, taps):
+    """One row a sequence: runs of eight rows from 768 (heads of 128) and 1,536 (of 64) on, beside steps of 100."""
+    rt, n, H, G = runtime("bfloat16"), 1600, 2, 1
+    p, w = rand((n, (H + G) * D), 41).bfloat16(), [rand((h * D, taps), 42 + h, 0.5) for h in (H, G)]
+    record, res = rand((n + 1, taps - 1, (H + G) * D), 45), []
+    for size in (n, 100):
+        cache = Cache([(KVRequest(num_kv_heads=G, head_dim=D, v_dim=D), StateRequest((taps - 1, (H + G) * D)))], n_slots=n, max_tokens=64 * n,
+                      dtype=rt.dtype, device="cuda")
+        slots = [cache.alloc() for _ in range(n)]
+        lc, outs = cache.layers[0], []
+        lc.aux.state.copy_(record)
+        for at in range(0, n, size):
+            ctx = context(rt, cache, slots[at:at + size], [1] * size)
+            x = p[at:at + size]
+            outs.append(rt.ops.conv_qk_store(ctx, x[:, :H * D], x[:, H * D:], lc, lc.aux.state, H, None, None, *w, None, None, 1e-5, 0.0, 0))
+            assert int(ctx.status.item()) == 0
+        res.append((torch.cat(outs), cache))
+    same(res[0][0], res[1][0], "queries")
+    same(res[0][1].layers[0].k, res[1][1].layers[0].k, "keys")
+    assert torch.equal(res[0][1].layers[0].aux.state, res[1][1].layers[0].aux.state)
