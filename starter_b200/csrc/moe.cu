@@ -17,6 +17,7 @@
 #define MOE_MAX_TOP 32
 
 #define MOE_ROUTE_FEW 64   // rows up to which a block takes a row's logits and its choice
+#define MOE_ROUTE_STATIC 128   // bytes of shared memory that this kernel declares: 32 logits
 #define MOE_ROUTE_ROWS 8   // rows that share one read of a router row
 
 __device__ __forceinline__ float4 load4f(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -134,7 +135,7 @@ moe_route_row_kernel(const T* __restrict__ h, const float* __restrict__ router, 
                      const float* __restrict__ bias, int over_chosen, float* __restrict__ logits, int* __restrict__ chosen,
                      float* __restrict__ weight, int width, int n_out, int ld, int top, float scale, int sigmoid, int groups, int keep) {
     extern __shared__ __align__(16) float route_sm[];
-    __shared__ float out_s[32];
+    __shared__ float out_s[MOE_ROUTE_STATIC / sizeof(float)];
     pdl_wait();
     const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     stage_rows<T>(route_sm, h + (long long)row * width, width, (width & 7) == 0);
@@ -574,6 +575,12 @@ __global__ void moe_combine_kernel(const T* __restrict__ h, const T* __restrict_
 
 extern "C" {
 
+// Kernels that a routing of these sizes launches: one for few rows and outputs whose row fits the shared memory that a launch may
+// use without asking, beside what the kernel keeps there itself (MOE_ROUTE_STATIC bytes); two otherwise.
+int sb_moe_route_launches(int rows, int width, int n_out) {
+    return rows <= MOE_ROUTE_FEW && n_out <= 32 && (size_t)width * sizeof(float) + MOE_ROUTE_STATIC <= 48 * 1024 ? 1 : 2;
+}
+
 int sb_moe_route(int dtype, const void* h, const float* router, const float* correction, const float* bias, int over_chosen,
                  float* logits, int* chosen, float* weight, int rows, int width, int n_out, int top, float scale, int sigmoid,
                  int groups, int keep, int extra, cudaStream_t stream) {
@@ -582,7 +589,7 @@ int sb_moe_route(int dtype, const void* h, const float* router, const float* cor
     if (groups < 1 || n_out % groups || keep < 1 || keep > groups || keep * (n_out / groups) < top || extra < 0)
         return (int)cudaErrorInvalidValue;
     if (n_out < 1 || n_out > MOE_MAX_OUTPUTS || top < 1 || top > MOE_MAX_TOP || top > n_out) return (int)cudaErrorInvalidValue;
-    if (rows <= MOE_ROUTE_FEW && n_out <= 32 && (size_t)width * sizeof(float) <= 48 * 1024) {
+    if (sb_moe_route_launches(rows, width, n_out) == 1) {
 #define SB_ROUTE_ROW(T)                                                                                                              \
     sb_launch(moe_route_row_kernel<T>, rows, 32 * (n_rows_out < 32 ? n_rows_out : 32), (size_t)width * sizeof(float), stream, (const T*)h, router, correction, bias, over_chosen,   \
               logits, chosen, weight, width, n_out, n_rows_out, top, scale, sigmoid, groups, keep)

@@ -191,6 +191,7 @@ class Ops:
             "sb_moe_route": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                              c_int, c_float, c_int, c_int, c_int, c_int, c_void_p],
             "sb_moe_sort": [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+            "sb_moe_route_launches": [c_int, c_int, c_int],
             "sb_moe_gather": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
             "sb_moe_pairs": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                              c_float, c_float, c_int, c_void_p],
@@ -1643,8 +1644,7 @@ class Ops:
         self._check(self.lib.sb_moe_route(_code(h.dtype), _ptr(h), _ptr(router), _ptr(correction), _ptr(bias), int(bool(over_chosen)),
                                           _ptr(logits), _ptr(chosen), _ptr(weight), rows, width, n_out, int(top), float(scale),
                                           int(scores == "sigmoid"), int(groups), int(keep_groups), int(extra), self._stream()), "moe_route")
-        if rows > 64 or n_out > 32 or width > 12288:
-            self.launches += 1   # logits, then the choice; few rows and outputs take both in one kernel
+        self.launches += self.lib.sb_moe_route_launches(rows, width, n_out) - 1   # logits, then the choice; few rows take both in one
         return (chosen, weight, logits[:, n_out:]) if extra else (chosen, weight)
 
     MOE_PAIRS_MAX = int(os.environ.get("STARTER_B200_MOE_PAIRS_MAX", 64))   # pairs up to which every pair streams its expert

@@ -94,3 +94,19 @@ def test_routes_of_few_rows_as_of_many(n_out, top, groups, keep, extra, mode, dt
         assert float((few[1] - many[1][:rows]).abs().max()) <= 1e-6
         if extra:
             assert torch.equal(few[2], many[2][:rows])
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("width", [12256, 12257, 12260, 12288, 12292])
+def test_rows_as_wide_as_the_shared_memory_of_a_launch(width, dtype):
+    """One kernel up to 12,256 columns (48 KB with what it keeps itself), two beyond: the same routing as among 70 rows."""
+    from starter_b200.csrc.ops import get_ops
+    ops, n_out = get_ops(verbose=False), 18
+    g = torch.Generator().manual_seed(6)
+    h = torch.randn(70, width, generator=g).to(getattr(torch, dtype)).cuda()
+    router = torch.randn(n_out, width, generator=g).cuda() * width ** -0.5
+    many = ops.moe_route(h, router, None, 4, 1.0)
+    before = ops.launches
+    few = ops.moe_route(h[:3].contiguous(), router, None, 4, 1.0)
+    assert ops.launches - before == (1 if width <= 12256 else 2)
+    assert torch.equal(few[0], many[0][:3]) and float((few[1] - many[1][:3]).abs().max()) <= 1e-6
