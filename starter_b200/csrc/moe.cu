@@ -119,10 +119,10 @@ __device__ __forceinline__ unsigned int order_key(float x) {
     return x != x ? 0u : (u & 0x80000000u ? ~u : u | 0x80000000u);
 }
 
-// The lane that holds the largest key (of equals the lowest); every lane gets its number.
+// The lane that holds the largest key (of equals the lowest; 0 when all are 0, as no score is above -inf); every lane gets its number.
 __device__ __forceinline__ int warp_largest(unsigned int key) {
     const unsigned int top = __reduce_max_sync(0xffffffffu, key);
-    return __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
+    return top == 0u ? 0 : __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
 }
 
 // Few rows (decoding) and up to 32 outputs: a block per row takes the row's logits, a warp per output, and its first warp
@@ -182,19 +182,17 @@ moe_route_row_kernel(const T* __restrict__ h, const float* __restrict__ router, 
             }
             mine = each > 1 ? first + second : first;
         }
-        unsigned int kept = 0u;
-        for (int k = 0; k < keep; ++k) {   // key 0 is out; a score of -inf stands above it, as the first of nothing better
-            const int at = warp_largest(lane < groups && !(kept >> lane & 1u) ? max(order_key(mine), 1u) : 0u);
-            kept |= 1u << at;
-        }
+        // groups of score +inf are kept beside the `keep` best; a group of score -inf (or NaN) is kept only as group 0 with nothing better left
+        unsigned int kept = __ballot_sync(0xffffffffu, lane < groups && mine == INFINITY);
+        for (int k = 0; k < keep; ++k)
+            kept |= 1u << warp_largest(lane < groups && !(kept >> lane & 1u) && mine > -INFINITY ? order_key(mine) : 0u);
         if (real && !(kept >> (lane / each) & 1u)) c = -INFINITY;
     }
     float total = 0.f;
     int mine = 0;                       // lane k keeps the k-th choice
     unsigned int key = real && c > -INFINITY ? order_key(c) : 0u;
     for (int k = 0; k < top; ++k) {
-        const unsigned int any = __reduce_max_sync(0xffffffffu, key);
-        const int at = any == 0u ? 0 : __ffs(__ballot_sync(0xffffffffu, key == any)) - 1;   // nothing above -inf: output 0
+        const int at = warp_largest(key);
         if (lane == k) mine = at;
         total += __shfl_sync(0xffffffffu, s, at);
         if (lane == at) key = 0u;

@@ -110,3 +110,25 @@ def test_rows_as_wide_as_the_shared_memory_of_a_launch(width, dtype):
     few = ops.moe_route(h[:3].contiguous(), router, None, 4, 1.0)
     assert ops.launches - before == (1 if width <= 12256 else 2)
     assert torch.equal(few[0], many[0][:3]) and float((few[1] - many[1][:3]).abs().max()) <= 1e-6
+
+
+@pytest.mark.parametrize("out, forced", [([0, 1, 2, 4, 5, 6, 8, 9, 10], []), ([3, 4, 5, 6, 7], []), ([0, 1, 2, 3, 4, 8, 9, 10, 11], []), ([4, 5], [9]),
+                                         ([], [0, 1, 6]), (list(range(12)), []), ([0, 1, 2, 3, 5, 6, 7], [8])])
+@pytest.mark.parametrize("scores", ["softmax", "sigmoid"])
+def test_groups_whose_outputs_are_shut_out_or_forced(out, forced, scores):
+    """A correction of -inf takes an output out and may leave its group's two best at -inf, one of +inf forces it: few rows are routed
+    as many are."""
+    from starter_b200.csrc.ops import get_ops
+    ops, width, n_out = get_ops(verbose=False), 64, 12
+    g = torch.Generator().manual_seed(8)
+    h = torch.randn(70, width, generator=g).bfloat16().cuda()
+    router = torch.randn(n_out, width, generator=g).cuda() * 0.3
+    correction = torch.zeros(n_out)
+    correction[out] = float("-inf")
+    correction[forced] = float("inf")
+    for keep in (1, 2, 3):
+        kind = dict(scores=scores, groups=3, keep_groups=keep)
+        many = ops.moe_route(h, router, correction.cuda(), 4, 1.0, **kind)
+        few = ops.moe_route(h[:9].contiguous(), router, correction.cuda(), 4, 1.0, **kind)
+        assert torch.equal(few[0], many[0][:9]), keep
+        assert float((few[1] - many[1][:9]).abs().max()) <= 1e-6
