@@ -62,9 +62,11 @@ __device__ __forceinline__ float xielu_value(float v, float a_pos, float a_neg) 
     return v > 0.f ? fmaf(a_pos * v, v, 0.5f * v) : fmaf(a_neg, expm1f(v) - v, 0.5f * v);
 }
 
-// The tanh form of gelu: z / 2 (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3))).
+// The tanh form of gelu, z / 2 (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3))), as z / (1 + exp(-2 sqrt(2 / pi) (...))): 1 + tanh cancels
+// for negative z.  With correctly rounded functions, over all finite bfloat16 z: the tanh is wrong by 5e-4 of the result at z = -4 and by
+// all of it below -6, 138 results round to another bfloat16 number than the exact one does; this by 9e-7 and 5e-6, none does.
 __device__ __forceinline__ float gelu_tanh_value(float z) {
-    return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * fmaf(0.044715f * z * z, z, z)));
+    return z / (1.0f + expf(-1.5957691216057308f * fmaf(0.044715f * z * z, z, z)));
 }
 
 // Two 32-bit operations in one instruction (sm_100): a * b + c and a + b on pairs, each element rounded as the single

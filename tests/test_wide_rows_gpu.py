@@ -204,3 +204,21 @@ def test_convolved_rows_of_many_sequences(D, taps):
     same(res[0][0], res[1][0], "queries")
     same(res[0][1].layers[0].k, res[1][1].layers[0].k, "keys")
     assert torch.equal(res[0][1].layers[0].aux.state, res[1][1].layers[0].aux.state)
+
+
+def test_gated_gelu_rounds_a_row_as_its_other_forms_do():
+    """Every finite bfloat16 number through the kernel of 16 bytes a thread: the 32-bit kernel's result, rounded once; and that result
+    against 64 bits: up to eight roundings of 2^-24, and four of them times the exponent where that is large."""
+    ops = runtime("bfloat16").ops
+    g = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    g = g[torch.isfinite(g)].cuda()
+    g = g[:g.numel() // 8 * 8].view(1, -1)
+    u = rand(g.shape, 51).bfloat16()
+    wide, narrow = ops.gated_gelu(torch.cat([g, u], 1).float()), ops.gated_gelu(torch.cat([g, u], 1))
+    assert torch.equal(narrow, wide.bfloat16())
+    z = g.double()
+    exponent = -2.0 * (2.0 / torch.pi) ** 0.5 * (z + 0.044715 * z ** 3)
+    want = z / (1.0 + torch.exp(exponent)) * u.double()
+    error = (wide.double() - want).abs()
+    sound = (want.abs() > 1e-30) & (want.abs() < 1e30)
+    assert bool((error <= want.abs() * (4.0 + 2.0 * exponent.clamp(min=0.0)) * 2.0 ** -23)[sound].all())
