@@ -125,9 +125,7 @@ __global__ void gated_clamp_vec_kernel(const __nv_bfloat16* __restrict__ gu, __n
             const float2 gf = __bfloat1622float2(gh[e]), uf = __bfloat1622float2(uh[e]);
             const float g0 = fminf(gf.x, limit), g1 = fminf(gf.y, limit);
             const float u0 = fminf(fmaxf(uf.x, -limit), limit), u1 = fminf(fmaxf(uf.y, -limit), limit);
-            // the division by the fast unit: its error (2^-22) is far below the bfloat16 rounding that follows
-            rh[e] = __floats2bfloat162_rn(__fdividef(g0, 1.0f + expf(-alpha * g0)) * (u0 + 1.0f),
-                                          __fdividef(g1, 1.0f + expf(-alpha * g1)) * (u1 + 1.0f));
+            rh[e] = __floats2bfloat162_rn(g0 / (1.0f + expf(-alpha * g0)) * (u0 + 1.0f), g1 / (1.0f + expf(-alpha * g1)) * (u1 + 1.0f));
         }
         *reinterpret_cast<uint4*>(out + row * inter + c) = res;
     }

@@ -222,3 +222,15 @@ def test_gated_gelu_rounds_a_row_as_its_other_forms_do():
     error = (wide.double() - want).abs()
     sound = (want.abs() > 1e-30) & (want.abs() < 1e30)
     assert bool((error <= want.abs() * (4.0 + 2.0 * exponent.clamp(min=0.0)) * 2.0 ** -23)[sound].all())
+
+
+def test_the_clamped_activation_rounds_a_row_as_its_other_forms_do():
+    """Every finite bfloat16 number through the kernel of 16 bytes a thread: the 32-bit kernel's result, rounded once."""
+    ops = runtime("bfloat16").ops
+    g = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    g = g[torch.isfinite(g)].cuda()
+    g = g[:g.numel() // 8 * 8].view(1, -1)
+    for seed in (52, 53, 54):
+        u = rand(g.shape, seed, 3.0).bfloat16()
+        wide, narrow = ops.gated_clamp(torch.cat([g, u], 1).float(), 1.702, 7.0), ops.gated_clamp(torch.cat([g, u], 1), 1.702, 7.0)
+        assert torch.equal(narrow, wide.bfloat16())
