@@ -267,6 +267,15 @@ class Ops:
             return _RAW_STREAM(_DEVICE())
         return torch.cuda.current_stream().cuda_stream
 
+    @staticmethod
+    def _room_for(floats: int, device):
+        """Scratch that a faster form of a call wants and a slower one does without: None where the GPU has no room for it, as
+        when a session has given its memory to pages."""
+        try:
+            return torch.empty(floats, dtype=torch.float32, device=device)
+        except torch.OutOfMemoryError:
+            return None
+
     def _check(self, code: int, what: str) -> None:
         self.launches += 1
         if code:
@@ -611,7 +620,7 @@ class Ops:
         out = torch.empty((M, N), dtype=torch.float32 if out_float32 else a.dtype, device=a.device)
         a = a.contiguous()
         floats = self.lib.sb_gemm_general_scratch(M, N, K)
-        parts = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
+        parts = self._room_for(floats, a.device) if floats else None   # without: the chunks of k one after another, the same sums
         self._check(self.lib.sb_gemm_general(_code(a.dtype), int(out_float32 or a.dtype == torch.float32), _ptr(a), _ptr(w),
                                              _ptr(out), M, N, K, _ptr(parts), self._stream()), "gemm_general")
         return out
@@ -1193,14 +1202,16 @@ class Ops:
                      cap=0.0, q_scale=1.0, out_scale=1.0, last=None, last_offset=0) -> bool:
         """The recurrence of wkv_scan, gla_scan or mlstm_scan over 64 tokens at a time, all chunks side by side
         (chunk_memory.cu); False, with nothing done, where the walk token by token has to do it: 32-bit runs, heads of more
-        than 128 channels, and steps that it does sooner."""
+        than 128 channels, steps that it does sooner, and a GPU too full for the chunks' workspace."""
         rows = q.shape[0]
         if q.dtype != torch.bfloat16 or not self.chunk_memory_pays(ctx.n_seqs, rows, ctx.max_q_len, H, V):
             return False
         floats = self.lib.sb_chunk_memory_floats(kind, rows, ctx.n_seqs, H, D, V)
         if floats < 0:
             return False
-        work = torch.empty(floats, dtype=torch.float32, device=q.device)
+        work = self._room_for(floats, q.device)
+        if work is None:
+            return False
         a = SbChunkMem(_ptr(q), _ptr(k), _ptr(v), _ptr(g), ld, _ptr(z), z.stride(0), int(z_cols[0]), int(z_cols[1]), _ptr(bias), _ptr(bias2),
                        _ptr(norm), norm_stride, float(eps), float(inv_tau), float(cap), float(q_scale), float(out_scale), _ptr(state),
                        state.stride(0), _ptr(last), last.shape[1] if last is not None else 0, int(last_offset), _ptr(y), y.stride(0),

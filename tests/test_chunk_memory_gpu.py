@@ -196,3 +196,50 @@ def test_a_walk_of_many_sequences_leaves_what_each_alone_does(H, D, V, counts):
     finally:
         del ops.force_chunk_memory
     assert torch.equal(together[n], state[n])
+
+
+@pytest.fixture
+def little_room():
+    """Leaves the allocator 60 MB beyond what it holds, then everything again."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+
+    def limit():
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 60 * 2 ** 20) / total)
+    yield limit
+    torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def test_a_step_without_room_for_the_chunks_is_walked(little_room):
+    from starter_b200.csrc.ops import get_ops
+    ops, H, D, V, rows = get_ops(verbose=False), 16, 64, 128, 3333
+    ctx, _ = batch_of([rows], [0], 1)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")   # noqa: E731
+    p = rand(rows, 2 * H * (D + V)).bfloat16()
+    views = p.split([H * D, H * D, H * V, H * V], 1)
+    z, bias, norm = rand(rows, 2 * H), rand(H), rand(H * V)
+    states = [torch.zeros(2, H * D * V + H * D + H, device="cuda") for _ in range(2)]
+    run = lambda st: ops.mlstm_scan(ctx, *views, z, 0, H, bias, bias, 15.0, norm, EPS, D ** -0.5, st, H, D, V)   # noqa: E731
+    assert 4 * ops.lib.sb_chunk_memory_floats(ops.CHUNK_MLSTM, rows, 1, H, D, V) > 60 * 2 ** 20
+    ops.force_chunk_memory = False
+    try:
+        want = run(states[0])
+    finally:
+        del ops.force_chunk_memory
+    little_room()
+    assert ops.chunk_memory_pays(1, rows, rows, H, V)
+    assert torch.equal(run(states[1]), want) and torch.equal(states[0], states[1])
+
+
+def test_a_product_without_room_for_its_chunks_of_k_takes_them_in_order(little_room):
+    from starter_b200.csrc.ops import get_ops
+    ops, (M, N, K) = get_ops(verbose=False), (300, 19456, 2560)
+    g = torch.Generator(device="cuda").manual_seed(4)
+    a, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    assert 4 * ops.lib.sb_gemm_general_scratch(M, N, K) > 60 * 2 ** 20
+    want = ops.linear(a, w)
+    little_room()
+    assert torch.equal(ops.linear(a, w), want)
