@@ -385,9 +385,10 @@ static void gg_pick(const void* A, const void* W, void* C, int M, int N, int K, 
 
 extern "C" {
 
-// Floats of scratch that a product wants, 0 when its chunks of k run in one block.  Without them it does that too.
-long long sb_gemm_general_scratch(int M, int N, int K) {
-    if (M <= 0 || N <= 0) return 0;
+// Floats of scratch that a product wants, 0 when its chunks of k run in one block.  Without them it does that too; with them it
+// is two kernels.
+long long sb_gemm_general_scratch(int dtype, int M, int N, int K) {
+    if (M <= 0 || N <= 0 || (dtype != SB_F32 && (long long)M * N <= GG_DOT_MAX)) return 0;
     return gg_plan(M, N, K, true).apart ? (long long)M * N * ((K + GG_CHUNK - 1) / GG_CHUNK) : 0;
 }
 

@@ -231,7 +231,7 @@ class Ops:
         lib.sb_chunk_memory_floats.restype = c_longlong
         lib.sb_delta_chunk_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.sb_delta_chunk_floats.restype = c_longlong
-        lib.sb_gemm_general_scratch.argtypes = [c_int, c_int, c_int]
+        lib.sb_gemm_general_scratch.argtypes = [c_int, c_int, c_int, c_int]
         lib.sb_gemm_general_scratch.restype = c_longlong
         lib.sb_set_pdl.argtypes = [c_int]
         lib.sb_set_pdl.restype = None
@@ -619,10 +619,12 @@ class Ops:
                 return torch.mm(a, w.t())
         out = torch.empty((M, N), dtype=torch.float32 if out_float32 else a.dtype, device=a.device)
         a = a.contiguous()
-        floats = self.lib.sb_gemm_general_scratch(M, N, K)
+        floats = self.lib.sb_gemm_general_scratch(_code(a.dtype), M, N, K)
         parts = self._room_for(floats, a.device) if floats else None   # without: the chunks of k one after another, the same sums
         self._check(self.lib.sb_gemm_general(_code(a.dtype), int(out_float32 or a.dtype == torch.float32), _ptr(a), _ptr(w),
                                              _ptr(out), M, N, K, _ptr(parts), self._stream()), "gemm_general")
+        if parts is not None:
+            self.launches += 1   # the chunks' sums are added up
         return out
 
     def linear_swiglu(self, h, w_gate_up, norm=None):

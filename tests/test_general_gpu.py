@@ -97,3 +97,13 @@ def test_product_32_bit_whatever_the_tile(ops, M, N, K):
         got = ops.linear(a.bfloat16(), w.bfloat16(), out_float32=True)
         want = a.bfloat16().double() @ w.bfloat16().double().T
         assert float((got - want).norm() / want.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("M, N, K, dtype, kernels", [(300, 2560, 4096, "float32", 2), (300, 600, 500, "float32", 1), (4, 300, 2560, "float32", 2),
+                                                     (20, 100, 1030, "bfloat16", 1), (200, 200, 1030, "bfloat16", 2), (200, 200, 100, "bfloat16", 1)])
+def test_the_count_of_launches(ops, M, N, K, dtype, kernels):
+    """Chunks of k side by side and the kernel that adds them up are two; a warp per output, or all chunks in one block, is one."""
+    a, w = rand((M, K), 1).to(getattr(torch, dtype)), rand((N, K), 2).to(getattr(torch, dtype))
+    before = ops.launches
+    ops.linear(a, w)
+    assert ops.launches - before == kernels
