@@ -62,6 +62,7 @@ struct SbChunkMem {
     void* y;
     long long y_ld;
     float* work;            // sb_chunk_memory_floats() floats
+    long long head_floats;  // as given to sb_chunk_memory_floats()
     int H;
     int D;
     int V;
@@ -905,16 +906,17 @@ static long long cm_head_floats(long long cells, int D, int V) {
 
 static long long cm_gate_floats(int kind, long long rows, int H, int D) { return (rows * H * (kind == CM_MLSTM ? 3 : D) + 3) / 4 * 4; }
 
-// Heads that are worked on together: as many as keep the workspace within 512 MB (at least one).
-static int cm_heads(long long cells, int H, int D, int V) {
-    const long long fit = (128ll << 20) / cm_head_floats(cells, D, V);
+// Heads that are worked on together: as many as keep their share of the workspace, states and normalisers, within head_floats (at
+// least one).  The gates or decays of all rows and heads, cm_gate_floats, come on top.
+static int cm_heads(long long head_floats, long long cells, int H, int D, int V) {
+    const long long fit = head_floats / cm_head_floats(cells, D, V);
     return fit < 1 ? 1 : (fit < H ? (int)fit : H);
 }
 
 template <int KIND, int DP, int VP>
 static int launch_chunk_memory(SbChunkMem a, SbBatch batch, int vec, cudaStream_t stream) {
     const long long cells = batch.n_rows / CM_L + batch.n_seqs;
-    const int per = cm_heads(cells, a.H, a.D, a.V);
+    const int per = cm_heads(a.head_floats, cells, a.H, a.D, a.V);
     constexpr size_t states_smem = (size_t)CM_L * (DP + 4) * 4 * (KIND == CM_MLSTM ? 1 : 2) + (size_t)CM_L * (VP + 8) * 2;
     constexpr size_t out_smem = outputs_smem<KIND, DP, VP>();
     cudaError_t err = cudaFuncSetAttribute(chunk_states_kernel<KIND, DP, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)states_smem);
@@ -944,16 +946,23 @@ static int launch_chunk_memory(SbChunkMem a, SbBatch batch, int vec, cudaStream_
 
 extern "C" {
 
-// Floats of workspace for a step of n_rows rows of n_seqs sequences, or -1 for heads that these kernels do not take.
-long long sb_chunk_memory_floats(int kind, int n_rows, int n_seqs, int H, int D, int V) {
+// Floats of workspace for a step of n_rows rows of n_seqs sequences whose heads may take head_floats of them together, or -1 for heads
+// that these kernels do not take.
+long long sb_chunk_memory_floats(int kind, int n_rows, int n_seqs, int H, int D, int V, long long head_floats) {
     if (n_rows < 1 || n_seqs < 1 || H < 1 || H > 65535 || D < 1 || V < 1 || D > 128 || V > 128 || (kind == CM_WKV && D != V)) return -1;
     const long long cells = n_rows / CM_L + n_seqs;
-    return cm_gate_floats(kind, n_rows, H, D) + cm_heads(cells, H, D, V) * cm_head_floats(cells, D, V);
+    return cm_gate_floats(kind, n_rows, H, D) + cm_heads(head_floats, cells, H, D, V) * cm_head_floats(cells, D, V);
+}
+
+// Kernels that such a step launches.
+int sb_chunk_memory_launches(int kind, int n_rows, int n_seqs, int H, int D, int V, long long head_floats) {
+    const int per = cm_heads(head_floats, n_rows / CM_L + n_seqs, H, D, V);
+    return (H + per - 1) / per * (kind == CM_MLSTM ? 4 : 3);   // the gates, the chunks' shares, the walk over them, the outputs
 }
 
 int sb_chunk_memory(int kind, SbChunkMem a, SbBatch batch, cudaStream_t stream) {
     if (batch.n_seqs <= 0 || batch.n_rows <= 0) return 0;
-    if (sb_chunk_memory_floats(kind, batch.n_rows, batch.n_seqs, a.H, a.D, a.V) < 0 || a.work == nullptr
+    if (sb_chunk_memory_floats(kind, batch.n_rows, batch.n_seqs, a.H, a.D, a.V, a.head_floats) < 0 || a.work == nullptr
         || (kind == CM_GLA && !(a.inv_tau > 0.f)) || (kind == CM_MLSTM && !(a.cap > 0.f)))
         return (int)cudaErrorInvalidValue;
     const auto aligned = [](const void* p, size_t n) { return (reinterpret_cast<size_t>(p) & (n - 1)) == 0; };

@@ -64,8 +64,8 @@ class SbChunkMem(Structure):
                 ("z_ld", c_longlong), ("i_col", c_int), ("f_col", c_int), ("bias", c_void_p), ("bias2", c_void_p), ("norm", c_void_p),
                 ("norm_stride", c_int), ("eps", c_float), ("inv_tau", c_float), ("cap", c_float), ("q_scale", c_float),
                 ("out_scale", c_float), ("state", c_void_p), ("state_stride", c_longlong), ("last", c_void_p), ("last_width", c_int),
-                ("last_offset", c_int), ("y", c_void_p), ("y_ld", c_longlong), ("work", c_void_p), ("H", c_int), ("D", c_int),
-                ("V", c_int)]
+                ("last_offset", c_int), ("y", c_void_p), ("y_ld", c_longlong), ("work", c_void_p),
+                ("head_floats", c_longlong), ("H", c_int), ("D", c_int), ("V", c_int)]
 
 
 class SbDecay(Structure):
@@ -199,6 +199,7 @@ class Ops:
                            c_int, c_void_p],
             "sb_moe_combine": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                c_int, c_void_p, c_int, c_void_p],
+            "sb_chunk_memory_launches": [c_int, c_int, c_int, c_int, c_int, c_int, c_longlong],
             "sb_chunk_memory": [c_int, SbChunkMem, SbBatch, c_void_p],
             "sb_decay_step": [c_int, SbDecay, SbBatch, c_void_p, c_int, c_void_p],
             "sb_decay_chunk": [SbDecay, SbBatch, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p],
@@ -227,7 +228,7 @@ class Ops:
                    lib.sb_talking_decode_smem):
             fn.argtypes = [c_int, c_int, c_int, c_int]
             fn.restype = c_longlong
-        lib.sb_chunk_memory_floats.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int]
+        lib.sb_chunk_memory_floats.argtypes = [c_int, c_int, c_int, c_int, c_int, c_int, c_longlong]
         lib.sb_chunk_memory_floats.restype = c_longlong
         lib.sb_delta_chunk_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
         lib.sb_delta_chunk_floats.restype = c_longlong
@@ -1186,6 +1187,7 @@ class Ops:
 
     CHUNK_WKV, CHUNK_GLA, CHUNK_MLSTM = 0, 1, 2
     force_chunk_memory = None   # True or False for tests and tuning; None = the rule below
+    chunk_head_floats = 128 << 20   # floats of workspace (512 MB) that the heads of a step may take; beyond, they go in groups
 
     def chunk_memory_pays(self, n_seqs: int, rows: int, max_q_len: int, H: int, V: int) -> bool:
         """Whether a step of this shape is sooner done in chunks than token by token.  The walk is a chain over the longest
@@ -1193,7 +1195,9 @@ class Ops:
         one per chunk and head.  The three rates below are fits to (us, walk / chunks): 32 heads of 64 x 64 (wkv), one sequence of
         64 / 128 / 256 / 2,048 rows: 34 / 33, 62 / 34, 118 / 38, 903 / 113, 16 of 64 and 128 rows: 93 / 75, 172 / 123, 64 of 16 and 64
         rows: 97 / 171, 325 / 246; 16 heads of 64 x 128, one of 64 / 128 / 3,333 rows: gla 32 / 39, 55 / 39, 1,277 / 140, mlstm 32 / 34,
-        55 / 34, 1,135 / 118, 64 of 16 and 64 rows: gla 99 / 152, 320 / 214, mlstm 154 / 181, 385 / 183."""
+        55 / 34, 1,135 / 118, 64 of 16 and 64 rows: gla 99 / 152, 320 / 214, mlstm 154 / 181, 385 / 183.  Over 1,344 steps of 1 to
+        100 sequences of equal and unequal lengths, 8 to 32 heads of all three, the chunks were chosen and slower once (64 rows of 8
+        heads, gla: 29 / 34); the walk was in 173 (mlstm, 16 heads, eight sequences of up to 150 rows: 112 / 44)."""
         if self.force_chunk_memory is not None:
             return self.force_chunk_memory
         chunks = rows / 64 + n_seqs / 2
@@ -1208,7 +1212,7 @@ class Ops:
         rows = q.shape[0]
         if q.dtype != torch.bfloat16 or not self.chunk_memory_pays(ctx.n_seqs, rows, ctx.max_q_len, H, V):
             return False
-        floats = self.lib.sb_chunk_memory_floats(kind, rows, ctx.n_seqs, H, D, V)
+        floats = self.lib.sb_chunk_memory_floats(kind, rows, ctx.n_seqs, H, D, V, self.chunk_head_floats)
         if floats < 0:
             return False
         work = self._room_for(floats, q.device)
@@ -1217,9 +1221,9 @@ class Ops:
         a = SbChunkMem(_ptr(q), _ptr(k), _ptr(v), _ptr(g), ld, _ptr(z), z.stride(0), int(z_cols[0]), int(z_cols[1]), _ptr(bias), _ptr(bias2),
                        _ptr(norm), norm_stride, float(eps), float(inv_tau), float(cap), float(q_scale), float(out_scale), _ptr(state),
                        state.stride(0), _ptr(last), last.shape[1] if last is not None else 0, int(last_offset), _ptr(y), y.stride(0),
-                       _ptr(work), H, D, V)
+                       _ptr(work), self.chunk_head_floats, H, D, V)
         self._check(self.lib.sb_chunk_memory(kind, a, self._batch(ctx), self._stream()), "chunk_memory")
-        self.launches += 3 if kind == self.CHUNK_MLSTM else 2   # the gates, the chunks' shares, the walk over them, the outputs
+        self.launches += self.lib.sb_chunk_memory_launches(kind, rows, ctx.n_seqs, H, D, V, self.chunk_head_floats) - 1
         return True
 
     # ---- a residual in streams, two-map attention, gated linear attention, experts -------

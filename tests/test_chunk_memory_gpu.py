@@ -223,7 +223,7 @@ def test_a_step_without_room_for_the_chunks_is_walked(little_room):
     z, bias, norm = rand(rows, 2 * H), rand(H), rand(H * V)
     states = [torch.zeros(2, H * D * V + H * D + H, device="cuda") for _ in range(2)]
     run = lambda st: ops.mlstm_scan(ctx, *views, z, 0, H, bias, bias, 15.0, norm, EPS, D ** -0.5, st, H, D, V)   # noqa: E731
-    assert 4 * ops.lib.sb_chunk_memory_floats(ops.CHUNK_MLSTM, rows, 1, H, D, V) > 60 * 2 ** 20
+    assert 4 * ops.lib.sb_chunk_memory_floats(ops.CHUNK_MLSTM, rows, 1, H, D, V, ops.chunk_head_floats) > 60 * 2 ** 20
     ops.force_chunk_memory = False
     try:
         want = run(states[0])
@@ -243,3 +243,19 @@ def test_a_product_without_room_for_its_chunks_of_k_takes_them_in_order(little_r
     want = ops.linear(a, w)
     little_room()
     assert torch.equal(ops.linear(a, w), want)
+
+
+@pytest.mark.parametrize("kind", ["wkv", "gla", "mlstm"])
+@pytest.mark.parametrize("together", [1, 2, 4])
+def test_heads_in_groups(monkeypatch, kind, together):
+    """A workspace for fewer heads than the layer has: the same numbers as with all heads at once, the last group smaller."""
+    from starter_b200.csrc.ops import get_ops
+    ops, H, D, V, counts = get_ops(verbose=False), 5, 64, 64, [150, 3, 70]
+    ((y, st), _), _, _ = run_kind(kind, H, D, V, counts, 1.0, 0)
+    cells = sum(counts) // 64 + len(counts)
+    monkeypatch.setattr(ops, "chunk_head_floats", together * cells * (D * V + 3 * D * V // 2 + 2 * D))
+    codes = (sum(counts), len(counts), H, D, V, ops.chunk_head_floats)
+    code = {"wkv": ops.CHUNK_WKV, "gla": ops.CHUNK_GLA, "mlstm": ops.CHUNK_MLSTM}[kind]
+    assert ops.lib.sb_chunk_memory_launches(code, *codes) == -(-H // together) * (4 if kind == "mlstm" else 3)
+    ((few, st_few), _), _, _ = run_kind(kind, H, D, V, counts, 1.0, 0)
+    assert torch.equal(few, y) and torch.equal(st_few, st)
