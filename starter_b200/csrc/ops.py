@@ -1666,7 +1666,8 @@ class Ops:
 
     MOE_PAIRS_MAX = int(os.environ.get("STARTER_B200_MOE_PAIRS_MAX", 64))   # pairs up to which every pair streams its expert
 
-    MOE_FEW_MAX = int(os.environ.get("STARTER_B200_MOE_FEW_MAX", 512))   # pairs up to which moe_few.cu serves a step
+    MOE_FEW_TAKES = 1024   # pairs that a block of moe_few.cu lists
+    MOE_FEW_MAX = min(int(os.environ.get("STARTER_B200_MOE_FEW_MAX", 512)), MOE_FEW_TAKES)   # pairs up to which moe_few.cu serves a step
 
     def _moe_takes_few(self, h, pairs, n_experts, width, ff, w_gate_up, w_down) -> bool:
         """The kernel of an expert at a time (moe_few.cu).  With fewer pairs than experts hardly two pairs share one, and a

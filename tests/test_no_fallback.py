@@ -42,3 +42,14 @@ def test_a_source_that_does_not_compile_is_an_error_with_the_compiler_s_words(mo
     monkeypatch.setenv("STARTER_B200_BUILD_DIR", str(tmp_path / "out"))
     with pytest.raises(BuildError, match="nvcc failed on broken.cu"):
         build.load(verbose=False)
+
+
+def test_a_setting_beyond_what_a_kernel_lists_does_not_reach_it():
+    """More pairs of a step's experts than the kernel for few takes go to the kernels for many, whatever the variable says."""
+    import os
+    import subprocess
+    import sys
+    code = "from starter_b200.csrc.ops import Ops; print(Ops.MOE_FEW_MAX, Ops.MOE_FEW_TAKES)"
+    for value, want in (("5000", "1024 1024"), ("700", "700 1024"), ("0", "0 1024")):
+        run = subprocess.run([sys.executable, "-c", code], env={**os.environ, "STARTER_B200_MOE_FEW_MAX": value}, capture_output=True, text=True)
+        assert run.stdout.strip() == want, run.stderr
