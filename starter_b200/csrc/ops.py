@@ -1671,12 +1671,17 @@ class Ops:
 
     def _moe_takes_few(self, h, pairs, n_experts, width, ff, w_gate_up, w_down) -> bool:
         """The kernel of an expert at a time (moe_few.cu).  With fewer pairs than experts hardly two pairs share one, and a
-        block per pair is ahead (up to the 64 pairs it is built for); beyond some 32 pairs an expert the weights are read too
-        often and the grouped product is.  Measured (us a layer, pair by pair / this / grouped): 16 experts of 3 x 1,024 x 512: 8
+        block per pair is ahead (up to the 64 pairs it is built for).  Weights are read once for every 16 pairs of an expert: of a layer
+        that stays in L2 (126 MB) the second time costs little and the grouped product is ahead from some 32 pairs an expert on, of
+        larger ones from 20, beyond 600 MB from 14 (this / grouped: 16 experts of 3 x 1,024 x 4,096, 16 pairs an expert 113 / 122, 24
+        141 / 124, 32 181 / 122; 16 of 3 x 2,048 x 1,024, 24 an expert 83 / 82, 32 94 to 102 / 79; 8 of 3 x 4,096 x 1,408, 16 an expert 80 / 110,
+        24 108 to 116 / 108, 32 130 / 110; 32 of them, 12 an expert 231 / 258, 16 288 / 260).  Measured (us a layer, pair by pair / this / grouped): 16 experts of 3 x 1,024 x 512: 8
         pairs 13 / 14 / 38, 16: 18 / 16 / 39, 64: 39 / 20 / 41, 96: 52 / 21 / 42, 256: - / 28 / 42, 512: - / 39 / 42, 768: - / 51 /
         43; 32 of 3 x 2,048 x 1,024: 16 pairs 40 / 42 / 72, 32: 57 / 53 / 92, 64: 110 / 65 / 96, 96: 157 / 78 / 114, 512: - / 113 /
         123, 768: - / 150 / 120."""
-        if self.MOE_FEW_MAX < pairs or pairs > 32 * n_experts or pairs < min(n_experts, self.MOE_PAIRS_MAX + 1):
+        weights = 6 * n_experts * width * ff   # bytes
+        most = 32 if weights <= 150e6 else 20 if weights <= 600e6 else 14
+        if self.MOE_FEW_MAX < pairs or pairs > most * n_experts or pairs < min(n_experts, self.MOE_PAIRS_MAX + 1):
             return False
         return (h.dtype == torch.bfloat16 and width % 32 == 0 and ff % 32 == 0 and h.is_contiguous() and h.data_ptr() % 16 == 0
                 and w_gate_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)

@@ -132,3 +132,13 @@ def test_groups_whose_outputs_are_shut_out_or_forced(out, forced, scores):
         few = ops.moe_route(h[:9].contiguous(), router, correction.cuda(), 4, 1.0, **kind)
         assert torch.equal(few[0], many[0][:9]), keep
         assert float((few[1] - many[1][:9]).abs().max()) <= 1e-6
+
+
+def test_the_rule_where_an_expert_s_weights_are_read_more_than_once():
+    from starter_b200.csrc.ops import get_ops
+    ops = get_ops(verbose=False)
+    h, w = torch.zeros(8, 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(8, dtype=torch.bfloat16, device="cuda")
+    takes = lambda pairs, E, width, ff: ops._moe_takes_few(h, pairs, E, width, ff, w, w)   # noqa: E731
+    assert [takes(n, 16, 1024, 512) for n in (320, 512)] == [True, True]            # 50 MB
+    assert [takes(n, 16, 1024, 4096) for n in (320, 321)] == [True, False]         # 403 MB
+    assert [takes(n, 32, 4096, 1408) for n in (448, 449)] == [True, False]         # 1.1 GB
