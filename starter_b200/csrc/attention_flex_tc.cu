@@ -1,7 +1,10 @@
 // The attention of attention_flex.cu for prompts on the Blackwell tensor cores: S = Q K^T and O = P V by tcgen05.mma, S, P
-// and O in tensor memory, keys and values brought in by TMA.  Key widths of 64, 96, 128 and 192 columns, values of 64 or
-// 128, bfloat16; any number of query heads per key/value head; every option of the call (scale, per-head temperature,
-// distance penalty, window, chunk, sink, fewer value heads than key heads, values inside the key rows).
+// and O in tensor memory, keys and values brought in by TMA, bfloat16.  Two entries:
+//   sb_flex_attention_tc        cache pages, key widths of 64 or 128 columns, values of 64 or 128; any number of query heads per
+//                               key/value head; every option of the call (scale, per-head temperature, distance penalty, window,
+//                               chunk, sink, fewer value heads than key heads, values inside the key rows) but pinned pages;
+//   sb_flex_attention_tc_rows   the step's own rows, one key head per query head, 64 + 32 key columns with values of 64 or 128 + 64
+//                               with values of 128; scale and sink.  Other widths have no such form here.
 //
 // The work is laid out as in attn_prefill_tc.cu, where the reasons are measured: a block owns 128 (position, query head of
 // the group) rows of one sequence and key/value head, one row per thread and per lane of tensor memory; one thread of a
@@ -10,7 +13,12 @@
 // start longest first across all heads.  What differs:
 //   * a weight w meets its value as two bfloat16 numbers hi + lo (hi = bf16(w), lo = bf16(w - hi)), so that it keeps 16
 //     bits, as in attention_flex_mma.cu: hi and lo take the two halves of the S buffer they came from, and eight products
-//     (instead of four) read them from there;
+//     (instead of four) read them from there.  w is one instruction (ex2.approx, 2^-22) where that kernel calls expf: next to the
+//     weight's 16 bits the difference is nothing.  Errors against 64 bits over 200 to 3,333 rows, up to 9,200 keys, scores of
+//     size 1 to 8, with sink, window, temperature and penalty: that kernel / this / this with expf 1.607334e-3 / 1.607334e-3 /
+//     1.607334e-3, 1.656125e-3 / 1.656126e-3 / 1.656126e-3, at most 1.645750e-3 / 1.645765e-3 / 1.645770e-3 (200 rows behind 9,000
+//     keys), the largest error the same in all; with expf a call takes 14 to 28% longer (2,048 rows of 16 heads on 8 of
+//     128 47.6 -> 54.7 us, with temperature and penalty 57.9 -> 72.4);
 //   * with a temperature or a penalty per head (BIASED) the scores are finished before their maximum is taken;
 //   * DENSE: keys and values are not in cache pages but rows of the step itself, every sequence at its start: a key is a
 //     head's own columns of one matrix beside columns of another that all heads share (a latent layer's plain and rotated

@@ -186,3 +186,16 @@ def test_the_plain_prompt_kernel_far_into_a_long_context(held):
     # that kernel's weights meet the values rounded to bfloat16: 2^-9 each, averaging out over thousands of keys
     got = got.view(rows, H, D).to(F)
     assert float((got - want).norm() / want.norm()) < 5e-3 and float((got - want).abs().max() / want.abs().max()) < 2e-2
+
+
+@pytest.mark.parametrize("D, V", [(128, 64), (128, 128), (64, 64)])
+@pytest.mark.parametrize("held, rows", [(0, 129), (70, 257)])
+def test_values_inside_the_key_rows(D, V, held, rows):
+    rt, H, G = runtime(), 6, 2
+    ctx, layer, k, _, rnd = long_context(rt, G, D, D, held, rows)
+    q = rnd(rows, H, D)
+    p = rt.ops._flex(layer, q, H, D ** -0.5, V, True)
+    assert rt.ops._flex_takes_tc(ctx, q, p)
+    got = rt.ops.flex_attention(ctx, q, layer, D ** -0.5, v_dim=V, values_in_keys=True)
+    assert rt.ops.read_kernel_status() == 0
+    close(got, oracle(q, k, k[:, :, :V], held, D ** -0.5, lambda h: h * G // H), f"values of {V} columns in keys of {D}")
