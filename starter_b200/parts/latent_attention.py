@@ -38,6 +38,17 @@ from ..cache.cache import PAGE, KVGroup, KVRequest, LayerCache, SharedRequest
 from .registry import build_part, register_part
 
 NARROW_MIN_ROWS = 64   # a first step of fewer rows stays on the one path that serves every step
+# A tile of the narrow form's attention is 128 rows of one sequence and head.  Several sequences of few rows each fill it with
+# padding (device us of a whole step of 64 sequences, the path that serves every step / narrow): 2 rows each 768 / 793 and 1,006 / 1,054
+# (six layers of 2,048 with two and four of them latent), 8 rows each 1,056 / 1,013 and 1,649 / 1,543.
+NARROW_MIN_EACH = 8
+
+
+def takes_narrow(ctx, rows, in_place):
+    """Whether a step takes the narrow form: nothing cached before it, and rows enough, in all and on average a sequence."""
+    if rows < NARROW_MIN_ROWS:
+        return False
+    return (ctx.n_seqs == 1 and ctx.kv_bound == rows) or (in_place and ctx.first and rows >= NARROW_MIN_EACH * ctx.n_seqs)
 
 
 class LatentAttention:
@@ -136,8 +147,7 @@ class LatentAttention:
         rows = h.shape[0]
         down = ops.linear(h, self.w_down)
         gate = down[:, self.gate_col:] if s.head_gate else None
-        first = (ctx.n_seqs == 1 and ctx.kv_bound == rows) or (ctx.first and self.in_place)   # nothing cached before the step
-        narrow = first and rows >= NARROW_MIN_ROWS
+        narrow = takes_narrow(ctx, rows, self.in_place)
         place = ("latent rows", id(layer_cache.group), layer_cache.index)                 # where the step's rows wait for their readers
         if not self.own_rows:
             cq, kept = ops.latent_prepare(ctx, down, None, s.q_rank, 0, 0, self.q_norm, None, self.eps), ctx.scratch.get(place)

@@ -180,3 +180,14 @@ def test_random_weights_from_the_command_line(tmp_path):
     assert sess.model.spec.vocab_size == 64 and len(sess.model.blocks) == 5
     seqs = random_tokens(64, (12,), seed=8)
     assert_close(run_whole(sess, seqs), cases.plain_logits(tmp_path / "model", seqs), "float32", "folder from the command line")
+
+
+@pytest.mark.parametrize("n_seqs, rows, kv_bound, first, in_place, want", [
+    (1, 64, 64, True, False, True), (1, 63, 63, True, True, False), (1, 64, 65, False, True, False), (1, 64, 64, True, True, True),
+    (8, 64, 8, True, True, True), (9, 64, 8, True, True, False), (64, 128, 2, True, True, False), (64, 512, 8, True, True, True),
+    (64, 512, 8, False, True, False), (64, 512, 8, True, False, False),
+])
+def test_which_first_steps_take_the_narrow_form(n_seqs, rows, kv_bound, first, in_place, want):
+    from types import SimpleNamespace
+    from starter_b200.parts.latent_attention import takes_narrow
+    assert takes_narrow(SimpleNamespace(n_seqs=n_seqs, kv_bound=kv_bound, first=first), rows, in_place) == want
