@@ -199,17 +199,15 @@ def test_a_walk_of_many_sequences_leaves_what_each_alone_does(H, D, V, counts):
 
 
 @pytest.fixture
-def little_room():
-    """Leaves the allocator 60 MB beyond what it holds, then everything again."""
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    total = torch.cuda.get_device_properties(0).total_memory
+def little_room(monkeypatch):
+    """Once called, the allocator has no room for more than 60 MB of floats at a time."""
+    empty = torch.empty
 
-    def limit():
-        torch.cuda.empty_cache()
-        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 60 * 2 ** 20) / total)
-    yield limit
-    torch.cuda.set_per_process_memory_fraction(1.0)
+    def limited(*size, dtype=None, **kwargs):
+        if dtype == torch.float32 and len(size) == 1 and isinstance(size[0], int) and 4 * size[0] > 60 * 2 ** 20:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*size, dtype=dtype, **kwargs)
+    return lambda: monkeypatch.setattr(torch, "empty", limited)
 
 
 def test_a_step_without_room_for_the_chunks_is_walked(little_room):
