@@ -18,16 +18,11 @@
 // One block per SM: warp 0 = TMA producer, warp 1 = MMA issuer and tensor-memory owner, warps 2-5 =
 // epilogue.  Every wait on an mbarrier gives up after a bounded time, raises SB_STATUS_TIMEOUT in the
 // status word, and the block leaves through its normal teardown (tensor memory freed).
-#include <cuda.h>
-#include <stdio.h>
-
-#include <mutex>
-#include <unordered_map>
-
+#include "tc_maps.cuh"
 #include "tc_utils.cuh"
 
 #define ST_BM 128               // rows of W per tile
-#define ST_BK 64                // columns of K per stage: 128 bytes, one swizzle span
+#define ST_BK 64                // columns of K per stage: 128 bytes, one swizzle span and a box of make_rows_map
 #define ST_THREADS 192
 
 __device__ __forceinline__ float silu_mul_rounded(float g, float u) {
@@ -326,38 +321,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
 // ---- host side ----------------------------------------------------------------------------------
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    });
-    return fn;
-}
-
-// A [rows, K] row-major bfloat16 matrix seen as boxes of box_rows x 64 columns, 128-byte swizzle,
-// zero fill outside the matrix.
-static int make_map(CUtensorMap* map, const void* ptr, long long rows, long long K, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return (int)cudaErrorNotSupported;
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    cuuint32_t box[2] = {ST_BK, (cuuint32_t)box_rows};
-    cuuint32_t elem[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
-}
-
 template <int BN, bool GU, int STAGES>
 static int launch_stream(const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensorMap& ma, StreamArgs args, int grid,
                          cudaStream_t stream) {
@@ -402,11 +365,11 @@ int sb_gemm_stream(const void* A, const void* W, void* C, int M, int n_out, int 
     if (M > 64 || (K & 7) || (gate_up && M > 32) || grid < 1) return (int)cudaErrorInvalidValue;
     const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
     CUtensorMap mw, mw2, ma;
-    int e = make_map(&mw, W, n_out, K, ST_BM);
+    int e = make_rows_map(&mw, W, n_out, K, K, ST_BM);
     if (e) return e;
-    e = make_map(&mw2, gate_up ? (const void*)((const __nv_bfloat16*)W + (long long)n_out * K) : W, n_out, K, ST_BM);
+    e = make_rows_map(&mw2, gate_up ? (const void*)((const __nv_bfloat16*)W + (long long)n_out * K) : W, n_out, K, K, ST_BM);
     if (e) return e;
-    e = make_map(&ma, A, M, K, bn);
+    e = make_rows_map(&ma, A, M, K, K, bn);
     if (e) return e;
     StreamArgs args;
     args.C = C; args.partial = partial; args.counters = counters; args.status = status;
