@@ -4,16 +4,16 @@
 // the bfloat16 path for shapes the tensor-core kernels refuse.  The reference's products are `x @ W.T` with W as
 // [out, in] (engine/model.py:291,295,297,299).
 //
-// Each output element is the sum, in order, of the sums over GG_CHUNK columns of k, each of them one running sum in
-// order: a function of K alone, so a row's result does not depend on how many other rows the call has, nor on which of
-// the tiles below took it, nor on whether the chunks ran side by side.
+// Each output element of a 32-bit product is the sum, in order, of the sums over GG_CHUNK columns of k, each of them one running
+// sum in order: a function of K alone, so a row's result does not depend on how many other rows the call has, nor on which of
+// the tiles below took it, nor on whether the chunks ran side by side.  So it is in bfloat16 from GG_DOT_MAX outputs on; up to there
+// the sums run along a warp's lanes, and a row's bits depend on which side of that the call's outputs lie.
 //
 // Bound: the 32-bit multiply-adds (148 SMs x 128 a clock: 74 TFLOP/s at 1,965 MHz).  A block of 256 threads owns a tile of
 // BM x BN, a thread TM x TN of it as pairs (`fma.rn.f32x2`: half the instructions, which leaves issue slots for the
 // shared-memory reads); 16 columns of k at a time through two shared-memory buffers, the next ones in registers while
-// a tile is worked on.  Rows of few activations take a tile of 8, 32 or 64 rows, so that a product of a few rows streams
-// its weights instead of working for padding.  Where the tiles do not fill the GPU, the chunks of k run as blocks of
-// their own and a second kernel adds them up in order (`SPLIT`).
+// a tile is worked on.  Tiles have 8, 32, 64 or 128 rows, and the chunks of k may run as blocks of their own, added up in order
+// by a second kernel (`SPLIT`): gg_plan says which.
 // Measured (B200, 32-bit; the kernel before had one tile of 64 x 64 with scalar loads: 12 TFLOP/s at 300 rows): 300 rows of
 // [6144, 2560] 245 us (38 TFLOP/s), [2560, 4096] 196, [19456, 2560] 759, [2560, 9728] 382; 2,048 rows of [19456, 2560] 4.06 ms
 // (50 TFLOP/s); one row of [151936, 2560] 275 us (5.7 TB/s); 300 rows' error against 64 bits 4.1e-7.
