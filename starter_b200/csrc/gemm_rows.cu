@@ -1,0 +1,369 @@
+// Products of many rows, C[M, N] = A[M, K] W[N, K]^T in bfloat16 with 32-bit sums, on tcgen05, with what follows the product in its
+// epilogue: the gated activations of a [gate; up] matrix, or the squared relu or the two-sided activation of a plain one; and per expert,
+// over rows that are sorted by expert.  The reference's products are `x @ W.T` (engine/model.py:291,295,297,299), its activation a
+// kernel of its own (engine/kernels/swiglu.py:13-25).
+//
+// A pair of blocks (a cluster of two SMs) owns tiles of 256 rows x BN columns of sums: each loads its 128 rows of A and half of the
+// tile's rows of W by TMA, 128 columns of k at a time through a ring of stages, one thread of the first block issues the products of both
+// (cta_group::2, so that each SM reads half of W from its neighbour's shared memory), each holds its rows' sums in tensor memory,
+// twice, so that the warps behind take a tile out while the next is summed.  Pairs walk the tiles from their own number on, a group of
+// row tiles side by side, so that what runs at one time shares its rows of A and W in L2.
+#include "tc_maps.cuh"
+#include "tc_utils.cuh"
+
+#define GT_MAX_EXPERTS 1024
+#define GT_GROUP 32       // row tiles side by side: 8 read W once more for every 2,048 rows (4,500 rows of [2 x 9,728, 2,560]: 308 us, so 298)
+
+enum { GT_PLAIN = 0, GT_SWIGLU = 1, GT_CLAMP = 2, GT_GELU = 3, GT_RELU2 = 4, GT_XIELU = 5 };
+
+struct GtArgs {
+    void* out;
+    const int* ends;      // grouped: rows of expert e end at ends[e] (and start where e - 1 ends)
+    int* status;
+    int M, N, K;          // N: output columns (half of W's rows for a gated pair)
+    int n_experts;
+    int m_tiles, n_tiles;
+    float alpha, limit;
+};
+
+__host__ __device__ constexpr bool gt_gated(int epi) { return epi == GT_SWIGLU || epi == GT_CLAMP || epi == GT_GELU; }
+
+template <int CG, int BN, int EPI = GT_PLAIN> struct GtShape {
+    // Warp 0 copies, warp 1 issues products, the rest take tiles out.  Exponentials and divisions at full precision are chains of
+    // their own: only more warps hide them (clamped, 4,500 rows of [2 x 4,096, 1,024]: 84 us with 8 warps, 64 with 16).
+    static constexpr int OUT_WARPS = EPI == GT_CLAMP || EPI == GT_GELU || EPI == GT_XIELU ? 16 : 8, THREADS = 64 + 32 * OUT_WARPS;
+    static constexpr int BM = 128 * CG;
+    static constexpr int A_BYTES = 128 * 128, B_BYTES = BN / CG * 128, HALF = A_BYTES + B_BYTES, STAGE = 2 * HALF;   // a half: 64 columns of k
+    static constexpr int SLAB = 2048, SLABS = OUT_WARPS * SLAB;
+    static constexpr int STAGES = (221 * 1024 - SLABS) / STAGE < 8 ? (221 * 1024 - SLABS) / STAGE : 8;
+    static constexpr int TMEM = 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
+    static constexpr int SMEM = 1024 + STAGES * STAGE + SLABS + (2 * STAGES + 4) * 8 + 16;
+};
+
+__device__ __forceinline__ uint32_t gt_in_block(const void* p, uint32_t rank) {   // the address of p's place in a block of the cluster
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+template <int CG> __device__ __forceinline__ void gt_load(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    if (CG == 2)
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                     ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                     ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+template <int CG> __device__ __forceinline__ void gt_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    if (CG == 2)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+    else tc_mma(d, a, b, idesc, acc);
+}
+template <int CG> __device__ __forceinline__ void gt_commit(uint64_t* bar) {   // arrives at the barrier of this place in every block of the pair
+    if (CG == 2)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+    else tc_commit(bar);
+}
+
+// Where a tile lies: its first row, the row behind its last, its first output column, the expert.
+struct GtTile {
+    int row, row_end, col, expert;
+};
+
+template <int CG, int BN, int EPI, bool GROUPED>
+__device__ __forceinline__ GtTile gt_tile(const GtArgs& a, const int* starts, int t) {
+    constexpr int BM = GtShape<CG, BN>::BM, OUT = gt_gated(EPI) ? BN / 2 : BN;
+    if (GROUPED) {
+        int lo = 0, hi = a.n_experts;   // the last expert whose first tile is at or before t
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) / 2;
+            if (starts[mid] * a.n_tiles <= t) lo = mid;
+            else hi = mid;
+        }
+        const int mt = starts[lo + 1] - starts[lo], r = t - starts[lo] * a.n_tiles;
+        const int first = lo ? a.ends[lo - 1] : 0;
+        return {first + r % mt * BM, a.ends[lo], r / mt * OUT, lo};
+    }
+    const int per = GT_GROUP * a.n_tiles, g = t / per, r = t - g * per;
+    const int rows = min(GT_GROUP, a.m_tiles - g * GT_GROUP);
+    return {(g * GT_GROUP + r % rows) * BM, a.M, r / rows * OUT, 0};
+}
+
+// The activation of two neighbours, from the values that the product would leave in memory (one instruction rounds both).
+template <int EPI> __device__ __forceinline__ float2 gt_act(float2 g, float2 u, float alpha, float limit) {
+    g = __bfloat1622float2(__floats2bfloat162_rn(g.x, g.y));
+    if (EPI == GT_RELU2) {
+        g.x = fmaxf(g.x, 0.f), g.y = fmaxf(g.y, 0.f);
+        return make_float2(g.x * g.x, g.y * g.y);
+    }
+    if (EPI == GT_XIELU) return make_float2(xielu_value(g.x, alpha, limit), xielu_value(g.y, alpha, limit));
+    u = __bfloat1622float2(__floats2bfloat162_rn(u.x, u.y));
+    if (EPI == GT_SWIGLU) {   // by the fast units, as swiglu_vec_kernel: their error is far below the rounding that follows
+        g = __bfloat1622float2(__floats2bfloat162_rn(__fdividef(g.x, 1.0f + __expf(-g.x)), __fdividef(g.y, 1.0f + __expf(-g.y))));
+        return make_float2(__fmul_rn(g.x, u.x), __fmul_rn(g.y, u.y));
+    }
+    if (EPI == GT_CLAMP) {
+        g.x = fminf(g.x, limit), g.y = fminf(g.y, limit);
+        u.x = fminf(fmaxf(u.x, -limit), limit), u.y = fminf(fmaxf(u.y, -limit), limit);
+        return make_float2(g.x / (1.0f + expf(-alpha * g.x)) * (u.x + 1.0f), g.y / (1.0f + expf(-alpha * g.y)) * (u.y + 1.0f));
+    }
+    return make_float2(gelu_tanh_value(g.x) * u.x, gelu_tanh_value(g.y) * u.y);
+}
+
+template <int CG, int BN, int EPI, bool GROUPED>
+__global__ void __launch_bounds__(GtShape<CG, BN, EPI>::THREADS, 1)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GtArgs args) {
+    typedef GtShape<CG, BN, EPI> S;
+    constexpr bool GATED = gt_gated(EPI);
+    constexpr int OUT = GATED ? BN / 2 : BN;
+    extern __shared__ unsigned char gt_raw[];
+    __shared__ int starts[GROUPED ? GT_MAX_EXPERTS + 1 : 1];
+    __shared__ uint32_t tmem_s;
+    __shared__ int abort_s;
+    unsigned char* sm = gt_raw + ((1024 - (smem_u32(gt_raw) & 1023)) & 1023);
+    unsigned char* slabs = sm + S::STAGES * S::STAGE;
+    uint64_t* full = reinterpret_cast<uint64_t*>(slabs + S::SLABS);
+    uint64_t* empty = full + S::STAGES;
+    uint64_t* sum_full = empty + S::STAGES;   // [2]: a tile's sums are complete
+    uint64_t* sum_empty = sum_full + 2;       // [2]: they have been read
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = CG == 2 ? blockIdx.x & 1 : 0, unit = blockIdx.x / CG, units = gridDim.x / CG;
+    volatile int* abort_flag = &abort_s;
+
+    if (tid == 0) {
+        abort_s = 0;
+        for (int s = 0; s < S::STAGES; ++s) mbar_init(full + s, 1), mbar_init(empty + s, 1);
+        for (int b = 0; b < 2; ++b) mbar_init(sum_full + b, 1), mbar_init(sum_empty + b, S::OUT_WARPS * CG);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+    }
+    if (warp == 1) {
+        if (CG == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "r"((uint32_t)S::TMEM) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            tmem_alloc(&tmem_s, S::TMEM);
+        }
+    }
+    pdl_wait();
+    if (GROUPED && warp == 0) {   // the experts' first tiles
+        int before = 0;
+        for (int e0 = 0; e0 < args.n_experts; e0 += 32) {
+            const int e = e0 + lane;
+            int n = 0;
+            if (e < args.n_experts) n = (args.ends[e] - (e ? args.ends[e - 1] : 0) + S::BM - 1) / S::BM;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, n, o);
+                if (lane >= o) n += v;
+            }
+            if (e < args.n_experts) starts[e + 1] = before + n;
+            before += __shfl_sync(0xffffffffu, n, 31);
+        }
+        if (lane == 0) starts[0] = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (CG == 2) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    tc_fence_after();
+    const uint32_t tmem = tmem_s;
+    const int tiles = GROUPED ? starts[args.n_experts] * args.n_tiles : args.m_tiles * args.n_tiles;
+    const int turns = (args.K + 63) / 64;
+
+    if (warp == 0) {
+        if (lane == 0) {   // ---- copies
+            int stage = 0, phase = 0;
+            bool ok = true;
+            for (int t = unit; t < tiles && ok; t += units) {
+                const GtTile tile = gt_tile<CG, BN, EPI, GROUPED>(args, starts, t);
+                const int ya = tile.row + rank * 128;
+                const int w_rows = GATED ? 2 * args.N : args.N;
+                const int yw = tile.expert * w_rows + tile.col + (GATED ? rank * args.N : rank * (BN / CG));
+                for (int k = 0; k < turns; k += 2) {
+                    ok = mbar_wait(empty + stage, phase ^ 1, abort_flag, args.status);
+                    if (!ok) break;
+                    const int halves = min(2, turns - k);
+                    if (rank == 0) mbar_expect_tx(full + stage, CG * halves * S::HALF);
+                    const uint32_t bar = CG == 2 ? gt_in_block(full + stage, 0) : smem_u32(full + stage);
+                    for (int h = 0; h < halves; ++h) {
+                        unsigned char* a_s = sm + stage * S::STAGE + h * S::HALF;
+                        unsigned char* b_s = a_s + S::A_BYTES;
+                        gt_load<CG>(a_s, &map_a, (k + h) * 64, ya, bar);
+                        gt_load<CG>(b_s, &map_w, (k + h) * 64, yw, bar);
+                        if (GATED && CG == 1) gt_load<CG>(b_s + BN / 2 * 128, &map_w, (k + h) * 64, yw + args.N, bar);
+                    }
+                    if (++stage == S::STAGES) stage = 0, phase ^= 1;
+                }
+            }
+            pdl_launch_dependents();
+            if (*abort_flag) {   // copies may still be under way: they end long before this does
+                const long long t0 = clock64();
+                while (clock64() - t0 < (1ll << 22)) {}
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {   // ---- products
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(S::BM >> 4) << 24);
+            const uint64_t desc0 = desc_k_major(sm);   // the address fields of all stages lie below their 14 bits: no carry
+            int stage = 0, phase = 0, n = 0;
+            bool ok = true;
+            for (int t = unit; t < tiles && ok; t += units, ++n) {
+                const int buf = n & 1;
+                ok = mbar_wait(sum_empty + buf, ((n >> 1) & 1) ^ 1, abort_flag, args.status);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d = tmem + buf * BN;
+                for (int k = 0; k < turns; k += 2) {
+                    ok = mbar_wait(full + stage, phase, abort_flag, args.status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t da = desc0 + stage * (S::STAGE >> 4), db = da + (S::A_BYTES >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk) gt_mma<CG>(d, da + 2 * kk, db + 2 * kk, idesc, k > 0 || kk > 0);
+                    if (k + 1 < turns) {
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) gt_mma<CG>(d, da + (S::HALF >> 4) + 2 * kk, db + (S::HALF >> 4) + 2 * kk, idesc, 1);
+                    }
+                    gt_commit<CG>(empty + stage);
+                    if (++stage == S::STAGES) stage = 0, phase ^= 1;
+                }
+                if (ok) gt_commit<CG>(sum_full + buf);
+            }
+        }
+        __syncwarp();
+    } else {   // ---- the tiles' way out: a warp takes its share of the runs of 32 columns of the 32 rows whose lanes it may read
+        const int quarter = warp & 3, part = (warp - 2) >> 2;
+        constexpr int STEP = S::OUT_WARPS * 8;
+        unsigned char* slab = slabs + (warp - 2) * S::SLAB;
+        int n = 0;
+        for (int t = unit; t < tiles; t += units, ++n) {
+            const GtTile tile = gt_tile<CG, BN, EPI, GROUPED>(args, starts, t);
+            const int buf = n & 1;
+            if (!mbar_wait<true>(sum_full + buf, (n >> 1) & 1, abort_flag, args.status)) break;
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t src = tmem + buf * BN + ((uint32_t)(quarter * 32) << 16);
+            const int row0 = tile.row + rank * 128 + quarter * 32;
+            auto release = [&]() {   // this warp is done with the tile's sums
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (CG == 2) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(gt_in_block(sum_empty + buf, 0)) : "memory");
+                    else mbar_arrive(sum_empty + buf);
+                }
+            };
+            if (part * 32 >= OUT) release();
+#pragma unroll 1
+            for (int c = part * 32; c < OUT; c += STEP) {
+                // Rows meet the slab 16 bytes at a time at places that keep eight lanes on different banks, and leave it in whole runs.
+                const int at = lane * 64, turn = (lane >> 1) & 3;
+                if constexpr (EPI != GT_PLAIN) {
+                    // Eight columns at a time: straight-line code for all 32 is fetched as slowly as it runs once a tile.
+#pragma unroll 1
+                    for (int i = 0; i < 4; ++i) {
+                        float g[8], u[8];
+                        tc_ld8_async(src + c + 8 * i, reinterpret_cast<uint32_t*>(g));
+                        if (GATED) tc_ld8_async(src + BN / 2 + c + 8 * i, reinterpret_cast<uint32_t*>(u));
+                        tc_wait_ld();
+                        if (i == 3 && c + STEP >= OUT) release();
+#pragma unroll
+                        for (int e = 0; e < 8; e += 2) {
+                            const float2 y = gt_act<EPI>(make_float2(g[e], g[e + 1]), GATED ? make_float2(u[e], u[e + 1]) : make_float2(0.f, 0.f),
+                                                         args.alpha, args.limit);
+                            g[e] = y.x, g[e + 1] = y.y;
+                        }
+                        store_bf16<8>(reinterpret_cast<__nv_bfloat16*>(slab + at + ((i ^ turn) << 4)), g);
+                    }
+                } else {
+                    float v[32];
+                    tc_ld32(src + c, v);
+                    if (c + STEP >= OUT) release();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        float f[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) f[e] = v[8 * i + e];
+                        store_bf16<8>(reinterpret_cast<__nv_bfloat16*>(slab + at + ((i ^ turn) << 4)), f);
+                    }
+                }
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int r = j * 8 + (lane >> 2), i = lane & 3, col = tile.col + c + i * 8;
+                    const uint4 x = *reinterpret_cast<const uint4*>(slab + r * 64 + ((i ^ ((r >> 1) & 3)) << 4));
+                    if (row0 + r < tile.row_end && col < args.N)
+                        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(args.out) + (long long)(row0 + r) * args.N + col) = x;
+                }
+                __syncwarp();
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (CG == 2) {   // neither block leaves while the other may still reach its shared memory
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    if (warp == 1) {
+        if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)S::TMEM) : "memory");
+        else tmem_dealloc(tmem, S::TMEM);
+    }
+}
+
+// ---- host side ----------------------------------------------------------------------------------
+
+template <int CG, int BN, int EPI, bool GROUPED>
+static int gt_launch(const CUtensorMap& ma, const CUtensorMap& mw, const GtArgs& args, int blocks, cudaStream_t stream) {
+    typedef GtShape<CG, BN, EPI> S;
+    static const cudaError_t configured =
+        cudaFuncSetAttribute(gemm_rows_kernel<CG, BN, EPI, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+    if (configured != cudaSuccess) return (int)configured;
+    sb_launch_cluster(gemm_rows_kernel<CG, BN, EPI, GROUPED>, dim3(blocks), dim3(S::THREADS), dim3(CG), S::SMEM, stream, ma, mw, args);
+    return (int)cudaGetLastError();
+}
+
+template <int CG, int BN>
+static int gt_experts(int epi, const CUtensorMap& ma, const CUtensorMap& mw, const GtArgs& args, int blocks, cudaStream_t stream) {
+    if (epi == GT_PLAIN) return gt_launch<CG, BN, GT_PLAIN, true>(ma, mw, args, blocks, stream);
+    if (epi == GT_SWIGLU) return gt_launch<CG, BN, GT_SWIGLU, true>(ma, mw, args, blocks, stream);
+    return gt_launch<CG, BN, GT_CLAMP, true>(ma, mw, args, blocks, stream);
+}
+
+// out [M, N] = epilogue(a w^T).  a: M rows of K bfloat16 numbers, lda apart; w: N rows (2 N for a gated epilogue, gate over up) of K,
+// contiguous; grouped (ends != nullptr; no epilogue or the two gated ones that experts have): w holds n_experts such matrices, and rows
+// ends[e - 1] to ends[e] - 1 of a meet the e-th (rows behind the last expert's stay unwritten).  K and N are multiples of 8, the addresses
+// of 16 bytes.  wide: pairs of blocks with tiles of 256 x 256; otherwise (grouped only) single blocks with 128 x 128.
+extern "C" int sb_gemm_rows(const void* a, long long lda, const void* w, void* out, int M, int N, int K, int epi, const int* ends, int n_experts,
+                            float alpha, float limit, int wide, int sms, int* status, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    const bool grouped = ends != nullptr, gated = gt_gated(epi);
+    if (K <= 0 || K % 8 || N % 8 || lda < K || lda % 8 || !sb_aligned(16, (const char*)a, (const char*)w, (const char*)out) || sms < 2 ||
+        (grouped ? n_experts < 1 || n_experts > GT_MAX_EXPERTS || epi < GT_PLAIN || epi > GT_CLAMP : !wide || epi < GT_SWIGLU || epi > GT_XIELU))
+        return (int)cudaErrorInvalidValue;
+    const int cg = wide ? 2 : 1, bn = wide ? 256 : 128, bm = 128 * cg, n_out = gated ? bn / 2 : bn;
+    const long long w_rows = (long long)N * (gated ? 2 : 1) * (grouped ? n_experts : 1);
+    GtArgs args = {out, ends, status, M, N, K, n_experts, (M + bm - 1) / bm, (N + n_out - 1) / n_out, alpha, limit};
+    long long tiles = (long long)args.m_tiles * args.n_tiles;
+    if (grouped) tiles += (long long)n_experts * args.n_tiles;   // at most a ragged tile an expert
+    if (w_rows > 0x7fffffff || tiles > 0x3fffffff) return (int)cudaErrorInvalidValue;
+    CUtensorMap ma, mw;
+    int e = make_rows_map(&ma, a, M, K, lda, 128);
+    if (e) return e;
+    e = make_rows_map(&mw, w, w_rows, K, K, gated && cg == 1 ? bn / 2 : bn / cg);
+    if (e) return e;
+    const int units = sms / cg, blocks = cg * (int)(tiles < units ? tiles : units);
+    if (grouped) return wide ? gt_experts<2, 256>(epi, ma, mw, args, blocks, stream) : gt_experts<1, 128>(epi, ma, mw, args, blocks, stream);
+    switch (epi) {
+        case GT_SWIGLU: return gt_launch<2, 256, GT_SWIGLU, false>(ma, mw, args, blocks, stream);
+        case GT_CLAMP: return gt_launch<2, 256, GT_CLAMP, false>(ma, mw, args, blocks, stream);
+        case GT_GELU: return gt_launch<2, 256, GT_GELU, false>(ma, mw, args, blocks, stream);
+        case GT_RELU2: return gt_launch<2, 256, GT_RELU2, false>(ma, mw, args, blocks, stream);
+        default: return gt_launch<2, 256, GT_XIELU, false>(ma, mw, args, blocks, stream);
+    }
+}

@@ -121,6 +121,8 @@ class Ops:
             "sb_tile_matrix": [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
             "sb_gemm_stream": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                c_void_p, c_void_p],
+            "sb_gemm_rows": [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float, c_float, c_int,
+                             c_int, c_void_p, c_void_p],
             "sb_gemm_stream_plan": [c_int, c_int, c_int, POINTER(c_int), POINTER(c_int), POINTER(c_int)],
             "sb_attn_prefill_tc": [c_void_p, c_void_p, SbBatch, SbKV, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p],
             "sb_attn_prefill": [c_void_p, c_void_p, SbBatch, SbKV, c_int, c_float, c_int, c_int, c_void_p],
@@ -241,6 +243,7 @@ class Ops:
         self.force_skinny = None  # (K slices, tiled, warps) for tests and tuning runs; None = the rules below
         self._tiled_bytes = 0     # bytes of tile-major copies alive (a copy hangs on its matrix as ._sb_tiled = (copy, halves))
         self.decode_copy = os.environ.get("STARTER_B200_DECODE_COPY", "auto")   # "1", "0" or "auto"
+        self.use_rows = os.environ.get("STARTER_B200_ROWS", "1") != "0"      # products of many rows with their activation in one kernel
         self.use_stream = os.environ.get("STARTER_B200_STREAM", "1") != "0"  # the TMA + tcgen05 product for decode
         self._kernel_status = None
         self._status_override = None
@@ -628,6 +631,42 @@ class Ops:
             self.launches += 1   # the chunks' sums are added up
         return out
 
+    # What follows a product of many rows in its epilogue (gemm_rows.cu)
+    ROWS_PLAIN, ROWS_SWIGLU, ROWS_CLAMP, ROWS_GELU, ROWS_RELU2, ROWS_XIELU = range(6)
+    ROWS_EXPERTS_MAX = 1024
+    # Pairs an expert beyond which the grouped product takes pairs of SMs with 256 x 256 tiles (below, single ones with 128 x 128): 16 experts of
+    # 3 x 1,024 x 512, both products, us by pairs an expert, wide / narrow: 100: 23.8 / 18.6, 200: 24.6 / 26.9, 900: 52 / 66; 32 of 3 x 2,048 x
+    # 1,024: 100: 98 / 85, 200: 103 / 124
+    ROWS_WIDE_PAIRS = 128
+    ROWS_MIN = 700
+    ROWS_FILL = 0.8
+
+    def _takes_rows(self, h, w, n_out, gated) -> bool:
+        """Whether a product of many rows and the activation behind it run as one kernel (gemm_rows.cu: pairs of SMs with tiles of
+        256 rows by 256 columns of sums).  Its product alone is at best level with the library's, which has tiles for every size; what it
+        saves is the activation's launch and its trip through memory.  So: where ragged edges and the last round of tiles leave
+        less than a fifth of the pairs' time empty.  Library and activation kernel / this (us, graph replay): [2 x 9,728, 2,560] silu, 700 rows 63.9
+        / 62.7, 1,024 81.8 / 79.2, 2,048 167 / 144, 4,500 410 / 312; [2 x 6,144, 2,048] silu, 500 rows 25.0 / 28.9, 1,024 44.0 / 41.2, 4,500 178 /
+        152; [2 x 8,192, 2,048] clamped, 700 rows 43.9 / 46.1, 1,024 59.9 / 56.9, 2,048 125 / 98; [2 x 2,048, 1,024] clamped, 1,500 rows (a round
+        and a third of tiles) 17.8 / 24.1, 2,048 22.6 / 21.1, 4,500 40.9 / 36.7."""
+        M, K = h.shape
+        if (M < self.ROWS_MIN or K % 8 or n_out % 8 or h.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or w.shape[1] != K
+                or not self.use_rows or h.stride(1) != 1 or h.stride(0) % 8 or h.data_ptr() % 16 or not w.is_contiguous() or w.data_ptr() % 16):
+            return False
+        pairs = self.sm_count() // 2
+        tiles = -(-M // 256) * -(-n_out // (128 if gated else 256))
+        columns = n_out * (2 if gated else 1)
+        return M * columns >= self.ROWS_FILL * (-(-tiles // pairs) * pairs * 65536)
+
+    def _rows_product(self, h, w, n_out, epilogue, alpha=0.0, limit=0.0, ends=None, n_experts=0, wide=True):
+        """epilogue(h w^T) by gemm_rows.cu; with ``ends``, rows sorted by expert against the expert's own matrix."""
+        M, K = h.shape
+        out = torch.empty((M, n_out), dtype=torch.bfloat16, device=h.device)
+        self._check(self.lib.sb_gemm_rows(_ptr(h), h.stride(0), _ptr(w), _ptr(out), M, n_out, K, epilogue, _ptr(ends), n_experts, float(alpha),
+                                          float(limit), int(wide), self.sm_count(), _ptr(self.kernel_status(h.device)), self._stream()),
+                    "gemm_rows")
+        return out
+
     def linear_swiglu(self, h, w_gate_up, norm=None):
         """swiglu(h @ w_gate_up^T) for a fused [gate; up] matrix: [M, K] -> [M, rows / 2].  norm: as in ``linear``."""
         M, K = h.shape
@@ -640,6 +679,8 @@ class Ops:
                 return self._stream_product(h, w_gate_up, w_gate_up.shape[0] // 2, True, False)
             if M <= self.SKINNY_MAX_ROWS:
                 return self._skinny(h, w_gate_up, w_gate_up.shape[0] // 2, True, False)
+        if self._takes_rows(h, w_gate_up, w_gate_up.shape[0] // 2, True):
+            return self._rows_product(h, w_gate_up, w_gate_up.shape[0] // 2, self.ROWS_SWIGLU)
         return self.swiglu(self.linear(h, w_gate_up))
 
     def linear_gated_clamp(self, h, w_gate_up, alpha, limit):
@@ -648,6 +689,8 @@ class Ops:
         M, K = h.shape
         if h.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 and K % 8 == 0 and M <= self.SKINNY_MAX_ROWS:
             return self._skinny(h, w_gate_up, w_gate_up.shape[0] // 2, True, False, act=(alpha, limit))
+        if self._takes_rows(h, w_gate_up, w_gate_up.shape[0] // 2, True):
+            return self._rows_product(h, w_gate_up, w_gate_up.shape[0] // 2, self.ROWS_CLAMP, alpha, limit)
         return self.gated_clamp(self.linear(h, w_gate_up), alpha, limit)
 
     def gated_gelu(self, gu):
@@ -665,6 +708,8 @@ class Ops:
         M, K = h.shape
         if h.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 and K % 8 == 0 and M <= self.SKINNY_MAX_ROWS:
             return self._skinny(h, w_gate_up, w_gate_up.shape[0] // 2, True, False, act="gelu")
+        if self._takes_rows(h, w_gate_up, w_gate_up.shape[0] // 2, True):
+            return self._rows_product(h, w_gate_up, w_gate_up.shape[0] // 2, self.ROWS_GELU)
         return self.gated_gelu(self.linear(h, w_gate_up))
 
     # ---- layer norms, the capped head ----------------------------------------------------
@@ -1344,6 +1389,8 @@ class Ops:
         M, K = h.shape
         if h.dtype == torch.bfloat16 and w_up.dtype == torch.bfloat16 and K % 8 == 0 and M <= self.SKINNY_MAX_ROWS:
             return self._skinny(h, w_up, w_up.shape[0], False, False, unary="relu2")
+        if self._takes_rows(h, w_up, w_up.shape[0], False):
+            return self._rows_product(h, w_up, w_up.shape[0], self.ROWS_RELU2)
         return self.relu2(self.linear(h, w_up))
 
     def conv_qk_store(self, ctx, q, k, layer_cache, state, n_heads, q_bias, k_bias, q_conv, k_conv, q_norm, k_norm, eps,
@@ -1691,8 +1738,8 @@ class Ops:
         its sigmoid factor ``alpha`` and ``limit``, or silu(gate) * up when ``alpha`` is None) with stacked
         matrices w_gate_up [experts, 2 ff, width] (gate over up) and w_down [experts, width, ff]; a choice >= n_experts
         is an identity output and adds weight * h.  A few pairs: each pair streams its expert's matrices; some hundreds: every
-        expert's matrices are read once for its pairs (this library's kernels).  Many pairs in bfloat16: the pairs are put in the order of their experts on the device and each matrix
-        takes one grouped product of the vendor's library, as the plain products of a prompt do."""
+        expert's matrices are read once for its pairs.  Many pairs in bfloat16: the pairs are put in the order of their experts on the
+        device and each matrix takes one grouped product, the first with the activation in its epilogue (gemm_rows.cu)."""
         rows, width = h.shape
         top = chosen.shape[1]
         pairs = rows * top
@@ -1712,7 +1759,7 @@ class Ops:
                                                 self._stream()), "moe_few")
                 self.launches += 1
             elif (h.dtype == torch.bfloat16 and pairs > self.MOE_PAIRS_MAX and width % 8 == 0 and ff % 8 == 0
-                    and hasattr(torch, "_grouped_mm")):
+                    and n_experts <= self.ROWS_EXPERTS_MAX and w_gate_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0):
                 ends = torch.empty(n_experts, dtype=torch.int32, device=h.device)
                 slot_of_pair = torch.empty(pairs, dtype=torch.int32, device=h.device)
                 pair_of_slot = torch.empty(pairs, dtype=torch.int32, device=h.device)
@@ -1721,9 +1768,10 @@ class Ops:
                 xs = torch.empty((pairs, width), dtype=h.dtype, device=h.device)
                 self._check(self.lib.sb_moe_gather(dt, _ptr(h), _ptr(pair_of_slot), _ptr(ends), n_experts, pairs, top, width,
                                                    _ptr(xs), self._stream()), "moe_gather")
-                gu = torch._grouped_mm(xs, w_gate_up.transpose(1, 2), offs=ends)
-                act = self.swiglu(gu) if alpha is None else self.gated_clamp(gu, alpha, limit)
-                down = torch._grouped_mm(act, w_down.transpose(1, 2), offs=ends)
+                wide = pairs > self.ROWS_WIDE_PAIRS * n_experts
+                act = self._rows_product(xs, w_gate_up, ff, self.ROWS_SWIGLU if alpha is None else self.ROWS_CLAMP, alpha or 0.0, limit or 0.0, ends,
+                                         n_experts, wide)
+                down = self._rows_product(act, w_down, width, self.ROWS_PLAIN, 0.0, 0.0, ends, n_experts, wide)
             else:
                 act = torch.empty((pairs, ff), dtype=h.dtype, device=h.device)
                 down = torch.empty((pairs, width), dtype=h.dtype, device=h.device)
@@ -1830,6 +1878,8 @@ class Ops:
         M, K = h.shape
         if h.dtype == torch.bfloat16 and w_up.dtype == torch.bfloat16 and K % 8 == 0 and M <= self.SKINNY_MAX_ROWS:
             return self._skinny(h, w_up, w_up.shape[0], False, False, unary=(a_pos, a_neg))
+        if self._takes_rows(h, w_up, w_up.shape[0], False):
+            return self._rows_product(h, w_up, w_up.shape[0], self.ROWS_XIELU, a_pos, a_neg)
         return self.xielu(self.linear(h, w_up), a_pos, a_neg)
 
     def qk_norm_store(self, ctx, qkv, layer_cache, n_heads, q_norm, k_norm, eps):

@@ -1,0 +1,82 @@
+"""Products of many rows with the activation in their epilogue, dense and per expert: at the borders of tiles, stages and pairs of blocks,
+against 64 bits with the roundings of the product and the activation kernel."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from starter_b200.csrc.ops import get_ops
+    return get_ops(verbose=False)
+
+
+def rand(shape, seed, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * scale).bfloat16()
+
+
+def activated(ops, z, epilogue):
+    if epilogue == ops.ROWS_PLAIN:
+        return z
+    z = z.bfloat16().double()     # the product as it would lie in memory
+    if epilogue == ops.ROWS_RELU2:
+        return torch.relu(z) ** 2
+    if epilogue == ops.ROWS_XIELU:
+        return torch.where(z > 0, 0.7 * z * z + 0.5 * z, 0.9 * (torch.expm1(torch.clamp(z, max=0.0)) - z) + 0.5 * z)
+    g, u = z.chunk(2, 1)
+    if epilogue == ops.ROWS_SWIGLU:
+        return (g * torch.sigmoid(g)).bfloat16().double() * u
+    if epilogue == ops.ROWS_CLAMP:
+        g, u = g.clamp(max=0.9), u.clamp(-0.9, 0.9)
+        return g * torch.sigmoid(0.7 * g) * (u + 1.0)
+    return torch.nn.functional.gelu(g, approximate="tanh") * u
+
+
+def close(got, want):
+    # bfloat16 results (2^-9 a value) of sums that may have been rounded to the neighbour before the activation (2^-8 of a factor)
+    assert float((got.double() - want).norm() / want.norm()) < 4e-3
+    assert float(((got.double() - want).abs() / (want.abs() + want.square().mean().sqrt())).max()) < 2.5e-2
+
+
+# tiles of 256 rows by 256 sums (128 gated columns), 128 columns of k a stage, three stages, 74 pairs; one tile, many rounds, ragged edges
+@pytest.mark.parametrize("M, N, K", [(1, 8, 8), (256, 256, 128), (257, 264, 136), (700, 1000, 520), (3000, 2056, 64), (129, 5128, 1032)])
+@pytest.mark.parametrize("name", ["SWIGLU", "CLAMP", "GELU", "RELU2", "XIELU"])
+def test_dense(ops, M, N, K, name):
+    epilogue = getattr(ops, "ROWS_" + name)
+    h = rand((M, K + 16), 1)[:, 8:K + 8]      # rows inside wider ones
+    w = rand((N * (2 if name in ("SWIGLU", "CLAMP", "GELU") else 1), K), 2, K ** -0.5)
+    got = ops._rows_product(h, w, N, epilogue, 0.7, 0.9)
+    close(got, activated(ops, h.double() @ w.double().T, epilogue))
+    assert ops.read_kernel_status() == 0
+
+
+@pytest.mark.parametrize("counts", [[0, 5, 300, 0, 257, 1, 128], [1], [0, 0, 0], [600, 0, 1, 2000], [3] * 40, [7] * 1024])
+@pytest.mark.parametrize("name", ["PLAIN", "SWIGLU", "CLAMP"])
+@pytest.mark.parametrize("wide", [False, True])
+def test_per_expert(ops, counts, name, wide):
+    epilogue, (K, N) = getattr(ops, "ROWS_" + name), (72, 136)
+    E, P = len(counts), sum(counts) + 37       # rows behind the last expert's stay out of it
+    h, ends = rand((P, K), 3), torch.tensor(counts, device="cuda").cumsum(0).int()
+    w = rand((E, N * (1 if name == "PLAIN" else 2), K), 4, K ** -0.5)
+    got = ops._rows_product(h, w, N, epilogue, 0.7, 0.9, ends, E, wide)
+    at = 0
+    wants = []
+    for e, n in enumerate(counts):
+        wants.append(activated(ops, h[at:at + n].double() @ w[e].double().T, epilogue))
+        at += n
+    if at:
+        close(got[:at], torch.cat(wants))
+    assert ops.read_kernel_status() == 0
+
+
+def test_which_steps(ops):
+    h, w = rand((2048, 512), 5), rand((2 * 4096, 512), 6)
+    assert ops._takes_rows(h, w, 4096, True) and not ops._takes_rows(h[:600], w, 4096, True)
+    assert not ops._takes_rows(h.float(), w, 4096, True) and not ops._takes_rows(h, w[:8184], 4092, True)
+    assert not ops._takes_rows(h[:, 1:505], w[:, :504], 4096, True)
+    before = ops.launches
+    fused = ops.linear_swiglu(h, w)
+    assert ops.launches == before + 1
+    close(fused, ops.swiglu(torch.mm(h, w.t())).double())
