@@ -4,7 +4,7 @@
 // kernel of its own (engine/kernels/swiglu.py:13-25).
 //
 // A pair of blocks (a cluster of two SMs) owns tiles of 256 rows x BN columns of sums: each loads its 128 rows of A and half of the
-// tile's rows of W by TMA, 128 columns of k at a time through a ring of stages, one thread of the first block issues the products of both
+// tile's rows of W by TMA, 64 or 128 columns of k at a time through a ring of stages, one thread of the first block issues the products of both
 // (cta_group::2, so that each SM reads half of W from its neighbour's shared memory), each holds its rows' sums in tensor memory,
 // twice, so that the warps behind take a tile out while the next is summed.  Pairs walk the tiles from their own number on, a group of
 // row tiles side by side, so that what runs at one time shares its rows of A and W in L2.
@@ -33,8 +33,11 @@ template <int CG, int BN, int EPI = GT_PLAIN> struct GtShape {
     // their own: only more warps hide them (clamped, 4,500 rows of [2 x 4,096, 1,024]: 84 us with 8 warps, 64 with 16).
     static constexpr int OUT_WARPS = EPI == GT_CLAMP || EPI == GT_GELU || EPI == GT_XIELU ? 16 : 8, THREADS = 64 + 32 * OUT_WARPS;
     static constexpr int BM = 128 * CG;
-    static constexpr int A_BYTES = 128 * 128, B_BYTES = BN / CG * 128, HALF = A_BYTES + B_BYTES, STAGE = 2 * HALF;   // a half: 64 columns of k
+    static constexpr int A_BYTES = 128 * 128, B_BYTES = BN / CG * 128, HALF = A_BYTES + B_BYTES;   // a half: 64 columns of k
     static constexpr int SLAB = 2048, SLABS = OUT_WARPS * SLAB;
+    // Two halves a stage (16 prompts of the 1.7B sizes: 54.2 ms, with one 56.2), except beside the slabs of 16 warps, where only two such stages
+    // fit (2,048 rows of [2 x 8,192, 2,048] clamped: 118 us, with five stages of one half 101).
+    static constexpr int HALVES = OUT_WARPS > 8 ? 1 : 2, STAGE = HALVES * HALF;
     static constexpr int STAGES = (221 * 1024 - SLABS) / STAGE < 8 ? (221 * 1024 - SLABS) / STAGE : 8;
     static constexpr int TMEM = 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
     static constexpr int SMEM = 1024 + STAGES * STAGE + SLABS + (2 * STAGES + 4) * 8 + 16;
@@ -184,10 +187,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 const int ya = tile.row + rank * 128;
                 const int w_rows = GATED ? 2 * args.N : args.N;
                 const int yw = tile.expert * w_rows + tile.col + (GATED ? rank * args.N : rank * (BN / CG));
-                for (int k = 0; k < turns; k += 2) {
+                for (int k = 0; k < turns; k += S::HALVES) {
                     ok = mbar_wait(empty + stage, phase ^ 1, abort_flag, args.status);
                     if (!ok) break;
-                    const int halves = min(2, turns - k);
+                    const int halves = min(S::HALVES, turns - k);
                     if (rank == 0) mbar_expect_tx(full + stage, CG * halves * S::HALF);
                     const uint32_t bar = CG == 2 ? gt_in_block(full + stage, 0) : smem_u32(full + stage);
                     for (int h = 0; h < halves; ++h) {
@@ -219,14 +222,14 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d = tmem + buf * BN;
-                for (int k = 0; k < turns; k += 2) {
+                for (int k = 0; k < turns; k += S::HALVES) {
                     ok = mbar_wait(full + stage, phase, abort_flag, args.status);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t da = desc0 + stage * (S::STAGE >> 4), db = da + (S::A_BYTES >> 4);
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) gt_mma<CG>(d, da + 2 * kk, db + 2 * kk, idesc, k > 0 || kk > 0);
-                    if (k + 1 < turns) {
+                    if (S::HALVES == 2 && k + 1 < turns) {
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) gt_mma<CG>(d, da + (S::HALF >> 4) + 2 * kk, db + (S::HALF >> 4) + 2 * kk, idesc, 1);
                     }

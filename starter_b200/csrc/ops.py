@@ -639,16 +639,17 @@ class Ops:
     # 1,024: 100: 98 / 85, 200: 103 / 124
     ROWS_WIDE_PAIRS = 128
     ROWS_MIN = 700
-    ROWS_FILL = 0.8
+    ROWS_FILL = 0.82
 
     def _takes_rows(self, h, w, n_out, gated) -> bool:
         """Whether a product of many rows and the activation behind it run as one kernel (gemm_rows.cu: pairs of SMs with tiles of
         256 rows by 256 columns of sums).  Its product alone is at best level with the library's, which has tiles for every size; what it
         saves is the activation's launch and its trip through memory.  So: where ragged edges and the last round of tiles leave
-        less than a fifth of the pairs' time empty.  Library and activation kernel / this (us, graph replay): [2 x 9,728, 2,560] silu, 700 rows 63.9
-        / 62.7, 1,024 81.8 / 79.2, 2,048 167 / 144, 4,500 410 / 312; [2 x 6,144, 2,048] silu, 500 rows 25.0 / 28.9, 1,024 44.0 / 41.2, 4,500 178 /
-        152; [2 x 8,192, 2,048] clamped, 700 rows 43.9 / 46.1, 1,024 59.9 / 56.9, 2,048 125 / 98; [2 x 2,048, 1,024] clamped, 1,500 rows (a round
-        and a third of tiles) 17.8 / 24.1, 2,048 22.6 / 21.1, 4,500 40.9 / 36.7."""
+        less than 18% of the pairs' time empty.  Library and activation kernel / this (us, graph replay): [2 x 9,728, 2,560] silu, 700 rows
+        63.3 / 62.5, 1,024 81.3 / 79.8, 2,048 157 / 144, 4,500 335 / 303; [2 x 6,144, 2,048] silu, 1,024 rows 44.3 / 41.3, 4,500 178 / 148; [2 x 8,192,
+        2,048] clamped, 700 rows 48.0 / 48.1, 1,024 60.0 / 57.3, 2,048 120 / 101, 4,500 271 / 238; gelu, 2,048 rows 117 / 101; [2 x 2,048, 1,024] clamped,
+        1,500 rows (a round and a third of tiles) 17.7 / 24.1, 2,048 22.5 / 20.9, 4,500 40.7 / 36.9; [2 x 4,096, 2,048] clamped, 3,333 rows (six rounds and a
+        tile) 94 / 98, 4,500 127 / 123."""
         M, K = h.shape
         if (M < self.ROWS_MIN or K % 8 or n_out % 8 or h.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or w.shape[1] != K
                 or not self.use_rows or h.stride(1) != 1 or h.stride(0) % 8 or h.data_ptr() % 16 or not w.is_contiguous() or w.data_ptr() % 16):
