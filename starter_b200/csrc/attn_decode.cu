@@ -57,7 +57,13 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restric
     // the lengths, the page table, the norm weights and rotary tables, and pages before the one that holds
     // the new token.  If that kernel releases this one early, the look-ups and first copies below overlap it.
     sb_stamp(4, 0);
-    const int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
+    int seq = blockIdx.x, kvh = blockIdx.y;
+    const int split = blockIdx.z;
+    if (FUSED && fused.order != nullptr) {   // blocks start in the order of their numbers: the longest sequence's pairs first
+        const int number = blockIdx.y * gridDim.x + blockIdx.x;
+        seq = fused.order[number / gridDim.y];
+        kvh = number % gridDim.y;
+    }
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = n_heads / kv.n_kv_heads;
     const int slot = batch.seq_slot[seq];

@@ -239,6 +239,22 @@ __global__ void advance_lengths_kernel(SbBatch b, int* lengths) {
     if (slot != b.null_slot) lengths[slot] += b.cu_q[s + 1] - b.cu_q[s];
 }
 
+// order: the step's sequences by falling length, equal ones by their number.  One block; what it costs is two look-ups and n_seqs
+// comparisons a thread (2 to 4 us), once a step.
+__global__ void __launch_bounds__(1024) length_order_kernel(SbBatch b, int* __restrict__ order) {
+    __shared__ int held[1024];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int s = threadIdx.x;
+    if (s < b.n_seqs) held[s] = b.lengths[b.seq_slot[s]];
+    __syncthreads();
+    if (s >= b.n_seqs) return;
+    const int own = held[s];
+    int rank = 0;
+    for (int j = 0; j < b.n_seqs; ++j) rank += held[j] > own || (held[j] == own && j < s);
+    order[rank] = s;
+}
+
 static inline int row_threads(int width) {
     int t = 32;
     while (t < 256 && t * 4 < width) t <<= 1;
@@ -346,6 +362,14 @@ int sb_swiglu(int dtype, const void* gu, void* out, int rows, int inter, cudaStr
 int sb_advance_lengths(SbBatch b, int* lengths, cudaStream_t stream) {
     if (b.n_seqs <= 0) return 0;
     sb_launch(advance_lengths_kernel, (b.n_seqs + 127) / 128, 128, 0, stream, b, lengths);
+    SB_LAUNCH_CHECK();
+}
+
+// n_seqs <= 1024.
+int sb_length_order(SbBatch b, int* order, cudaStream_t stream) {
+    if (b.n_seqs <= 0) return 0;
+    if (b.n_seqs > 1024) return (int)cudaErrorInvalidValue;
+    sb_launch(length_order_kernel, 1, (b.n_seqs + 31) / 32 * 32, 0, stream, b, order);
     SB_LAUNCH_CHECK();
 }
 

@@ -61,6 +61,7 @@ class DecoderModel:
                 raise ValueError("layers that run in passes need one 32-bit residual and positions that enter in the mixers")
             self.pass_starts = spec.pass_starts()
             self.loop_steps = checkpoint.load(names.loop_step, torch.float32, device).float().contiguous()
+        self.ranks_lengths = any(getattr(part, "ranks_lengths", False) for part in self.parts())   # see ops.begin_step
         self.order = spec.execution_order()
         for i in self.order:
             if not 0 <= i < len(self.blocks):
@@ -128,6 +129,9 @@ class DecoderModel:
 
     def hidden(self, ctx: StepContext, tokens: torch.Tensor):
         """Run the step's rows through every layer; returns the residual stream before the final norm."""
+        begin = getattr(ctx.ops, "begin_step", None)
+        if begin is not None and self.ranks_lengths:
+            begin(ctx)
         if self.spec.streams is not None:   # 32-bit copies of the scaled embedding rows, side by side
             x = ctx.ops.embed_streams(tokens, self.embedding, ctx.status, self.spec.embedding_scale, self.spec.streams)
             stream = StreamResidual(x, self.spec.streams)

@@ -28,6 +28,8 @@ from .registry import build_part, register_part
 
 
 class Attention:
+    ranks_lengths = True   # its decode kernel takes sequences by length where a step ranks them (ops.begin_step)
+
     @staticmethod
     def weight_shapes(spec):
         hq, hkv, d, h = spec.num_heads, spec.num_kv_heads, spec.head_dim, spec.hidden_size
