@@ -14,6 +14,7 @@
 // together once there are enough warps for the GPU either way: 300 rows, 32 heads on 8 of 128, 32-bit: 404 us with a warp
 // per head, 154 with one per four heads (B200).
 #include "common.cuh"
+#include "mma_utils.cuh"
 
 #define AG_MAX_D 256
 
@@ -144,6 +145,152 @@ __global__ void attention_general_kernel(const T* __restrict__ q, T* __restrict_
     }
 }
 
+#define AR_ROWS 8        // rows (warps) of a block
+#define AR_D 128         // head sizes up to this, multiples of 4
+#define AR_LD (AR_D + 4) // a key row's floats in shared memory: lanes read 16 bytes of a row each from different banks
+
+template <int HG> constexpr int ar_smem() {
+    return (2 * 32 * (AR_LD + AR_D) + AR_ROWS * HG * (AR_D + 32)) * (int)sizeof(float);
+}
+
+// The same in 32 bits for steps of long pieces: AR_ROWS neighbouring rows and HG heads a block, a warp a row; the block brings 32 keys
+// and values at a time into shared memory, one tile ahead, for all of them.  Every sum runs in the order of the kernel above, so the
+// results are its results, bit for bit.  Bound: reads of shared memory, a key once for HG heads.  The kernel
+// above read a line of every key row per lane and instruction, for each row anew (300 rows, 32 heads on 8 of 128: 151 us).
+template <int HG>
+__global__ void __launch_bounds__(32 * AR_ROWS, 2) attention_general_rows_kernel(const float* __restrict__ q, float* __restrict__ out, SbBatch batch, SbKV kv,
+                                                                                 int n_heads, float scale, int window) {
+    extern __shared__ __align__(16) float ar_sm[];
+    float* ks = ar_sm;                              // [2][32][AR_LD]
+    float* vs = ks + 2 * 32 * AR_LD;                // [2][32][AR_D]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, D = kv.head_dim;
+    float* qs = vs + 2 * 32 * AR_D + warp * HG * (AR_D + 32);   // this warp's queries [HG][AR_D], then probabilities [HG][32]
+    float* ps = qs + HG * AR_D;
+    pdl_wait();
+    const int row_a = blockIdx.x * AR_ROWS, row_z = min(row_a + AR_ROWS, batch.n_rows), row = row_a + warp;
+    const int head = blockIdx.y * HG, kvh = head / (n_heads / kv.n_kv_heads);
+    const int own_seq = row < row_z ? batch.row_seq[row] : -1;
+    if (own_seq >= 0)
+        for (int h = 0; h < HG; ++h)
+            for (int d = lane; d < D; d += 32) qs[h * AR_D + d] = q[((long long)row * n_heads + head + h) * D + d];
+    __syncwarp();
+    float m[HG], l[HG], acc[HG][AR_D / 32];
+#pragma unroll
+    for (int h = 0; h < HG; ++h) {
+        m[h] = -INFINITY;
+        l[h] = 0.f;
+#pragma unroll
+        for (int j = 0; j < AR_D / 32; ++j) acc[h][j] = 0.f;
+    }
+    const float* kbase = (const float*)kv.k;
+    const float* vbase = (const float*)kv.v;
+    const int last_seq = batch.row_seq[row_z - 1];
+    for (int sq = batch.row_seq[row_a]; sq <= last_seq; ++sq) {   // the sequences that have rows here
+        const int c0 = batch.cu_q[sq], r0 = max(c0, row_a), r1 = min(batch.cu_q[sq + 1], row_z);
+        if (r0 >= r1) continue;
+        const int slot = batch.seq_slot[sq], held = batch.lengths[slot];
+        const int pos_max = held + r1 - 1 - c0, first_pos = held + r0 - c0, pos = held + row - c0;
+        const int lo_min = window > 0 ? max(0, first_pos - window + 1) : 0, lo = window > 0 ? max(0, pos - window + 1) : 0;
+        const int n_first = lo_min / 32 * 32, tiles = (pos_max - n_first) / 32 + 1;
+        auto fetch = [&](int i) {   // 32 keys lie in one page; a tile without a page is skipped below
+            const int n0 = n_first + i * 32;
+            const long long off = i < tiles ? kv_offset(kv, slot, n0, kvh) : -1;
+            if (off >= 0) {
+                const int per = D / 4;
+                for (int e = tid; e < 32 * per; e += 32 * AR_ROWS) {
+                    const int t = e / per, c = (e - t * per) * 4;
+                    float* kd = ks + ((i & 1) * 32 + t) * AR_LD + c;
+                    float* vd = vs + ((i & 1) * 32 + t) * AR_D + c;
+                    if (n0 + t <= pos_max) {
+                        cp_async_16(kd, kbase + off + (long long)t * D + c);
+                        cp_async_16(vd, vbase + off + (long long)t * D + c);
+                    } else {
+                        *reinterpret_cast<float4*>(kd) = make_float4(0.f, 0.f, 0.f, 0.f);
+                        *reinterpret_cast<float4*>(vd) = make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                }
+            }
+            cp_async_commit();
+        };
+        fetch(0);
+        for (int i = 0; i < tiles; ++i) {
+            const int n0 = n_first + i * 32;
+            fetch(i + 1);
+            cp_async_wait<1>();
+            __syncthreads();
+            const int t_lo = max(lo - n0, 0), t_hi = min(pos - n0, 31);
+            if (own_seq == sq && t_lo <= t_hi && kv_offset(kv, slot, n0, kvh) >= 0) {
+                const bool valid = lane >= t_lo && lane <= t_hi;
+                const float* kr = ks + ((i & 1) * 32 + lane) * AR_LD;
+                float s[HG];
+#pragma unroll
+                for (int h = 0; h < HG; ++h) s[h] = 0.f;
+#pragma unroll 4
+                for (int d = 0; d < D; d += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(kr + d);
+#pragma unroll
+                    for (int h = 0; h < HG; ++h) {
+                        const float4 x = *reinterpret_cast<const float4*>(qs + h * AR_D + d);
+                        s[h] = fmaf(x.x, v.x, s[h]);
+                        s[h] = fmaf(x.y, v.y, s[h]);
+                        s[h] = fmaf(x.z, v.z, s[h]);
+                        s[h] = fmaf(x.w, v.w, s[h]);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < HG; ++h) {
+                    s[h] = valid ? s[h] * scale : -INFINITY;
+                    const float m_new = fmaxf(m[h], warp_max(s[h]));
+                    const float p = valid && m_new != -INFINITY ? expf(s[h] - m_new) : 0.f;
+                    const float alpha = m_new == -INFINITY ? 1.f : expf(m[h] - m_new);
+                    l[h] = l[h] * alpha + warp_sum(p);
+                    m[h] = m_new;
+                    ps[h * 32 + lane] = p;
+#pragma unroll
+                    for (int j = 0; j < AR_D / 32; ++j) acc[h][j] *= alpha;
+                }
+                __syncwarp();
+                const float* vt = vs + (i & 1) * 32 * AR_D + lane;
+#pragma unroll 4
+                for (int t = t_lo; t <= t_hi; ++t) {
+                    float pt[HG];
+#pragma unroll
+                    for (int h = 0; h < HG; ++h) pt[h] = ps[h * 32 + t];
+#pragma unroll
+                    for (int j = 0; j < AR_D / 32; ++j) {
+                        const float v = vt[t * AR_D + 32 * j];   // columns past D are never stored
+#pragma unroll
+                        for (int h = 0; h < HG; ++h) acc[h][j] = fmaf(pt[h], v, acc[h][j]);
+                    }
+                }
+                __syncwarp();
+            }
+            __syncthreads();
+        }
+        cp_async_wait<0>();
+    }
+    if (own_seq < 0) return;
+#pragma unroll
+    for (int h = 0; h < HG; ++h) {
+        float* orow = out + ((long long)row * n_heads + head + h) * D;
+        const float inv = 1.0f / l[h];
+#pragma unroll
+        for (int j = 0; j < AR_D / 32; ++j) {
+            const int d = lane + 32 * j;
+            if (d < D) orow[d] = acc[h][j] * inv;
+        }
+    }
+}
+
+template <int HG>
+static int ar_launch(const float* q, float* out, SbBatch batch, SbKV kv, int n_heads, float scale, int window, cudaStream_t stream) {
+    static const cudaError_t configured = cudaFuncSetAttribute(attention_general_rows_kernel<HG>, cudaFuncAttributeMaxDynamicSharedMemorySize, ar_smem<HG>());
+    if (configured != cudaSuccess) return (int)configured;
+    sb_launch(attention_general_rows_kernel<HG>, dim3((batch.n_rows + AR_ROWS - 1) / AR_ROWS, n_heads / HG), dim3(32 * AR_ROWS), ar_smem<HG>(), stream, q, out,
+              batch, kv, n_heads, scale, window);
+    return 0;
+}
+
 template <class T, int HG>
 static void ag_launch(const void* q, void* out, SbBatch batch, SbKV kv, int n_heads, float scale, int window, cudaStream_t stream) {
     const dim3 grid(batch.n_rows, n_heads / HG);
@@ -169,6 +316,17 @@ extern "C" int sb_attention_general(int dtype, const void* q, void* out, SbBatch
     if (batch.n_rows <= 0) return 0;
     if (kv.head_dim > AG_MAX_D || n_heads % kv.n_kv_heads) return (int)cudaErrorInvalidValue;
     if (n_heads > 65535) return (int)cudaErrorInvalidValue;
+    // Rows that share their keys: pieces of some length on average (a block's rows then lie in one sequence or two).
+    const int G = n_heads / kv.n_kv_heads;
+    if (dtype == SB_F32 && batch.n_rows >= 64 && batch.n_rows / 16 >= batch.n_seqs && kv.head_dim <= AR_D && kv.head_dim % 4 == 0 &&
+        sb_aligned(16, (const char*)kv.k, (const char*)kv.v)) {
+        static_assert(SB_PAGE % 32 == 0, "a tile of 32 keys lies in one page");
+        const int e = G % 4 == 0   ? ar_launch<4>((const float*)q, (float*)out, batch, kv, n_heads, scale, window, stream)
+                      : G % 2 == 0 ? ar_launch<2>((const float*)q, (float*)out, batch, kv, n_heads, scale, window, stream)
+                                   : ar_launch<1>((const float*)q, (float*)out, batch, kv, n_heads, scale, window, stream);
+        if (e) return e;
+        SB_LAUNCH_CHECK();
+    }
     if (dtype == SB_F32)
         ag_pick<float>(q, out, batch, kv, n_heads, scale, window, stream);
     else

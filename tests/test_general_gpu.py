@@ -107,3 +107,36 @@ def test_the_count_of_launches(ops, M, N, K, dtype, kernels):
     before = ops.launches
     ops.linear(a, w)
     assert ops.launches - before == kernels
+
+
+@pytest.mark.parametrize("D, G, Gk", [(128, 4, 2), (36, 6, 1), (64, 1, 3)])
+@pytest.mark.parametrize("window", [None, 70])
+def test_attention_32_bit_of_long_pieces(ops, D, G, Gk, window):
+    """From 64 rows on rows share their keys in shared memory: the same bits as row by row, at pieces that end inside blocks of 8
+    rows and tiles of 32 keys."""
+    H, lens = G * Gk, [97, 3, 201]
+    cache = Cache([KVRequest(Gk, D)], n_slots=4, max_tokens=64 * 16, dtype=torch.float32, device="cuda", max_seq_tokens=320)
+    layer, slots = cache.layers[0], [cache.alloc() for _ in lens]
+    for s, n in zip(slots, lens):
+        cache.reserve(s, n)
+    cache.flush()
+    layer.k.copy_(rand(layer.k.shape, 3)), layer.v.copy_(rand(layer.v.shape, 4))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    q = rand((sum(lens), H * D), 5)
+
+    def run(held, counts, rows):
+        cache.lengths.zero_()
+        cache.lengths[torch.tensor(slots, device="cuda")] = i32(held)
+        cu = [sum(counts[:b]) for b in range(4)]
+        ctx = StepContext(runtime=None, cache=cache, n_seqs=3, n_rows=cu[3], max_q_len=max(counts), kv_bound=300, seq_slot=i32(slots), cu_q=i32(cu),
+                          row_seq=i32([b for b, n in enumerate(counts) for _ in range(n)]), lengths=cache.lengths, status=i32([0]))
+        return ops.attention(ctx, rows, layer, H, D ** -0.5, window)
+
+    got = run([0, 0, 0], lens, q)
+    first = [0, 97, 100]
+    for piece in range(0, 201, 19):      # up to 57 rows a step: a warp a row
+        counts = [max(0, min(19, n - piece)) for n in lens]
+        held = [min(piece, n) for n in lens]
+        rows = torch.cat([q[f + h:f + h + c] for f, h, c in zip(first, held, counts)])
+        want = run(held, counts, rows)
+        assert torch.equal(torch.cat([got[f + h:f + h + c] for f, h, c in zip(first, held, counts)]), want)
