@@ -24,19 +24,37 @@ __device__ __forceinline__ void mf_mma(float (&c)[4], const uint4& a, const uint
     mma_bf16(c, hi, x.z, x.w);
 }
 
+// An expert that every row of the step takes beside the chosen ones (a shared expert): its columns are blocks of the same launches,
+// the first ones, since it is the widest.  rows = 0: there is none.
+struct MfShared {
+    const __nv_bfloat16* x;
+    const __nv_bfloat16* w;
+    __nv_bfloat16* out;
+    int rows, K, n_cols, silu;
+    float alpha, limit;
+};
+
 // GATE_UP: out[pair][c] = act(gate_c, up_c) of x = h's row pair / top, w = [2 n_cols][K] per expert, gate over up.  Otherwise
 // out[pair][c] = w_c x with x = the pair's own row, w = [n_cols][K] per expert.
 template <bool GATE_UP>
 __global__ void __launch_bounds__(32 * MF_WARPS, 3)
-moe_few_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ chosen, const __nv_bfloat16* __restrict__ w,
-               __nv_bfloat16* __restrict__ out, int n_pairs, int top, int K, int n_cols, float alpha, float limit, int silu) {
+moe_few_kernel(const __nv_bfloat16* x, const int* __restrict__ chosen, const __nv_bfloat16* w, __nv_bfloat16* out, int n_pairs, int top, int K,
+               int n_cols, float alpha, float limit, int silu, MfShared shared) {
     constexpr int M = GATE_UP ? 2 : 1;
     __shared__ int list[MF_MAX_PAIRS];
     __shared__ int count_s;
     __shared__ float red[MF_WARPS][M][MF_NT][16][9];
     pdl_wait();
-    const int e = blockIdx.y, c0 = blockIdx.x * 16, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    if (warp == 0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int first_blocks = shared.rows > 0 ? (shared.n_cols + 15) / 16 : 0, per_expert = (n_cols + 15) / 16;
+    const bool all = (int)blockIdx.x < first_blocks;
+    const int b0 = blockIdx.x - (all ? 0 : first_blocks), e = all ? 0 : b0 / per_expert, c0 = (all ? b0 : b0 % per_expert) * 16;
+    if (all) {
+        x = shared.x, w = shared.w, out = shared.out, K = shared.K, n_cols = shared.n_cols, silu = shared.silu, alpha = shared.alpha, limit = shared.limit;
+        top = 1;
+        for (int i = threadIdx.x; i < shared.rows; i += 32 * MF_WARPS) list[i] = i;
+        if (threadIdx.x == 0) count_s = shared.rows;
+    } else if (warp == 0) {
         int n = 0;
         for (int p0 = 0; p0 < n_pairs; p0 += 32) {
             const bool hit = p0 + lane < n_pairs && chosen[p0 + lane] == e;
@@ -115,7 +133,8 @@ moe_few_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ chos
                 if (GATE_UP) {
                     float gt = rnd<__nv_bfloat16>(s[0]), up = rnd<__nv_bfloat16>(s[M - 1]);
                     if (silu) {
-                        y = gt / (1.0f + expf(-gt)) * up;
+                        const float a = gt / (1.0f + expf(-gt));
+                        y = (all ? rnd<__nv_bfloat16>(a) : a) * up;   // a dense feed-forward rounds silu(gate) first
                     } else {
                         gt = fminf(gt, limit);
                         up = fminf(fmaxf(up, -limit), limit);
@@ -132,17 +151,26 @@ moe_few_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ chos
 extern "C" {
 
 // h [rows, width], act [n_pairs, ff], down [n_pairs, width]; w_gate_up [experts, 2 ff, width], w_down [experts, width, ff];
-// width and ff multiples of 32, everything 16-byte aligned.
+// width and ff multiples of 32, everything 16-byte aligned.  s_ff > 0: the shared expert's s_gate_up [2 s_ff, width], s_down [width, s_ff],
+// s_act [rows, s_ff] and s_out [rows, width] under the same conditions.
 int sb_moe_few(const void* h, const int* chosen, const void* w_gate_up, const void* w_down, void* act, void* down, int n_pairs, int top,
-               int n_experts, int width, int ff, float alpha, float limit, int silu, cudaStream_t stream) {
+               int n_experts, int width, int ff, float alpha, float limit, int silu, const void* s_gate_up, const void* s_down, void* s_act,
+               void* s_out, int s_ff, float s_alpha, float s_limit, int s_silu, cudaStream_t stream) {
     if (n_pairs <= 0 || n_experts <= 0) return 0;
-    if (n_pairs > MF_MAX_PAIRS || n_experts > 65535 || width % 32 || ff % 32 || top < 1 || !sb_aligned(16, h, w_gate_up, w_down, act, down))
+    if (n_pairs > MF_MAX_PAIRS || n_experts > 65535 || width % 32 || ff % 32 || top < 1 || !sb_aligned(16, h, w_gate_up, w_down, act, down) ||
+        s_ff < 0 || s_ff % 32 || (s_ff > 0 && !sb_aligned(16, s_gate_up, s_down, s_act, s_out)))
         return (int)cudaErrorInvalidValue;
     typedef __nv_bfloat16 bf;
-    sb_launch(moe_few_kernel<true>, dim3((ff + 15) / 16, n_experts), 32 * MF_WARPS, 0, stream, (const bf*)h, chosen, (const bf*)w_gate_up,
-              (bf*)act, n_pairs, top, width, ff, alpha, limit, silu);
-    sb_launch(moe_few_kernel<false>, dim3((width + 15) / 16, n_experts), 32 * MF_WARPS, 0, stream, (const bf*)act, chosen, (const bf*)w_down,
-              (bf*)down, n_pairs, top, ff, width, 0.f, 0.f, 0);
+    const int rows = s_ff > 0 ? n_pairs / top : 0;
+    const MfShared up = {(const bf*)h, (const bf*)s_gate_up, (bf*)s_act, rows, width, s_ff, s_silu, s_alpha, s_limit};
+    const MfShared dn = {(const bf*)s_act, (const bf*)s_down, (bf*)s_out, rows, s_ff, width, 0, 0.f, 0.f};
+    const long long b1 = (long long)((ff + 15) / 16) * n_experts + (rows ? (s_ff + 15) / 16 : 0);
+    const long long b2 = (long long)((width + 15) / 16) * (n_experts + (rows ? 1 : 0));
+    if (b1 > 0x7fffffff || b2 > 0x7fffffff) return (int)cudaErrorInvalidValue;
+    sb_launch(moe_few_kernel<true>, dim3((unsigned int)b1), 32 * MF_WARPS, 0, stream, (const bf*)h, chosen, (const bf*)w_gate_up, (bf*)act, n_pairs,
+              top, width, ff, alpha, limit, silu, up);
+    sb_launch(moe_few_kernel<false>, dim3((unsigned int)b2), 32 * MF_WARPS, 0, stream, (const bf*)act, chosen, (const bf*)w_down, (bf*)down, n_pairs,
+              top, ff, width, 0.f, 0.f, 0, dn);
     SB_LAUNCH_CHECK();
 }
 

@@ -199,7 +199,7 @@ class Ops:
             "sb_moe_pairs": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                              c_float, c_float, c_int, c_void_p],
             "sb_moe_few": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
-                           c_int, c_void_p],
+                           c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_float, c_int, c_void_p],
             "sb_moe_combine": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                c_int, c_void_p, c_int, c_void_p],
             "sb_chunk_memory_launches": [c_int, c_int, c_int, c_int, c_int, c_int, c_longlong],
@@ -1752,13 +1752,30 @@ class Ops:
         return (h.dtype == torch.bfloat16 and width % 32 == 0 and ff % 32 == 0 and h.is_contiguous() and h.data_ptr() % 16 == 0
                 and w_gate_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
 
-    def moe_experts(self, h, chosen, weight, w_gate_up, w_down, n_experts, alpha, limit, base, base_gate=None):
+    SHARED_FEW_MIN, SHARED_FEW_ROWS = 17, 32   # rows at which the shared expert runs inside the kernels of the chosen ones
+
+    def moe_takes_shared(self, h, top, n_experts, w_gate_up, w_down, s_gate_up, s_down) -> bool:
+        """Whether a step's shared expert (a gated feed-forward that every row takes: s_gate_up [2 s_ff, width], s_down [width, s_ff]) runs in the
+        launches of the chosen experts (moe_few.cu) and not as products of its own: three launches less a layer.  Six layers of 16 experts
+        of 3 x 1,024 x 512 and a shared one of 3 x 1,024 x 2,048, 24 rows: 506 -> 455 us a step.  Up to 16 rows the shared expert has the
+        decode products (tile-major weights, activation in their epilogue), which stream a wide one sooner (3 x 2,048 x 4,096, 8 rows: 647
+        us with them, 655 among the chosen); more than two reads of its weights are not made up for."""
+        rows, width = h.shape
+        if n_experts < 1 or not self.SHARED_FEW_MIN <= rows <= self.SHARED_FEW_ROWS:
+            return False
+        return (self._moe_takes_few(h, rows * top, n_experts, width, w_down.shape[2], w_gate_up, w_down) and s_down.shape[1] % 32 == 0
+                and s_gate_up.dtype == torch.bfloat16 and s_gate_up.is_contiguous() and s_down.is_contiguous()
+                and s_gate_up.data_ptr() % 16 == 0 and s_down.data_ptr() % 16 == 0)
+
+    def moe_experts(self, h, chosen, weight, w_gate_up, w_down, n_experts, alpha, limit, base, base_gate=None, shared=None):
         """base (times sigmoid(base_gate), 32-bit [rows, 1], when given) + sum_k weight[:, k] * expert_chosen[:, k](h): experts are gated feed-forwards (the clamped activation with
         its sigmoid factor ``alpha`` and ``limit``, or silu(gate) * up when ``alpha`` is None) with stacked
         matrices w_gate_up [experts, 2 ff, width] (gate over up) and w_down [experts, width, ff]; a choice >= n_experts
         is an identity output and adds weight * h.  A few pairs: each pair streams its expert's matrices; some hundreds: every
         expert's matrices are read once for its pairs.  Many pairs in bfloat16: the pairs are put in the order of their experts on the
-        device and each matrix takes one grouped product, the first with the activation in its epilogue (gemm_rows.cu)."""
+        device and each matrix takes one grouped product, the first with the activation in its epilogue (gemm_rows.cu).
+        ``shared`` (in ``base``'s place, where ``moe_takes_shared`` says so): (s_gate_up, s_down, alpha or None, limit) of the expert
+        whose output is the base."""
         rows, width = h.shape
         top = chosen.shape[1]
         pairs = rows * top
@@ -1770,11 +1787,20 @@ class Ops:
                     or not w_gate_up.is_contiguous() or not w_down.is_contiguous() or w_gate_up.dtype != h.dtype):
                 raise KernelError("moe_experts: stacked matrices [experts, 2 ff, width] and [experts, width, ff] in the run's dtype")
             few = self._moe_takes_few(h, pairs, n_experts, width, ff, w_gate_up, w_down)
+            s_args = (None, None, None, None, 0, 0.0, 0.0, 0)
+            if shared is not None:
+                s_gate_up, s_down, s_alpha, s_limit = shared
+                s_ff = s_down.shape[1]
+                if not few or base is not None or tuple(s_gate_up.shape) != (2 * s_ff, width) or s_down.shape[0] != width:
+                    raise KernelError("moe_experts: a shared expert [2 s_ff, width], [width, s_ff] goes with the kernels of few rows")
+                s_act = torch.empty((rows, s_ff), dtype=h.dtype, device=h.device)
+                base = torch.empty((rows, width), dtype=h.dtype, device=h.device)
+                s_args = (_ptr(s_gate_up), _ptr(s_down), _ptr(s_act), _ptr(base), s_ff, float(s_alpha or 0.0), float(s_limit or 0.0), int(s_alpha is None))
             if few:
                 act = torch.empty((pairs, ff), dtype=h.dtype, device=h.device)
                 down = torch.empty((pairs, width), dtype=h.dtype, device=h.device)
                 self._check(self.lib.sb_moe_few(_ptr(h), _ptr(chosen), _ptr(w_gate_up), _ptr(w_down), _ptr(act), _ptr(down), pairs, top,
-                                                n_experts, width, ff, float(alpha or 0.0), float(limit or 0.0), int(alpha is None),
+                                                n_experts, width, ff, float(alpha or 0.0), float(limit or 0.0), int(alpha is None), *s_args,
                                                 self._stream()), "moe_few")
                 self.launches += 1
             elif (h.dtype == torch.bfloat16 and pairs > self.MOE_PAIRS_MAX and width % 8 == 0 and ff % 8 == 0

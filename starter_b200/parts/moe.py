@@ -80,13 +80,21 @@ class MixtureOfExperts:
 
     def forward(self, ctx, h):
         s, ops = self.spec, self.ops
-        base = self.shared.forward(ctx, h) if self.shared is not None else None
+        f, more = self.shared, {}
+        takes = getattr(ops, "moe_takes_shared", None) if f is not None else None
+        if takes is not None and f.activation in ("silu", "clamped_swish") and takes(h, s.top, s.n_experts, self.w_gate_up, self.w_down,
+                                                                                     f.w_gate_up, f.w_down):
+            base = None   # the shared expert runs among the chosen ones
+            more["shared"] = (f.w_gate_up, f.w_down, *((f.alpha, f.limit) if f.activation == "clamped_swish" else (None, 0.0)))
+        else:
+            base = f.forward(ctx, h) if f is not None else None
         options = {}
         if s.scores != "softmax" or s.groups > 1 or self.gated:
             options = {"scores": s.scores, "groups": s.groups, "keep_groups": s.keep_groups, "extra": int(self.gated)}
         chosen, weight, *gate = ops.moe_route(h, self.router, self.correction, s.top, float(s.route_scale), bias=self.bias,
                                               over_chosen=s.over_chosen, **options)
-        more = {"base_gate": gate[0]} if self.gated else {}
+        if self.gated:
+            more["base_gate"] = gate[0]
         return ops.moe_experts(h, chosen, weight, self.w_gate_up, self.w_down, s.n_experts, self.alpha, self.limit, base, **more)
 
 

@@ -142,3 +142,37 @@ def test_the_rule_where_an_expert_s_weights_are_read_more_than_once():
     assert [takes(n, 16, 1024, 512) for n in (320, 512)] == [True, True]            # 50 MB
     assert [takes(n, 16, 1024, 4096) for n in (320, 321)] == [True, False]         # 403 MB
     assert [takes(n, 32, 4096, 1408) for n in (448, 449)] == [True, False]         # 1.1 GB
+
+
+@pytest.mark.parametrize("rows, E, width, ff, s_ff", [(17, 3, 64, 32, 96), (25, 4, 96, 64, 32), (32, 2, 32, 32, 160), (19, 6, 160, 96, 2048)])
+@pytest.mark.parametrize("alpha, s_alpha", [(None, None), (1.3, None), (None, 0.7)])
+def test_the_shared_expert_among_the_chosen(rows, E, width, ff, s_ff, alpha, s_alpha):
+    """Every row's pair of the shared expert in the launches of the chosen ones: against its products in 64 bits, and the chosen experts as
+    they are without it."""
+    from starter_b200.csrc.ops import get_ops
+    ops, top = get_ops(verbose=False), 2
+    g = torch.Generator().manual_seed(rows)
+    rand = lambda *s, scale=1.0: (torch.randn(*s, generator=g) * scale).bfloat16().cuda()   # noqa: E731
+    chosen = torch.stack([torch.randperm(E + 1, generator=g)[:top] for _ in range(rows)]).int().cuda()
+    h, weight = rand(rows, width), torch.rand(rows, top, generator=g).cuda()
+    gu, down = rand(E, 2 * ff, width, scale=width ** -0.5), rand(E, width, ff, scale=ff ** -0.5)
+    s_gu, s_down = rand(2 * s_ff, width, scale=width ** -0.5), rand(width, s_ff, scale=s_ff ** -0.5)
+    z = (h.double() @ s_gu.double().T).bfloat16().double()
+    a, b = z[:, :s_ff], z[:, s_ff:]
+    if s_alpha is None:
+        act = (a * torch.sigmoid(a)).bfloat16().double() * b
+    else:
+        a, b = a.clamp(max=0.8), b.clamp(-0.8, 0.8)
+        act = a * torch.sigmoid(s_alpha * a) * (b + 1.0)
+    base = act.bfloat16().double() @ s_down.double().T
+    takes = ops._moe_takes_few
+    ops._moe_takes_few = lambda *a: True
+    try:
+        assert ops.moe_takes_shared(h, top, E, gu, down, s_gu, s_down) and not ops.moe_takes_shared(h[:16], top, E, gu, down, s_gu, s_down)
+        got = ops.moe_experts(h, chosen, weight, gu, down, E, alpha, 3.0, None, shared=(s_gu, s_down, s_alpha, 0.8))
+        want = ops.moe_experts(h, chosen, weight, gu, down, E, alpha, 3.0, base.bfloat16())
+    finally:
+        ops._moe_takes_few = takes
+    # the base may have been rounded to its neighbour (2^-8 of a value), so may the sum
+    assert float((got.double() - want.double()).abs().max()) <= 2 ** -6 * float(want.double().abs().max())
+    assert float((got.double() - want.double()).norm() / want.double().norm()) < 4e-3
