@@ -1,0 +1,420 @@
+// Products of 32-bit numbers on the bfloat16 tensor cores, C[M, N] = A[M, K] W[N, K]^T: every number is the sum of three bfloat16 numbers
+// (8 + 8 + 8 bits of its 24), and of the nine products of their parts the six largest are summed, in 32 bits; what is left out is below
+// 2^-25 of a product.  For more than a few rows of the matrices of a model's layers; gemm_general.cu takes the others.
+//
+// Bound: six bfloat16 products on tcgen05 where the CUDA cores have one 32-bit multiply-add: 270 TFLOP/s of 32-bit work at the measured
+// bfloat16 rate against their 74.
+//
+// Precision.  The tensor core adds to its 32-bit sums without rounding to nearest.  So its sums run over 64 columns of k only, the five
+// small products first and the large one last (four additions at the size of the sum); the sums of 64 columns are added in
+// registers, rounded to nearest, in order.  Error against 64 bits (2-norm, normally distributed numbers, 1 to 4,500 rows of [2,560 to
+// 151,936, 2,560 to 9,728]): 1.1e-7 to 1.4e-7, the CUDA cores' product 4.1e-7.
+//
+// An output is a function of its row of A, its row of W and of N and K: the columns of k are cut into segments by N and K alone, a segment
+// is one running sum over its 64s in order, and segments are added in order; which rows stand beside it changes nothing.
+//
+// A pair of blocks (two SMs) takes units of (256 rows of W, NT rows of A, segment).  W comes by TMA as it is; eight warps split it, half a
+// row of a stage a thread, into tensor memory, where it is the product's left operand; A was split by a kernel before (it is read by all
+// rows of W) and comes by TMA as the right one, half of it to each SM; one thread issues the products of the pair; four warps add the
+// finished sums to their own, and the last to bring a segment of its columns adds the segments up.  A number that is infinite or NaN, or
+// too large for bfloat16, makes its parts' sums NaN: outputs that are not finite are worked out again from the numbers themselves.
+#include "tc_maps.cuh"
+#include "tc_utils.cuh"
+
+#define GS_THREADS 512     // warp 0: copies, 1: products, 4 to 11: split W, 12 to 15: sums; groups of four with registers of their own
+#define GS_NT_MAX 112      // rows of A in a unit: what four warps' registers hold
+#define GS_W_BYTES 32768   // a stage's 128 rows x 64 columns of W
+#define GS_STAGES_MAX 6
+#define GS_SMEM (226 * 1024)
+#define GS_A_COL 224       // tensor memory: two buffers of NT sums from column 0, three of 3 x 32 columns of split W from here
+#define GS_A_BUFS 3
+
+struct GsArgs {
+    const float* a;
+    const float* w;
+    float* out;
+    float* sums;          // [n_seg][M][N] where there is more than one segment
+    int* arrived;         // [w_tiles][x_tiles][8 warps]: segments whose sums are there
+    int* status;
+    int M, N, K, nt, stages, seg_k, n_seg, w_tiles, x_tiles;
+};
+
+__device__ __forceinline__ uint32_t gs_in_block(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void gs_load(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void gs_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void gs_commit(uint64_t* bar) {   // to this place in both blocks
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void gs_arrive_first(uint64_t* bar) {   // at the first block's barrier
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(gs_in_block(bar, 0)) : "memory");
+}
+__device__ __forceinline__ void gs_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+                   "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                 : "memory");
+}
+
+// Two neighbours as three pairs of bfloat16 numbers, the first in the low half.
+__device__ __forceinline__ void gs_split(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+    auto pack = [](float lo, float hi) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&v);
+    };
+    h = pack(x, y);
+    x -= __uint_as_float(h << 16), y -= __uint_as_float(h & 0xffff0000u);
+    m = pack(x, y);
+    x -= __uint_as_float(m << 16), y -= __uint_as_float(m & 0xffff0000u);
+    l = pack(x, y);
+}
+
+// A as [3][M][K] bfloat16, the largest parts first.  K is a multiple of 8.  The counters of the kernel behind it start at zero.
+__global__ void __launch_bounds__(256) gemm_split_rows_kernel(const float* __restrict__ a, uint4* __restrict__ parts, long long n8, int* __restrict__ arrived,
+                                                              int n_arrived) {
+    pdl_wait();
+    pdl_launch_dependents();
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n_arrived; i += gridDim.x * 256) arrived[i] = 0;
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n8; i += gridDim.x * 256ll) {
+        const float4 x = reinterpret_cast<const float4*>(a)[2 * i], y = reinterpret_cast<const float4*>(a)[2 * i + 1];
+        uint4 h, m, l;
+        gs_split(x.x, x.y, h.x, m.x, l.x);
+        gs_split(x.z, x.w, h.y, m.y, l.y);
+        gs_split(y.x, y.y, h.z, m.z, l.z);
+        gs_split(y.z, y.w, h.w, m.w, l.w);
+        parts[i] = h, parts[n8 + i] = m, parts[2 * n8 + i] = l;
+    }
+}
+
+// Sixteen sums of a column, row after row, and whether one is not finite.  A function of its own: written out for every sum of a unit,
+// the code is fetched as slowly as it runs once a unit.
+__device__ __noinline__ bool gs_store16(float* out, long long ld, int rows, float v0, float v1, float v2, float v3, float v4, float v5, float v6, float v7,
+                                        float v8, float v9, float v10, float v11, float v12, float v13, float v14, float v15) {
+    const float v[16] = {v0, v1, v2, v3, v4, v5, v6, v7, v8, v9, v10, v11, v12, v13, v14, v15};
+    bool odd = false;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        if (i < rows) {
+            __stcg(out + i * ld, v[i]);
+            odd |= !(fabsf(v[i]) <= 3.402823466e38f);
+        }
+    return odd;
+}
+#define GS_STORE16(out, ld, rows, v, o)                                                                                                          \
+    gs_store16(out, ld, rows, (v)[o], (v)[o + 1], (v)[o + 2], (v)[o + 3], (v)[o + 4], (v)[o + 5], (v)[o + 6], (v)[o + 7], (v)[o + 8], (v)[o + 9], \
+               (v)[o + 10], (v)[o + 11], (v)[o + 12], (v)[o + 13], (v)[o + 14], (v)[o + 15])
+
+__global__ void __launch_bounds__(GS_THREADS, 1) __cluster_dims__(2, 1, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ GsArgs args) {
+    extern __shared__ unsigned char gs_raw[];
+    __shared__ uint64_t w_full[GS_STAGES_MAX], w_empty[GS_STAGES_MAX], x_full[GS_STAGES_MAX], x_empty[GS_STAGES_MAX];
+    __shared__ uint64_t a_ready[GS_A_BUFS], a_empty[GS_A_BUFS], sum_full[2], sum_empty[2];
+    __shared__ uint32_t tmem_s;
+    __shared__ int abort_s;
+    unsigned char* sm = gs_raw + ((1024 - (smem_u32(gs_raw) & 1023)) & 1023);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = blockIdx.x & 1;
+    volatile int* abort_flag = &abort_s;
+    const int x_part = args.nt * 64;                 // bytes of a part of this block's NT / 2 rows: 128 a row
+    const int stage_bytes = GS_W_BYTES + 3 * x_part;
+
+    if (tid == 0) {
+        abort_s = 0;
+        for (int s = 0; s < GS_STAGES_MAX; ++s) mbar_init(w_full + s, 1), mbar_init(w_empty + s, 8), mbar_init(x_full + s, 1), mbar_init(x_empty + s, 1);
+        for (int b = 0; b < GS_A_BUFS; ++b) mbar_init(a_ready + b, 16), mbar_init(a_empty + b, 1);
+        for (int b = 0; b < 2; ++b) mbar_init(sum_full + b, 1), mbar_init(sum_empty + b, 8);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_s)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    pdl_wait();
+    tc_fence_before();
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    tc_fence_after();
+    const uint32_t tmem = tmem_s;
+    const int units = args.w_tiles * args.x_tiles * args.n_seg, pairs = gridDim.x >> 1;
+
+    auto unit_of = [&](int u, int& wt, int& xt, int& seg, int& turns) {   // neighbours share their rows of W
+        xt = u % args.x_tiles;
+        wt = u / args.x_tiles % args.w_tiles;
+        seg = u / args.x_tiles / args.w_tiles;
+        turns = (min(args.seg_k, args.K - seg * args.seg_k) + 63) / 64;
+    };
+
+    // The groups' registers (80, 104 twice, 208 a thread) stay within what the block was launched with, 4 x 128.
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 80;" ::: "memory");
+        if (warp == 0 && lane == 0) {   // ---- copies
+            int stage = 0, phase = 0;
+            bool ok = true;
+            for (int u = blockIdx.x >> 1; u < units && ok; u += pairs) {
+                int wt, xt, seg, turns;
+                unit_of(u, wt, xt, seg, turns);
+                const int yw = wt * 256 + rank * 128, yx = xt * args.nt + rank * (args.nt / 2);
+                for (int k = 0; k < turns; ++k) {
+                    ok = mbar_wait(w_empty + stage, phase ^ 1, abort_flag, args.status) && mbar_wait(x_empty + stage, phase ^ 1, abort_flag, args.status);
+                    if (!ok) break;
+                    unsigned char* w_s = sm + stage * stage_bytes;
+                    const int kx = seg * args.seg_k + k * 64;
+                    mbar_expect_tx(w_full + stage, GS_W_BYTES);
+                    tma_load_2d(w_s, &map_w, kx, yw, w_full + stage);
+                    tma_load_2d(w_s + GS_W_BYTES / 2, &map_w, kx + 32, yw, w_full + stage);
+                    if (rank == 0) mbar_expect_tx(x_full + stage, 6 * x_part);
+                    const uint32_t bar = gs_in_block(x_full + stage, 0);
+                    for (int p = 0; p < 3; ++p) gs_load(w_s + GS_W_BYTES + p * x_part, &map_x, kx, p * args.M + yx, bar);
+                    if (++stage == args.stages) stage = 0, phase ^= 1;
+                }
+            }
+            pdl_launch_dependents();
+            if (*abort_flag) {   // copies may still be under way: they end long before this does
+                const long long t0 = clock64();
+                while (clock64() - t0 < (1ll << 22)) {}
+            }
+        }
+        if (warp == 1 && lane == 0 && rank == 0) {   // ---- products
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(args.nt >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+            const uint64_t x0 = desc_k_major(sm + GS_W_BYTES);
+            int stage = 0, phase = 0, n = 0, ab = 0, ap = 0;
+            bool ok = true;
+            for (int u = blockIdx.x >> 1; u < units && ok; u += pairs) {
+                int wt, xt, seg, turns;
+                unit_of(u, wt, xt, seg, turns);
+                for (int k = 0; k < turns; ++k, ++n) {
+                    const int b = n & 1, ph = (n >> 1) & 1;
+                    ok = mbar_wait(sum_empty + b, ph ^ 1, abort_flag, args.status) && mbar_wait(x_full + stage, phase, abort_flag, args.status) &&
+                         mbar_wait(a_ready + ab, ap, abort_flag, args.status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t d = tmem + b * args.nt, wh = tmem + GS_A_COL + ab * 96, wm = wh + 32, wl = wh + 64;
+                    const uint64_t xh = x0 + (uint64_t)((stage * stage_bytes) >> 4), xm = xh + (x_part >> 4), xl = xm + (x_part >> 4);
+                    const uint32_t left[6] = {wl, wh, wm, wm, wh, wh};
+                    const uint64_t right[6] = {xh, xl, xm, xh, xm, xh};
+#pragma unroll
+                    for (int p = 0; p < 6; ++p)
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) gs_mma(d, left[p] + 8 * kk, right[p] + 2 * kk, idesc, p > 0 || kk > 0);
+                    gs_commit(x_empty + stage);
+                    gs_commit(a_empty + ab);
+                    gs_commit(sum_full + b);
+                    if (++ab == GS_A_BUFS) ab = 0, ap ^= 1;
+                    if (++stage == args.stages) stage = 0, phase ^= 1;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp < 12) {   // ---- split W
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 104;" ::: "memory");
+        const int half = (warp - 4) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+        const uint32_t dst0 = tmem + GS_A_COL + ((uint32_t)(quarter * 32) << 16) + half * 16;
+        int stage = 0, phase = 0, ab = 0, ap = 0;
+        bool ok = true;
+        for (int u = blockIdx.x >> 1; u < units && ok; u += pairs) {
+            int wt, xt, seg, turns;
+            unit_of(u, wt, xt, seg, turns);
+            for (int k = 0; k < turns; ++k) {
+                ok = mbar_wait(w_full + stage, phase, abort_flag, args.status);
+                if (!ok) break;
+                const unsigned char* src = sm + stage * stage_bytes + half * (GS_W_BYTES / 2) + row * 128;
+                uint32_t h[16], m[16], l[16];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float4 v = *reinterpret_cast<const float4*>(src + ((c ^ (row & 7)) << 4));
+                    gs_split(v.x, v.y, h[2 * c], m[2 * c], l[2 * c]);
+                    gs_split(v.z, v.w, h[2 * c + 1], m[2 * c + 1], l[2 * c + 1]);
+                }
+                ok = mbar_wait(a_empty + ab, ap ^ 1, abort_flag, args.status);   // the tensor core may still read this buffer
+                if (!ok) break;
+                __syncwarp();
+                tc_fence_after();
+                const uint32_t dst = dst0 + ab * 96;
+                gs_st16(dst, h);
+                gs_st16(dst + 32, m);
+                gs_st16(dst + 64, l);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(w_empty + stage);
+                    gs_arrive_first(a_ready + ab);
+                }
+                if (++stage == args.stages) stage = 0, phase ^= 1;
+                if (++ab == GS_A_BUFS) ab = 0, ap ^= 1;
+            }
+        }
+    } else {   // ---- sums: a row of W (a column of C) a thread, all rows of the unit
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;" ::: "memory");
+        const int quarter = warp & 3, groups = args.nt / 16;
+        const uint32_t src0 = tmem + ((uint32_t)(quarter * 32) << 16);
+        int n = 0;
+        bool ok = true;
+        for (int u = blockIdx.x >> 1; u < units && ok; u += pairs) {
+            int wt, xt, seg, turns;
+            unit_of(u, wt, xt, seg, turns);
+            float sum[GS_NT_MAX];
+#pragma unroll
+            for (int i = 0; i < GS_NT_MAX; ++i) sum[i] = 0.f;
+            for (int k = 0; k < turns; ++k, ++n) {
+                const int b = n & 1;
+                ok = mbar_wait<true>(sum_full + b, (n >> 1) & 1, abort_flag, args.status);
+                if (!ok) break;
+                __syncwarp();
+                tc_fence_after();
+#pragma unroll
+                for (int g = 0; g < GS_NT_MAX / 16; ++g)
+                    if (g < groups) {
+                        float v[16];
+                        tc_ld16(src0 + b * args.nt + g * 16, v);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) sum[g * 16 + i] += v[i];
+                    }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) gs_arrive_first(sum_empty + b);
+            }
+            if (!ok) break;
+            const int col = wt * 256 + rank * 128 + quarter * 32 + lane, row0 = xt * args.nt;
+            const int rows = col < args.N ? min(args.nt, args.M - row0) : 0;
+            float* out = args.out + (long long)row0 * args.N + col;
+            bool odd = false;
+            if (args.n_seg == 1) {
+#pragma unroll
+                for (int g = 0; g < GS_NT_MAX / 16; ++g)
+                    if (g < groups) odd |= GS_STORE16(out + (long long)(g * 16) * args.N, args.N, rows - g * 16, sum, g * 16);
+            } else {
+                const long long seg_size = (long long)args.M * args.N;
+                float* own = args.sums + seg * seg_size + (long long)row0 * args.N + col;
+#pragma unroll
+                for (int g = 0; g < GS_NT_MAX / 16; ++g)
+                    if (g < groups) GS_STORE16(own + (long long)(g * 16) * args.N, args.N, rows - g * 16, sum, g * 16);
+                __threadfence();
+                __syncwarp();
+                int* count = args.arrived + (wt * args.x_tiles + xt) * 8 + rank * 4 + quarter;
+                int before = 0;
+                if (lane == 0) before = atomicAdd(count, 1);
+                if (__shfl_sync(0xffffffffu, before, 0) != args.n_seg - 1) continue;
+                __threadfence();
+                const float* all = args.sums + (long long)row0 * args.N + col;
+#pragma unroll 1
+                for (int g = 0; g < groups; ++g) {
+                    float v[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) v[i] = 0.f;
+                    const float* p = all + (long long)(g * 16) * args.N;
+#pragma unroll 2
+                    for (int s = 0; s < args.n_seg; ++s, p += seg_size)
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (g * 16 + i < rows) v[i] += __ldcg(p + (long long)i * args.N);
+                    odd |= GS_STORE16(out + (long long)(g * 16) * args.N, args.N, rows - g * 16, v, 0);
+                }
+            }
+            if (__any_sync(0xffffffffu, odd)) {   // from the numbers themselves: an output at a time, the lanes along k
+                for (int i = 0; i < args.nt && row0 + i < args.M; ++i)
+                    for (int c = 0; c < 32 && col - lane + c < args.N; ++c) {
+                        float* o = args.out + (long long)(row0 + i) * args.N + col - lane + c;
+                        __syncwarp();
+                        if (fabsf(*reinterpret_cast<volatile float*>(o)) <= 3.402823466e38f) continue;
+                        float v = 0.f;
+                        for (int k = lane; k < args.K; k += 32)
+                            v = fmaf(args.a[(long long)(row0 + i) * args.K + k], args.w[(long long)(col - lane + c) * args.K + k], v);
+                        v = warp_sum(v);
+                        __syncwarp();
+                        if (lane == 0) *o = v;
+                    }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // neither leaves while the other may still reach it
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+}
+
+// ---- host side ----------------------------------------------------------------------------------
+
+static int gs_float_map(CUtensorMap* map, const void* ptr, long long rows, long long cols) {   // boxes of 128 rows x 32 floats
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return (int)cudaErrorNotSupported;
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
+    cuuint32_t box[2] = {32, 128};
+    cuuint32_t elem[2] = {1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
+// Columns of k in a segment, by N and K alone: as many segments as let a call of one unit's rows fill the GPU's 74 pairs, none shorter
+// than 512 columns.
+static int gs_seg_k(int N, int K) {
+    const int tiles = (N + 255) / 256;
+    int n = 74 / tiles;
+    if (n > K / 512) n = K / 512;
+    if (n < 1) n = 1;
+    return (((K + n - 1) / n) + 63) / 64 * 64;
+}
+
+extern "C" {
+
+// Segments of a product, 0 where it is not taken: K and N as TMA and the stores want them, matrices from 12 million numbers on (below, the
+// units do not fill the GPU).  A rule of N and K alone, so that calls of different rows on a matrix sum alike.
+int sb_gemm_split_segments(int N, int K) {
+    if (N < 1 || K < 512 || K % 8 || N % 4 || (long long)N * K < 12000000ll) return 0;
+    const int seg = gs_seg_k(N, K);
+    return (K + seg - 1) / seg;
+}
+
+// C [M, N] of a [M, K] and w [N, K], 32-bit, contiguous, on 16-byte boundaries.  parts: 3 M K bfloat16 and, on a boundary of 16 bytes behind
+// them, 8 (M / 16 + 1) (N / 256 + 1) counters; sums: segments x M x N floats, or nullptr where there is one segment.
+int sb_gemm_split(const float* a, const float* w, float* c, int M, int N, int K, void* parts, float* sums, int sms, int* status,
+                  cudaStream_t stream) {
+    if (M <= 0) return 0;
+    const int n_seg = sb_gemm_split_segments(N, K);
+    if (!n_seg || (n_seg > 1) != (sums != nullptr) || !sb_aligned(16, (const char*)a, (const char*)w, (const char*)c, (const char*)parts, (const char*)sums) ||
+        (long long)M * K > (1ll << 33) || M > (1 << 29) || sms < 2)
+        return (int)cudaErrorInvalidValue;
+    const int pairs = sms / 2, w_tiles = (N + 255) / 256;
+    // Rows of A to a unit: of the cuts that the registers allow, the one whose rounds of units take least; a round of fewer than 64 rows costs
+    // what splitting W and bringing it costs.
+    int best = 0, x_tiles = 1;
+    long long least = 0;
+    for (int t = (M + GS_NT_MAX - 1) / GS_NT_MAX, tries = 0; tries < 6; ++t, ++tries) {
+        const int nt = ((M + t - 1) / t + 15) / 16 * 16, used = (M + nt - 1) / nt;
+        const long long rounds = ((long long)w_tiles * used * n_seg + pairs - 1) / pairs, cost = rounds * (nt < 64 ? 64 : nt);
+        if (best == 0 || cost < least) best = nt, x_tiles = used, least = cost;
+        if (nt <= 16) break;
+    }
+    const long long units = (long long)w_tiles * x_tiles * n_seg;
+    if (units > 0x3fffffff) return (int)cudaErrorInvalidValue;
+    const int stage = GS_W_BYTES + 3 * best * 64, fit = (GS_SMEM - 1024) / stage;
+    int* arrived = reinterpret_cast<int*>((char*)parts + ((6ll * M * K + 15) & ~15ll));
+    GsArgs args = {a, w, c, sums, arrived, status, M, N, K, best, fit < GS_STAGES_MAX ? fit : GS_STAGES_MAX, gs_seg_k(N, K), n_seg, w_tiles, x_tiles};
+    CUtensorMap mw, mx;
+    int e = gs_float_map(&mw, w, N, K);
+    if (e) return e;
+    e = make_rows_map(&mx, parts, 3ll * M, K, K, best / 2);
+    if (e) return e;
+    static const cudaError_t configured = cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM);
+    if (configured != cudaSuccess) return (int)configured;
+    const long long n8 = (long long)M * K / 8, b8 = (n8 + 255) / 256;
+    sb_launch(gemm_split_rows_kernel, dim3((unsigned int)(b8 < 2368 ? b8 : 2368)), dim3(256), 0, stream, a, (uint4*)parts, n8, arrived,
+              n_seg > 1 ? w_tiles * x_tiles * 8 : 0);
+    sb_launch(gemm_split_kernel, dim3(2 * (unsigned int)(units < pairs ? units : pairs)), dim3(GS_THREADS), GS_SMEM, stream, mw, mx, args);
+    return (int)cudaGetLastError();
+}
+
+}  // extern "C"

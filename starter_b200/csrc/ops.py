@@ -108,6 +108,8 @@ class Ops:
             "sb_length_order": [SbBatch, c_void_p, c_void_p],
             "sb_advance_lengths": [SbBatch, c_void_p, c_void_p],
             "sb_gemm_general": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+            "sb_gemm_split_segments": [c_int, c_int],
+            "sb_gemm_split": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
             "sb_qk_rope_store": [c_int, c_int, c_void_p, c_void_p, SbBatch, SbKV, c_int, c_int, c_void_p, c_void_p,
                                  c_float, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
             "sb_attention_general": [c_int, c_void_p, c_void_p, SbBatch, SbKV, c_int, c_float, c_int, c_void_p],
@@ -245,6 +247,7 @@ class Ops:
         self._tiled_bytes = 0     # bytes of tile-major copies alive (a copy hangs on its matrix as ._sb_tiled = (copy, halves))
         self.decode_copy = os.environ.get("STARTER_B200_DECODE_COPY", "auto")   # "1", "0" or "auto"
         self.use_rows = os.environ.get("STARTER_B200_ROWS", "1") != "0"      # products of many rows with their activation in one kernel
+        self.use_split = os.environ.get("STARTER_B200_SPLIT", "1") != "0"    # 32-bit products of large matrices on the tensor cores
         self.use_stream = os.environ.get("STARTER_B200_STREAM", "1") != "0"  # the TMA + tcgen05 product for decode
         self._kernel_status = None
         self._status_override = None
@@ -639,6 +642,8 @@ class Ops:
                 return torch.mm(a, w.t())
         out = torch.empty((M, N), dtype=torch.float32 if out_float32 else a.dtype, device=a.device)
         a = a.contiguous()
+        if a.dtype == torch.float32 and self._split_product(a, w, out):
+            return out
         floats = self.lib.sb_gemm_general_scratch(_code(a.dtype), M, N, K)
         parts = self._room_for(floats, a.device) if floats else None   # without: the chunks of k one after another, the same sums
         self._check(self.lib.sb_gemm_general(_code(a.dtype), int(out_float32 or a.dtype == torch.float32), _ptr(a), _ptr(w),
@@ -646,6 +651,37 @@ class Ops:
         if parts is not None:
             self.launches += 1   # the chunks' sums are added up
         return out
+
+    SPLIT_MIN_ROWS = 9
+    SPLIT_SUMS = 64 << 20   # floats of segments' sums that a call keeps at most; more rows go in pieces, which changes no bit
+
+    def _split_product(self, a, w, out) -> bool:
+        """The 32-bit product as six bfloat16 products on the tensor cores (gemm_split.cu), where N and K and the addresses allow it and
+        its scratch can be had.  An output is the same number whichever rows stand beside its own; up to 8 rows are left to the kernel that
+        streams the weights, which is about twice as fast there and sums in another order."""
+        M, K = a.shape
+        N = w.shape[0]
+        segments = self.lib.sb_gemm_split_segments(N, K) if self.use_split else 0
+        if not segments or M < self.SPLIT_MIN_ROWS or not w.is_contiguous() or (a.data_ptr() | w.data_ptr() | out.data_ptr()) % 16:
+            return False
+        step = M if segments == 1 else max(1, min(M, self.SPLIT_SUMS // (segments * N)))
+        sums = None
+        while segments > 1:
+            sums = self._room_for(segments * step * N, a.device)
+            if sums is not None:
+                break
+            if step == 1:
+                return False
+            step = max(1, step // 4)
+        parts = self._room_for(3 * step * K // 2 + 4 + 8 * (step // 16 + 1) * (N // 256 + 1), a.device)   # three bfloat16 numbers each, counters
+        if parts is None:
+            return False
+        for m in range(0, M, step):
+            n = min(step, M - m)
+            self._check(self.lib.sb_gemm_split(a.data_ptr() + 4 * m * K, _ptr(w), out.data_ptr() + 4 * m * N, n, N, K, _ptr(parts), _ptr(sums),
+                                               self.sm_count(), _ptr(self.kernel_status(a.device)), self._stream()), "gemm_split")
+            self.launches += 1   # the rows' split
+        return True
 
     # What follows a product of many rows in its epilogue (gemm_rows.cu)
     ROWS_PLAIN, ROWS_SWIGLU, ROWS_CLAMP, ROWS_GELU, ROWS_RELU2, ROWS_XIELU = range(6)

@@ -1,0 +1,97 @@
+"""The 32-bit product as six bfloat16 products on the tensor cores: at the borders of its tiles, segments and stages, against 64 bits and the
+CUDA cores' product."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from starter_b200.csrc.ops import get_ops
+    return get_ops(verbose=False)
+
+
+def rand(shape, seed):
+    return torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda")
+
+
+def both(ops, a, w):
+    assert ops.lib.sb_gemm_split_segments(*w.shape) > 0
+    before = ops.launches
+    got = ops.linear(a, w)
+    assert ops.launches == before + 2
+    ops.use_split = False
+    try:
+        return got, ops.linear(a, w)
+    finally:
+        ops.use_split = True
+
+
+# 256 columns a tile, up to 112 rows a unit, 64 columns of k a stage; one to fourteen segments
+@pytest.mark.parametrize("M", [9, 15, 17, 112, 113, 225, 600])
+@pytest.mark.parametrize("N, K", [(3076, 4096), (2944, 4104), (6144, 2568), (23552, 512), (1280, 9728)])
+def test_against_64_bits(ops, M, N, K):
+    a, w = rand((M, K), 1), rand((N, K), 2) * K ** -0.5
+    got, cuda = both(ops, a, w)
+    want = a.double() @ w.double().T
+    off = float((got - want).norm() / want.norm())
+    # sums of 64 products are cut, not rounded, at 2^-24 of their size in four steps; the rest as the CUDA cores' sums in shorter runs
+    assert off < 4e-7 and off <= float((cuda - want).norm() / want.norm()) * 1.02
+    assert torch.equal(ops.linear(a[-9:].contiguous(), w), got[-9:]), "a row's sums depend on the rows beside it"
+    assert torch.equal(torch.cat([ops.linear(piece, w) for piece in a.split(50)]), got)
+    assert ops.read_kernel_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["positive", "wide", "large", "small"])
+def test_other_numbers(ops, kind):
+    """Sums without cancellation, factors of e^4 a standard deviation, numbers near the ends of what products may reach."""
+    a, w = rand((130, 2560), 3), rand((4736, 2560), 4)
+    if kind == "positive":
+        a, w = a.abs(), w.abs()
+    elif kind == "wide":
+        a, w = a * torch.exp(4 * rand(a.shape, 5)), w * torch.exp(4 * rand(w.shape, 6))
+    elif kind == "large":
+        a, w = a * 1e18, w * 1e18
+    else:
+        a, w = a * 1e-14, w * 1e-14
+    got, cuda = both(ops, a, w)
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert float(((got - want).abs() / size).max()) <= max(2.0 ** -22, float(((cuda - want).abs() / size).max()))
+
+
+def test_numbers_that_are_not_finite(ops):
+    """Infinities, NaN and numbers that bfloat16 rounds to infinity give what the 32-bit sums give; other rows and columns keep theirs."""
+    a, w = rand((40, 4096), 7), rand((3072, 4096), 8)
+    a[3, 5], a[7, 100], w[9, 11], a[11, 20], w[20, 20] = float("inf"), float("nan"), float("-inf"), 3.4e38, 1e-30
+    got, cuda = both(ops, a, w)
+    assert torch.equal(got.isnan(), cuda.isnan()) and torch.equal(got.isinf(), cuda.isinf())
+    assert torch.equal(got[got.isinf()], cuda[cuda.isinf()])
+    rest = torch.ones(40, dtype=torch.bool, device="cuda")
+    rest[[3, 7, 11]] = False
+    columns = torch.ones(3072, dtype=torch.bool, device="cuda")
+    columns[[9, 20]] = False
+    want = (a.double() @ w.double().T)[rest][:, columns]
+    assert float((got[rest][:, columns] - want).abs().max() / want.abs().max()) < 1e-6
+
+
+def test_without_room_the_rows_go_in_pieces(ops, monkeypatch):
+    a, w = rand((300, 4096), 9), rand((3072, 4096), 10)
+    want, empty = ops.linear(a, w), torch.empty
+
+    def limited(*size, dtype=None, **kwargs):
+        if dtype == torch.float32 and len(size) == 1 and isinstance(size[0], int) and 4 * size[0] > 4 * 2 ** 20:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*size, dtype=dtype, **kwargs)
+    monkeypatch.setattr(torch, "empty", limited)
+    assert torch.equal(ops.linear(a, w), want)
+
+
+def test_which_products(ops):
+    takes = lambda n, k: ops.lib.sb_gemm_split_segments(n, k) > 0   # noqa: E731
+    assert takes(3072, 4096) and not takes(2560, 4096) and not takes(3073, 4096) and not takes(3072, 4100) and not takes(100000, 504)
+    a, w = rand((20, 4096), 11), rand((3072 * 4096 + 1,), 12)[1:].view(3072, 4096)   # not on a 16-byte boundary: the CUDA cores
+    want = a.double() @ w.double().T
+    assert float((ops.linear(a, w) - want).norm() / want.norm()) < 1e-6
+    assert torch.equal(ops.linear(a[:8].contiguous(), w.clone()), ops.linear(a[:8].contiguous(), w))     # up to 8 rows they take both
