@@ -25,7 +25,7 @@ __device__ __forceinline__ void mf_mma(float (&c)[4], const uint4& a, const uint
 }
 
 // An expert that every row of the step takes beside the chosen ones (a shared expert): its columns are blocks of the same launches,
-// the first ones, since it is the widest.  rows = 0: there is none.
+// the first ones, since it is the widest.
 struct MfShared {
     const __nv_bfloat16* x;
     const __nv_bfloat16* w;
@@ -36,22 +36,28 @@ struct MfShared {
 
 // GATE_UP: out[pair][c] = act(gate_c, up_c) of x = h's row pair / top, w = [2 n_cols][K] per expert, gate over up.  Otherwise
 // out[pair][c] = w_c x with x = the pair's own row, w = [n_cols][K] per expert.
-template <bool GATE_UP>
+template <bool GATE_UP, bool SHARED>
 __global__ void __launch_bounds__(32 * MF_WARPS, 3)
-moe_few_kernel(const __nv_bfloat16* x, const int* __restrict__ chosen, const __nv_bfloat16* w, __nv_bfloat16* out, int n_pairs, int top, int K,
-               int n_cols, float alpha, float limit, int silu, MfShared shared) {
+moe_few_kernel(const __nv_bfloat16* __restrict__ x_in, const int* __restrict__ chosen, const __nv_bfloat16* __restrict__ w_in,
+               __nv_bfloat16* __restrict__ out_in, int n_pairs, int top_in, int K_in, int n_cols_in, float alpha_in, float limit_in, int silu_in,
+               MfShared shared) {
     constexpr int M = GATE_UP ? 2 : 1;
     __shared__ int list[MF_MAX_PAIRS];
     __shared__ int count_s;
     __shared__ float red[MF_WARPS][M][MF_NT][16][9];
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int first_blocks = shared.rows > 0 ? (shared.n_cols + 15) / 16 : 0, per_expert = (n_cols + 15) / 16;
-    const bool all = (int)blockIdx.x < first_blocks;
-    const int b0 = blockIdx.x - (all ? 0 : first_blocks), e = all ? 0 : b0 / per_expert, c0 = (all ? b0 : b0 % per_expert) * 16;
+    // Without a shared expert a block's expert and column are its place in the grid, and what it reads are the launch's arguments.
+    const int first_blocks = SHARED ? (shared.n_cols + 15) / 16 : 0, per_expert = (n_cols_in + 15) / 16;
+    const bool all = SHARED && (int)blockIdx.x < first_blocks;
+    const int b0 = blockIdx.x - first_blocks, e = all ? 0 : SHARED ? b0 / per_expert : blockIdx.y;
+    const int c0 = (all ? blockIdx.x : SHARED ? b0 % per_expert : blockIdx.x) * 16;
+    const __nv_bfloat16* __restrict__ x = all ? shared.x : x_in;
+    const __nv_bfloat16* __restrict__ w = all ? shared.w : w_in;
+    __nv_bfloat16* __restrict__ out = all ? shared.out : out_in;
+    const int K = all ? shared.K : K_in, n_cols = all ? shared.n_cols : n_cols_in, silu = all ? shared.silu : silu_in, top = all ? 1 : top_in;
+    const float alpha = all ? shared.alpha : alpha_in, limit = all ? shared.limit : limit_in;
     if (all) {
-        x = shared.x, w = shared.w, out = shared.out, K = shared.K, n_cols = shared.n_cols, silu = shared.silu, alpha = shared.alpha, limit = shared.limit;
-        top = 1;
         for (int i = threadIdx.x; i < shared.rows; i += 32 * MF_WARPS) list[i] = i;
         if (threadIdx.x == 0) count_s = shared.rows;
     } else if (warp == 0) {
@@ -164,12 +170,18 @@ int sb_moe_few(const void* h, const int* chosen, const void* w_gate_up, const vo
     const int rows = s_ff > 0 ? n_pairs / top : 0;
     const MfShared up = {(const bf*)h, (const bf*)s_gate_up, (bf*)s_act, rows, width, s_ff, s_silu, s_alpha, s_limit};
     const MfShared dn = {(const bf*)s_act, (const bf*)s_down, (bf*)s_out, rows, s_ff, width, 0, 0.f, 0.f};
-    const long long b1 = (long long)((ff + 15) / 16) * n_experts + (rows ? (s_ff + 15) / 16 : 0);
-    const long long b2 = (long long)((width + 15) / 16) * (n_experts + (rows ? 1 : 0));
+    if (rows == 0) {
+        sb_launch(moe_few_kernel<true, false>, dim3((ff + 15) / 16, n_experts), 32 * MF_WARPS, 0, stream, (const bf*)h, chosen, (const bf*)w_gate_up,
+                  (bf*)act, n_pairs, top, width, ff, alpha, limit, silu, up);
+        sb_launch(moe_few_kernel<false, false>, dim3((width + 15) / 16, n_experts), 32 * MF_WARPS, 0, stream, (const bf*)act, chosen, (const bf*)w_down,
+                  (bf*)down, n_pairs, top, ff, width, 0.f, 0.f, 0, dn);
+        SB_LAUNCH_CHECK();
+    }
+    const long long b1 = (long long)((ff + 15) / 16) * n_experts + (s_ff + 15) / 16, b2 = (long long)((width + 15) / 16) * (n_experts + 1);
     if (b1 > 0x7fffffff || b2 > 0x7fffffff) return (int)cudaErrorInvalidValue;
-    sb_launch(moe_few_kernel<true>, dim3((unsigned int)b1), 32 * MF_WARPS, 0, stream, (const bf*)h, chosen, (const bf*)w_gate_up, (bf*)act, n_pairs,
+    sb_launch(moe_few_kernel<true, true>, dim3((unsigned int)b1), 32 * MF_WARPS, 0, stream, (const bf*)h, chosen, (const bf*)w_gate_up, (bf*)act, n_pairs,
               top, width, ff, alpha, limit, silu, up);
-    sb_launch(moe_few_kernel<false>, dim3((unsigned int)b2), 32 * MF_WARPS, 0, stream, (const bf*)act, chosen, (const bf*)w_down, (bf*)down, n_pairs,
+    sb_launch(moe_few_kernel<false, true>, dim3((unsigned int)b2), 32 * MF_WARPS, 0, stream, (const bf*)act, chosen, (const bf*)w_down, (bf*)down, n_pairs,
               top, ff, width, 0.f, 0.f, 0, dn);
     SB_LAUNCH_CHECK();
 }
