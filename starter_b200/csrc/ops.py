@@ -617,7 +617,7 @@ class Ops:
     def linear(self, a, w, out_float32=False, norm=None, add_to=None):
         """a [M, K] times w [N, K] transposed -> [M, N] in a's dtype, or 32-bit when asked.
 
-        float32: this library's CUDA-core product, always.  bfloat16: the weight-streaming kernels for up
+        float32: this library's CUDA-core product, or the same from three-part numbers (``_split_product``).  bfloat16: the weight-streaming kernels for up
         to 16 rows (and for the output head up to 64), cuBLAS for larger products, the CUDA-core product for what is left.
 
         norm=(weight, eps[, statistics]): the product of the RMSNorm of a's rows; add_to=x: x += product, in place, x
