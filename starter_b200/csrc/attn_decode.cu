@@ -57,18 +57,22 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restric
     // the lengths, the page table, the norm weights and rotary tables, and pages before the one that holds
     // the new token.  If that kernel releases this one early, the look-ups and first copies below overlap it.
     sb_stamp(4, 0);
-    int seq = blockIdx.x, kvh = blockIdx.y;
+    int seq = blockIdx.x, kvh = blockIdx.y, slot, row, pos;   // pos: the new token's position; keys 0..pos are visible
     const int split = blockIdx.z;
-    if (FUSED && fused.order != nullptr) {   // blocks start in the order of their numbers: the longest sequence's pairs first
-        const int number = blockIdx.y * gridDim.x + blockIdx.x;
-        seq = fused.order[number / gridDim.y];
-        kvh = number % gridDim.y;
+    if (FUSED && fused.places != nullptr) {   // more blocks than the GPU holds; where lengths differ the longest sequence's start first
+        const int number = blockIdx.y * gridDim.x + blockIdx.x, n = gridDim.x;
+        const int4 plain = fused.places[blockIdx.x], ranked = fused.places[n + number / gridDim.y];
+        const bool by_rank = fused.places[2 * n].x != 0;
+        const int4 at = by_rank ? ranked : plain;
+        seq = at.x, slot = at.y, pos = at.z, row = at.w;
+        if (by_rank) kvh = number % gridDim.y;
+    } else {
+        slot = batch.seq_slot[seq];
+        row = batch.cu_q[seq];
+        pos = batch.lengths[slot];
     }
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = n_heads / kv.n_kv_heads;
-    const int slot = batch.seq_slot[seq];
-    const int row = batch.cu_q[seq];
-    const int pos = batch.lengths[slot];                   // the new token's position; keys 0..pos are visible
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
     const int first_page = lo / SB_PAGE, last_page = pos / SB_PAGE;
     const int n_pages = last_page - first_page + 1;

@@ -42,7 +42,7 @@ class SbKV(Structure):
 class SbFusedQK(Structure):
     _fields_ = [("qkv", c_void_p), ("q_norm", c_void_p), ("k_norm", c_void_p), ("cos_t", c_void_p), ("sin_t", c_void_p),
                 ("status", c_void_p), ("eps", c_float), ("norm_f32", c_int), ("store_kv", c_int), ("reserved", c_int),
-                ("next_w", c_void_p), ("next_bytes", c_longlong), ("order", c_void_p)]
+                ("next_w", c_void_p), ("next_bytes", c_longlong), ("places", c_void_p)]
 
 
 class SbFlex(Structure):
@@ -105,7 +105,7 @@ class Ops:
             "sb_gather_rows": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
             "sb_rmsnorm": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
             "sb_swiglu": [c_int, c_void_p, c_void_p, c_int, c_int, c_void_p],
-            "sb_length_order": [SbBatch, c_void_p, c_void_p],
+            "sb_length_places": [SbBatch, c_void_p, c_int, c_void_p],
             "sb_advance_lengths": [SbBatch, c_void_p, c_void_p],
             "sb_gemm_general": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
             "sb_gemm_split_segments": [c_int, c_int],
@@ -423,20 +423,23 @@ class Ops:
         self._check(self.lib.sb_swiglu(_code(gu.dtype), _ptr(gu), _ptr(out), gu.shape[0], inter, self._stream()), "swiglu")
         return out
 
+    ALWAYS_BY_RANK = 1.6   # blocks over the blocks that the GPU holds, from which on sequences of equal length go by rank too
+
     def begin_step(self, ctx) -> None:
         """Called before a step's first layer, for models whose attention asks for it (``ranks_lengths``).  Where decode attention has more
-        (sequence, kv head) blocks than the GPU holds at once, the sequences are ranked by length, once for all layers, and their blocks
-        start the longest first: 64 sequences of 128 to 2,048 tokens at the 4B sizes 4,711 -> 4,380 us a step.  An order that every block works
-        out for itself costs steps of equal lengths 2 to 5%."""
-        ctx.scratch.pop("length_order", None)   # of the step before, where a context is kept
+        (sequence, kv head) blocks than the GPU holds at once, one kernel writes down where every sequence stands, once for all layers, and ranks
+        the sequences by length: their blocks start the longest first where lengths differ.  PLACES_MEASURED"""
+        ctx.scratch.pop("length_places", None)   # of the step before, where a context is kept
         if not (ctx.runtime.is_bf16 and ctx.is_decode and 2 <= ctx.n_seqs <= 1024) or ctx.uneven:
             return
         heads = max((getattr(g.request, "num_kv_heads", 0) for g in ctx.cache.groups), default=0)
-        if ctx.n_seqs * heads <= self.decode_resident(128):
+        blocks, places = ctx.n_seqs * heads, self.decode_resident(128)
+        if blocks <= places:
             return
-        order = torch.empty(ctx.n_seqs, dtype=torch.int32, device=ctx.lengths.device)
-        self._check(self.lib.sb_length_order(self._batch(ctx), _ptr(order), self._stream()), "length_order")
-        ctx.scratch["length_order"] = order
+        table = torch.empty((2 * ctx.n_seqs + 1, 4), dtype=torch.int32, device=ctx.lengths.device)
+        self._check(self.lib.sb_length_places(self._batch(ctx), _ptr(table), int(blocks >= self.ALWAYS_BY_RANK * places), self._stream()),
+                    "length_places")
+        ctx.scratch["length_places"] = table
 
     def advance_lengths(self, ctx):
         self._check(self.lib.sb_advance_lengths(self._batch(ctx), _ptr(ctx.lengths), self._stream()), "advance_lengths")
@@ -966,7 +969,7 @@ class Ops:
         n_splits = self.decode_splits(ctx.n_seqs, kv.n_kv_heads, layer_cache.group.table_width, kv.head_dim)
         partial, counters = self._decode_scratch(qkv.device, ctx.n_seqs, n_heads, kv.n_kv_heads, kv.head_dim, n_splits)
         if ctx.n_seqs * kv.n_kv_heads * n_splits > self.decode_resident(kv.head_dim):
-            fused.order = _ptr(ctx.scratch.get("length_order"))
+            fused.places = _ptr(ctx.scratch.get("length_places"))
         self._check(self.lib.sb_attn_decode_fused(fused, _ptr(out), self._batch(ctx), kv, n_heads, scale, int(window or 0),
                                                   n_splits, _ptr(partial), _ptr(counters), self._stream()), "attn_decode_fused")
         return out

@@ -25,7 +25,7 @@ struct SbFusedQK {
     int reserved;
     const void* next_w;        // a matrix (16-byte aligned) that the kernel after this one streams: asked into L2 when
     long long next_bytes;      // this kernel's keys are read, so that memory stays busy through its merge; or null
-    const int* order;          // the split-key kernel: the sequences in the order in which their blocks start, or null: by number
+    const int4* places;        // the split-key kernel: what length_places_kernel leaves (rows.cu), or null
 };
 
 __device__ __forceinline__ void unpack4(const uint2 raw, float (&v)[4]) {

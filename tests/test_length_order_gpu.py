@@ -9,12 +9,13 @@ from starter_b200.engine.context import Runtime, StepContext
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n, splits", [(2, 1), (40, 1), (40, 2), (133, 1), (1024, 1)])
-def test_the_longest_first(monkeypatch, n, splits):
+@pytest.mark.parametrize("n, splits, most", [(2, 1, 130), (40, 1, 130), (40, 2, 130), (133, 1, 60), (1024, 1, 130)])
+@pytest.mark.parametrize("always", [0, 10 ** 9])
+def test_the_longest_first(monkeypatch, n, splits, most, always):
     from starter_b200.csrc.ops import get_ops
     ops, (G, H, D) = get_ops(verbose=False), (8, 16, 64)
     g = torch.Generator().manual_seed(n)
-    lengths = torch.randint(0, 130, (n,), generator=g).tolist()
+    lengths = torch.randint(0, most, (n,), generator=g).tolist()
     cache = Cache([KVRequest(G, D)], n_slots=n, max_tokens=64 * 3 * n, dtype=torch.bfloat16, device="cuda", max_seq_tokens=192)
     slots = [cache.alloc() for _ in range(n)]
     for s, length in zip(slots, lengths):
@@ -27,7 +28,7 @@ def test_the_longest_first(monkeypatch, n, splits):
     qkv = torch.randn(n, (H + 2 * G) * D, generator=fill, device="cuda").bfloat16()
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
     monkeypatch.setattr(ops, "decode_splits", lambda *a: splits)
-    monkeypatch.setattr(ops, "decode_resident", lambda d: 0)
+    monkeypatch.setattr(ops, "decode_resident", lambda d: 1)
 
     def run(ranked):
         layer.k.copy_(k0), layer.v.copy_(v0)
@@ -38,11 +39,15 @@ def test_the_longest_first(monkeypatch, n, splits):
         out = ops.qk_attention(ctx, qkv, layer, H, G, D, None, None, 1e-5, None, D ** -0.5, None)
         return ctx, out, layer.k.clone(), layer.v.clone()
 
+    monkeypatch.setattr(ops, "ALWAYS_BY_RANK", always)
     ctx, *got = run(True)
-    order = ctx.scratch["length_order"].tolist()
-    assert order == sorted(range(n), key=lambda s: (-lengths[s], s))
+    table = ctx.scratch["length_places"].tolist()
+    rows = [[s, slots[s], lengths[s], s] for s in range(n)]
+    assert table[:n] == rows and table[n:2 * n] == sorted(rows, key=lambda r: (-r[2], r[0]))
+    pages = [length // 64 + 1 for length in lengths]
+    assert table[2 * n][0] == int(not always or 4 * max(pages) * n > 5 * sum(pages))
     plain, *want = run(False)
-    assert "length_order" not in plain.scratch and all(torch.equal(a, b) for a, b in zip(got, want))
-    ctx.uneven = True      # very unequal lengths go to the kernel of equal shares: nothing is ranked, and an old order is dropped
+    assert "length_places" not in plain.scratch and all(torch.equal(a, b) for a, b in zip(got, want))
+    ctx.uneven = True      # very unequal lengths go to the kernel of equal shares: nothing is ranked, and an old table is dropped
     ops.begin_step(ctx)
-    assert "length_order" not in ctx.scratch
+    assert "length_places" not in ctx.scratch
