@@ -650,7 +650,7 @@ class TimedOps:
     def __getattr__(self, name):
         attr = getattr(self._ops, name)
         if not callable(attr) or name in ("prepare_matrix", "folds", "sm_count", "status_into", "set_dependent_launch",
-                                          "read_kernel_status", "kernel_status", "uneven_matters"):
+                                          "read_kernel_status", "kernel_status", "uneven_matters", "moe_takes_shared", "begin_step"):
             return attr
 
         def timed(*args, **kwargs):
