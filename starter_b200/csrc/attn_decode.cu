@@ -39,7 +39,7 @@ namespace cg = cooperative_groups;
 #define AD_MAX_CLUSTER 8
 #define AD_MAX_DEVICES 64     // devices whose per-device set-up this file remembers
 
-template <int D, bool FUSED, int AD_STAGES>
+template <int D, bool FUSED, int AD_STAGES, bool RANKED>
 __global__ void __launch_bounds__(AD_WARPS * 32)
 attn_decode_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ out, SbBatch batch, SbKV kv,
                    int n_heads, float scale_log2, int window, int n_splits, int cluster_merge, float* __restrict__ partial,
@@ -57,16 +57,16 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restric
     // the lengths, the page table, the norm weights and rotary tables, and pages before the one that holds
     // the new token.  If that kernel releases this one early, the look-ups and first copies below overlap it.
     sb_stamp(4, 0);
-    int seq = blockIdx.x, kvh = blockIdx.y, slot, row, pos;   // pos: the new token's position; keys 0..pos are visible
-    const int split = blockIdx.z;
-    if (FUSED && fused.places != nullptr) {   // more blocks than the GPU holds; where lengths differ the longest sequence's start first
-        const int number = blockIdx.y * gridDim.x + blockIdx.x, n = gridDim.x;
-        const int4 plain = fused.places[blockIdx.x], ranked = fused.places[n + number / gridDim.y];
-        const bool by_rank = fused.places[2 * n].x != 0;
-        const int4 at = by_rank ? ranked : plain;
+    // RANKED: more blocks than the GPU holds at once.  They start in the order of their numbers, so kv heads lie along x and sequences along
+    // y, the longest first; one read says where a sequence stands.  kvh stays the same number for the whole block either way, which keeps
+    // the addresses of the page loop out of its registers (taken from a look-up it cost steps of equal lengths 2%).
+    const int kvh = RANKED ? blockIdx.x : blockIdx.y, split = blockIdx.z;
+    int seq, slot, row, pos;                               // pos: the new token's position; keys 0..pos are visible
+    if (RANKED) {
+        const int4 at = fused.places[blockIdx.y];
         seq = at.x, slot = at.y, pos = at.z, row = at.w;
-        if (by_rank) kvh = number % gridDim.y;
     } else {
+        seq = blockIdx.x;
         slot = batch.seq_slot[seq];
         row = batch.cu_q[seq];
         pos = batch.lengths[slot];
@@ -443,7 +443,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restric
     sb_stamp(4, 5);
 }
 
-template <int D, bool FUSED, int AD_STAGES>
+template <int D, bool FUSED, int AD_STAGES, bool RANKED = false>
 static int launch_decode_staged(const void* q, void* out, SbBatch batch, SbKV kv, int n_heads, float scale, int window, int n_splits,
                          float* partial, int* counters, SbFusedQK fused, cudaStream_t stream) {
     const int pipe_bytes = AD_WARPS * AD_STAGES * 2 * AD_KEYS_PER_WARP * D * 2;
@@ -454,13 +454,13 @@ static int launch_decode_staged(const void* q, void* out, SbBatch batch, SbKV kv
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= AD_MAX_DEVICES) return (int)cudaErrorInvalidDevice;
     if (!configured[device]) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, FUSED, AD_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, FUSED, AD_STAGES, RANKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured[device] = true;
     }
     const int cluster_merge = n_splits >= 2 && n_splits <= AD_MAX_CLUSTER;
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(batch.n_seqs, kv.n_kv_heads, n_splits);
+    config.gridDim = RANKED ? dim3(kv.n_kv_heads, batch.n_seqs, n_splits) : dim3(batch.n_seqs, kv.n_kv_heads, n_splits);
     config.blockDim = dim3(AD_WARPS * 32);
     config.dynamicSmemBytes = smem;
     config.stream = stream;
@@ -480,7 +480,7 @@ static int launch_decode_staged(const void* q, void* out, SbBatch batch, SbKV kv
     }
     config.attrs = attr;
     config.numAttrs = n_attr;
-    cudaError_t e = cudaLaunchKernelEx(&config, attn_decode_kernel<D, FUSED, AD_STAGES>, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, batch,
+    cudaError_t e = cudaLaunchKernelEx(&config, attn_decode_kernel<D, FUSED, AD_STAGES, RANKED>, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, batch,
                                        kv, n_heads, scale * 1.4426950408889634f, window, n_splits, cluster_merge, partial,
                                        counters, fused);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
@@ -503,6 +503,10 @@ static int launch_decode(const void* q, void* out, SbBatch batch, SbKV kv, int n
     const long long blocks = (long long)batch.n_seqs * kv.n_kv_heads * n_splits;
     if (blocks <= sm_count)
         return launch_decode_staged<D, FUSED, 4>(q, out, batch, kv, n_heads, scale, window, n_splits, partial, counters, fused, stream);
+    if constexpr (FUSED) {
+        if (fused.places != nullptr && batch.n_seqs <= 65535)
+            return launch_decode_staged<D, true, 3, true>(q, out, batch, kv, n_heads, scale, window, n_splits, partial, counters, fused, stream);
+    }
     return launch_decode_staged<D, FUSED, 3>(q, out, batch, kv, n_heads, scale, window, n_splits, partial, counters, fused, stream);
 }
 

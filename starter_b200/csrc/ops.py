@@ -105,7 +105,7 @@ class Ops:
             "sb_gather_rows": [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p],
             "sb_rmsnorm": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
             "sb_swiglu": [c_int, c_void_p, c_void_p, c_int, c_int, c_void_p],
-            "sb_length_places": [SbBatch, c_void_p, c_int, c_void_p],
+            "sb_length_places": [SbBatch, c_void_p, c_void_p],
             "sb_advance_lengths": [SbBatch, c_void_p, c_void_p],
             "sb_gemm_general": [c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
             "sb_gemm_split_segments": [c_int, c_int],
@@ -423,24 +423,23 @@ class Ops:
         self._check(self.lib.sb_swiglu(_code(gu.dtype), _ptr(gu), _ptr(out), gu.shape[0], inter, self._stream()), "swiglu")
         return out
 
-    ALWAYS_BY_RANK = 1.6   # blocks over the blocks that the GPU holds, from which on sequences of equal length go by rank too
+    RANKED_FROM = 1.6   # blocks over the blocks that the GPU holds at once, beyond which sequences are ranked
 
     def begin_step(self, ctx) -> None:
         """Called before a step's first layer, for models whose attention asks for it (``ranks_lengths``).  Where decode attention has more
-        (sequence, kv head) blocks than the GPU holds at once, one kernel writes down where every sequence stands, once for all layers, and ranks
-        the sequences by length: their blocks start the longest first where lengths differ.  4B sizes, us a step: 64 sequences of 128 to 2,048 tokens
-        4,730 -> 4,366, 48 of 94 to 1,500 3,844 -> 3,588, 40 of 125 to 2,000 4,106 -> 3,911.  An order that every block works out for itself, or one more
-        look-up in front of slot and length, costs steps of equal lengths 2 to 5%."""
+        (sequence, kv head) blocks than the GPU holds at once, one kernel writes down where every sequence stands, by falling length, once for all
+        layers, and their blocks start in that order.  4B sizes, us a step, by number / ranked: 64 sequences of 128 to 2,048 tokens 4,730 / 4,366, 64 of
+        500 3,611 / 3,554, 64 of 1,500 5,004 / 4,922; with few more blocks than places the last ones run alone either way, and equal lengths lose a
+        little: 48 of 1,000 4,050 / 4,092, 40 of 500 3,412 / 3,436 (40 of 125 to 2,000 4,249 / 3,898: left out with them, since a captured step
+        does not know its lengths)."""
         ctx.scratch.pop("length_places", None)   # of the step before, where a context is kept
         if not (ctx.runtime.is_bf16 and ctx.is_decode and 2 <= ctx.n_seqs <= 1024) or ctx.uneven:
             return
         heads = max((getattr(g.request, "num_kv_heads", 0) for g in ctx.cache.groups), default=0)
-        blocks, places = ctx.n_seqs * heads, self.decode_resident(128)
-        if blocks <= places:
+        if ctx.n_seqs * heads <= self.RANKED_FROM * self.decode_resident(128):
             return
-        table = torch.empty((2 * ctx.n_seqs + 1, 4), dtype=torch.int32, device=ctx.lengths.device)
-        self._check(self.lib.sb_length_places(self._batch(ctx), _ptr(table), int(blocks >= self.ALWAYS_BY_RANK * places), self._stream()),
-                    "length_places")
+        table = torch.empty((ctx.n_seqs, 4), dtype=torch.int32, device=ctx.lengths.device)
+        self._check(self.lib.sb_length_places(self._batch(ctx), _ptr(table), self._stream()), "length_places")
         ctx.scratch["length_places"] = table
 
     def advance_lengths(self, ctx):

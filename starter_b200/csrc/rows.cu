@@ -239,12 +239,10 @@ __global__ void advance_lengths_kernel(SbBatch b, int* lengths) {
     if (slot != b.null_slot) lengths[slot] += b.cu_q[s + 1] - b.cu_q[s];
 }
 
-// Where the step's sequences stand, (number, slot, tokens held, row), in one read for every block of every layer's decode attention: places[0, n)
-// by number, places[n, 2 n) by falling length (equal ones by number), places[2 n].x: whether the second is to be used, which is where
-// the longest holds a quarter more pages than the mean, or `always`.  One block: two look-ups and n_seqs comparisons a thread, 2 to 4 us a step.
-__global__ void __launch_bounds__(1024) length_places_kernel(SbBatch b, int4* __restrict__ places, int always) {
+// Where the step's sequences stand, (number, slot, tokens held, row), by falling length (equal ones by number): one read for every block of
+// every layer's decode attention.  One block: two look-ups and n_seqs comparisons a thread, 2 to 4 us a step.
+__global__ void __launch_bounds__(1024) length_places_kernel(SbBatch b, int4* __restrict__ places) {
     __shared__ int held[1024];
-    __shared__ float red[33];
     pdl_wait();
     pdl_launch_dependents();
     const int s = threadIdx.x, n = b.n_seqs;
@@ -253,16 +251,12 @@ __global__ void __launch_bounds__(1024) length_places_kernel(SbBatch b, int4* __
         slot = b.seq_slot[s];
         held[s] = b.lengths[slot];
     }
-    const float pages = s < n ? (float)(held[s] / SB_PAGE + 1) : 0.f;
-    const float all = block_sum(pages, red);     // meets the block: every length is there
+    __syncthreads();
     if (s >= n) return;
     const int own = held[s];
     int rank = 0;
     for (int j = 0; j < n; ++j) rank += held[j] > own || (held[j] == own && j < s);
-    const int4 place = make_int4(s, slot, own, b.cu_q[s]);
-    places[s] = place;
-    places[n + rank] = place;
-    if (rank == 0) places[2 * n] = make_int4(always || pages * n > 1.25f * all, 0, 0, 0);
+    places[rank] = make_int4(s, slot, own, b.cu_q[s]);
 }
 
 static inline int row_threads(int width) {
@@ -375,11 +369,11 @@ int sb_advance_lengths(SbBatch b, int* lengths, cudaStream_t stream) {
     SB_LAUNCH_CHECK();
 }
 
-// n_seqs <= 1024; places: 2 n_seqs + 1.
-int sb_length_places(SbBatch b, int4* places, int always, cudaStream_t stream) {
+// n_seqs <= 1024; places: one a sequence.
+int sb_length_places(SbBatch b, int4* places, cudaStream_t stream) {
     if (b.n_seqs <= 0) return 0;
     if (b.n_seqs > 1024 || !sb_aligned(16, (const char*)places)) return (int)cudaErrorInvalidValue;
-    sb_launch(length_places_kernel, 1, (b.n_seqs + 31) / 32 * 32, 0, stream, b, places, always);
+    sb_launch(length_places_kernel, 1, (b.n_seqs + 31) / 32 * 32, 0, stream, b, places);
     SB_LAUNCH_CHECK();
 }
 
